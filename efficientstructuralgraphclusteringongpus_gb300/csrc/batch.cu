@@ -191,9 +191,6 @@ scan_status scan_batch_run(scan_batch* b, const char* const* eps_decimal, const 
     auto similarity = [&](uint32_t* launches) -> scan_status {
         if (d->has_split) return launch_cn(d, launches);
         PredParams on{};   // "prune on"; every other parameter comes from the pivot's graph
-        B_CUDA(cudaMemsetAsync(d->rs.sim, 0, d->E, s));
-        B_CUDA(cudaMemsetAsync(d->rs.sd, 0, d->n * sizeof(int32_t), s));
-        B_CUDA(cudaMemsetAsync(d->rs.ctr, 0, sizeof(RunCounters), s));
         return launch_cn(d, launches, &on, &d->rs, &bp);
     };
     auto queue = [&](uint32_t* launches) -> scan_status {

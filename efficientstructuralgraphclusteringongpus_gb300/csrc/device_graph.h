@@ -16,6 +16,16 @@
 namespace scan {
 struct CnTask;
 
+// The edges between larger vertices, for a kernel with a warp per edge: a hub's edges of this
+// kind sit together in its list (low ids in power-law graphs), and the few warps that drew
+// them would work on long after the others are done.
+struct LongEdges {
+    uint4* slot;         // bitmaps, bits that decide the edge, sizes (kernels_sketch.cuh: SketchSlot)
+    uint32_t* edge;      // edge id
+    uint32_t* count;     // edges offered (may exceed cap)
+    uint32_t cap;
+};
+
 // Task sizing of the similarity stage (set by the planner; re-planned by the autotuner).
 struct PlanParams {
     unsigned long long target_probes;          // probe work per hash-class task
@@ -87,6 +97,14 @@ struct DeviceGraph {
     uint32_t cap_small = 0, cap_big[scan::kNumBigClasses] = {}, cap_hubs = 0;   // task array capacities
     scan::PlanParams plan{};
     uint32_t long_words = 32;      // lists of >= long_words 16-byte words get a whole warp
+    // neighbourhood sketches (kernels_sketch.cuh; null when off)
+    uint2* sk_info = nullptr;          // n: first 16-byte unit of the vertex's bitmaps, degree
+    uint4* sk = nullptr;               // the bitmaps
+    uint32_t* pend_pivot = nullptr;    // n: one-shot runs, list work of the edges the sketches leave open
+    uint2* pend_lists = nullptr;       // slices of those pivots' tasks (one array, the task lists' order), ...
+    uint32_t* pend_counts = nullptr;   // ... their number per list, and the filter's queue counter
+    uint32_t cap_pend = 0;
+    scan::LongEdges long_edges{};
     uint32_t* cn = nullptr;        // E: common-neighbour counts (the serving cache)
     bool cn_valid = false;
     bool cn_valid_before = false;
@@ -110,20 +128,24 @@ void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E);
 // Upload a CSR (32- or 64-bit offsets), check it and build the orientation and task plan.
 // adj_in_host_memory: keep the adjacency in pinned, GPU-mapped host memory (the kernels read
 // it over the host link) instead of HBM -- the streamed mode for graphs above a device budget.
+// sketch_budget: device bytes the neighbourhood sketches may take (0: no limit); a graph
+// whose sketches need more goes without.  kNoSketches: for callers that only count in full.
+constexpr uint64_t kNoSketches = 1;
 scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_host, bool off64,
                           const uint32_t* adj_host, DeviceGraph** out, scan_stats* st,
-                          bool adj_in_host_memory = false);
+                          bool adj_in_host_memory = false, uint64_t sketch_budget = 0);
 // cn for every edge on d->stream.
-// cn for every edge; with `prune`, edges that the degree prune rules out at that eps are
-// skipped and keep cn = 0 (a one-shot run; the result is not a reusable cache).
-// With `fused` (a one-shot run whose plan splits no pivot), the kernels also run the
-// predicate: sim, sd and the run counters must be zeroed before, and launch_cluster is
-// then told so (predicate_done).
+// With `prune` (a one-shot run; the result is not a reusable cache, and run is the run's
+// scratch): edges that the degree prune rules out at that eps are skipped and keep cn = 0,
+// and where the graph has sketches they decide most of the others (run->sim holds the edge
+// states meanwhile).  When one_shot_predicate(d), the predicate is run too, into run's sim,
+// sd and counters, and launch_cluster is then told so (predicate_done).
 struct BatchParams;
-// bp (batched runs, with prune and fused): each pivot takes eps and the predicate from its
-// graph's entry of bp->gpp (prune then only supplies "on"); the one-shot fused path only.
+// bp (batched runs, with prune, no split pivot): each pivot takes eps and the predicate from
+// its graph's entry of bp->gpp (prune then only supplies "on").
 scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune = nullptr,
-                      const RunScratch* fused = nullptr, const BatchParams* bp = nullptr);
+                      const RunScratch* run = nullptr, const BatchParams* bp = nullptr);
+bool one_shot_predicate(const DeviceGraph* d);
 // Rebuild the similarity tasks for plan parameters pp.
 scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp);
 // Time the similarity stage under plan settings (small-pivot strategy and degree cut, task

@@ -193,12 +193,27 @@ struct FusedPred {
     uint8_t* sim;
     int32_t* sd;
     RunCounters* ctr;
+    const uint8_t* pend;   // after k_sketch_filter: its edge states (sim); only kEdgePending edges are counted.
+                           // Null: every edge of a task
+};
+
+// Edge states k_sketch_filter leaves in sim[]: pending, or 0 (decided: not similar).
+constexpr uint8_t kEdgePending = 2;
+
+// The part of a task list that a launch works on: order[0, *count) are slices of tasks with
+// pending edges, (index into the list, slice | slices << 16); slice i of a task takes every
+// slices-th batch of its edges from the i-th on.  Null: the whole list, tasks undivided.
+struct TaskPick {
+    const uint2* order;
+    const uint32_t* count;
+    __device__ __forceinline__ uint2 at(uint32_t t) const { return order ? order[t] : make_uint2(t, 1u << 16); }
 };
 
 // Warp-wide (holds a ballot): every lane calls it; lanes with valid set test edge k
 // {u lower, v pivot} with count t.  v is the same for every lane of the call.  decided: both
 // predicates reject the edge (pruned, or t below count_floor), so neither is evaluated.
-// sim starts zeroed, so only similar edges are written.
+// sim starts zeroed (or pending), so of the others only pending ones are written.
+template <bool kPending = true>   // false: no edge was pending (k_cn_small: its registers stay as they were)
 __device__ __forceinline__ void fused_predicate(const FusedPred& fp, const CnPrune& pr, bool valid, bool decided,
                                                 uint32_t k, uint32_t u, uint32_t v, uint32_t du, uint32_t dv,
                                                 uint32_t t, uint32_t lane, unsigned long long& nsim,
@@ -215,6 +230,7 @@ __device__ __forceinline__ void fused_predicate(const FusedPred& fp, const CnPru
             atomicAdd(&fp.sd[u], 1);
         }
     }
+    if (kPending && fp.pend && valid && !s) fp.sim[k] = 0;   // was pending
     const uint32_t nv = __popc(__ballot_sync(0xFFFFFFFFu, s));
     if (lane == 0 && nv) atomicAdd(&fp.sd[v], (int32_t)nv);
 }
@@ -529,7 +545,7 @@ k_cn_small(const uint32_t* __restrict__ pivots, uint32_t npiv, const uint32_t* _
             }
             if (vk) cn[kk] = mc;
             if (fp.sim)
-                fused_predicate(fp, P, vk, pruned || mc < count_floor(du, e - b, pt, P.eps), kk, u, v, du, e - b, mc, lane, nsim,
+                fused_predicate<false>(fp, P, vk, pruned || mc < count_floor(du, e - b, pt, P.eps), kk, u, v, du, e - b, mc, lane, nsim,
                                 ndis);
         }
         if (lane == 0 && counted) {
@@ -551,11 +567,14 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* queue, uint32_t prev, bo
     return *slot;
 }
 
+// kPick: a one-shot run after the sketches (pend and pick given); full counts keep the plain form.
+template <bool kPick>
 __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32_t* queue,
                          const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                          const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn, uint32_t long_words,
                          CnPrune pr, unsigned long long* __restrict__ ctr, uint32_t* __restrict__ miss,
-                         uint32_t nmiss, uint32_t stride) {
+                         uint32_t nmiss, uint32_t stride, const uint8_t* pend, TaskPick pick) {
+    if constexpr (kPick) ntasks = *pick.count;
     extern __shared__ __align__(16) uint32_t tab[];
     __shared__ uint32_t next_batch, task_slot;
     const uint32_t lane = threadIdx.x & 31;
@@ -565,7 +584,9 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         // stride (coprime to ntasks, 0: in order): the i-th task drawn is i * stride mod ntasks,
         // so the chunks of one split pivot, adjacent in the array, run spread over the launch
         // and the misses of the early ones can decide edges for the later ones
-        const CnTask tk = tasks[stride ? (uint32_t)((uint64_t)t * stride % ntasks) : t];
+        const uint32_t ti = stride ? (uint32_t)((uint64_t)t * stride % ntasks) : t;
+        const uint2 slice = kPick ? pick.at(ti) : make_uint2(ti, 1u << 16);
+        const CnTask tk = tasks[slice.x];
         for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x)
             reinterpret_cast<uint4*>(tab)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
         if (threadIdx.x == 0) next_batch = 0;
@@ -579,10 +600,11 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         for (;;) {
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
-            const uint32_t kb = tk.e0 + 32u * __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            const uint32_t kb = tk.e0 + 32u * (kPick ? (slice.y & 0xFFFFu) + j * (slice.y >> 16) : j);
             if (kb >= tk.e1) break;
             const uint32_t k = kb + lane;
-            const bool valid = k < tk.e1;
+            const bool valid = k < tk.e1 && (!kPick || pend[k] == kEdgePending);
             uint32_t ub = 0, ue = 0, u = 0, du = 0, tlo = 0, mi = 0xFFFFFFFFu;
             bool counted = false;
             if (valid) {
@@ -623,7 +645,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, counted));
             if (lane == 0 && (words | nc)) {
                 atomicAdd(&ctr[0], (unsigned long long)words);
-                atomicAdd(&ctr[1], (unsigned long long)nc);
+                if (!kPick) atomicAdd(&ctr[1], (unsigned long long)nc);
             }
             if (valid) {
                 if (!tk.chunked) {
@@ -729,7 +751,8 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
                             uint32_t* queue, const uint32_t* __restrict__ off,
                             const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
                             uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided) {
+                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
+    if (pick.count) ntasks = *pick.count;
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t log2bits = filter_log2bits(list_entries);
     const uint32_t nwords = (1u << log2bits) >> 5;
@@ -740,7 +763,8 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
     unsigned long long nsim = 0, ndis = 0;
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
-        const CnTask tk = tasks[t];
+        const uint2 slice = pick.at(t);
+        const CnTask tk = tasks[slice.x];
         CnPrune Pg;
         if constexpr (kPerGraph) Pg = prune_of_graph(pr, tk.v);
         const CnPrune& P = kPerGraph ? Pg : pr;
@@ -761,10 +785,10 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
             const uint32_t nbatch = (tk.e1 - tk.e0 + 31u) >> 5;
-            const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            const uint32_t j = (slice.y & 0xFFFFu) + __shfl_sync(0xFFFFFFFFu, bidx, 0) * (slice.y >> 16);
             if (j >= nbatch) break;
             const uint32_t k = strided ? tk.e0 + j + lane * nbatch : tk.e0 + 32u * j + lane;
-            const bool valid = k < tk.e1;
+            const bool valid = k < tk.e1 && (!fp.pend || fp.pend[k] == kEdgePending);
             uint32_t ub = 0, ue = 0, u = 0, du = 0, tlo = 0;
             bool pruned = false;
             if (valid) {
@@ -795,9 +819,9 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
             if (lane == 0 && (words | nc)) {
                 atomicAdd(&ctr[0], (unsigned long long)words);
-                atomicAdd(&ctr[1], (unsigned long long)nc);
+                if (!fp.pend) atomicAdd(&ctr[1], (unsigned long long)nc);
             }
-            if (valid) cn[k] = cnt;
+            if (valid && !fp.pend) cn[k] = cnt;
             fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, dv, cnt, lane, nsim, ndis);
         }
         __syncthreads();
@@ -811,9 +835,9 @@ __global__ void __launch_bounds__(512, 3) k_cn_filter_classes(const CnTask* __re
                             uint32_t* queue, const uint32_t* __restrict__ off,
                             const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
                             uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided) {
+                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
     cn_filter_body<kPerGraph, kWordsInFlight>(tasks, ntasks, list_entries, queue, off, adj, lo_adj, cn, long_words, pr, ctr, fp,
-                              strided);
+                              strided, pick);
 }
 
 template <bool kPerGraph>
@@ -821,9 +845,9 @@ __global__ void k_cn_filter(const CnTask* __restrict__ tasks, uint32_t ntasks, u
                             uint32_t* queue, const uint32_t* __restrict__ off,
                             const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
                             uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided) {
+                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
     cn_filter_body<kPerGraph, kWordsInFlightMidHub>(tasks, ntasks, list_entries, queue, off, adj, lo_adj, cn, long_words, pr, ctr, fp,
-                              strided);
+                              strided, pick);
 }
 
 // Bitmap path: one CTA of kBitmapThreads per task (pivot, edge slice), one CTA per SM.
@@ -850,12 +874,17 @@ __device__ __forceinline__ uint32_t bitmap_probe_word(const uint4 x, uint32_t p,
 }
 
 // task.cb carries the pivot's tail size.
-template <bool kPerGraph>
+// kPick: as in k_cn_big.
+template <bool kPerGraph, bool kPick>
 __global__ void __launch_bounds__(kBitmapThreads, 1)
 k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, const uint32_t* __restrict__ off,
             const uint32_t* __restrict__ radj, const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn,
             uint32_t long_words, CnPrune pr, unsigned long long* __restrict__ ctr, FusedPred fp,
-            uint32_t strided) {
+            uint32_t strided, TaskPick pick) {
+    if constexpr (kPick) {
+        ntasks = *pick.count;
+        if (ntasks == 0) return;
+    }
     extern __shared__ __align__(16) uint32_t smem[];
     uint32_t* bits = smem;                              // kHotBits / 32 words
     uint32_t* tail = smem + kHotBits / 32;              // kTailSlots words
@@ -866,7 +895,8 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
         reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
-        const CnTask tk = tasks[t];
+        const uint2 slice = kPick ? pick.at(t) : make_uint2(t, 1u << 16);
+        const CnTask tk = tasks[slice.x];
         CnPrune Pg;
         if constexpr (kPerGraph) Pg = prune_of_graph(pr, tk.v);
         const CnPrune& P = kPerGraph ? Pg : pr;
@@ -889,12 +919,13 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
             const uint32_t nbatch = (tk.e1 - tk.e0 + 31u) >> 5;
-            const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            const uint32_t b = __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            const uint32_t j = kPick ? (slice.y & 0xFFFFu) + b * (slice.y >> 16) : b;
             if (j >= nbatch) break;
             // one-shot runs: strided, as k_cn_filter's hub launch; full counts (every edge
             // counted, no pruned majority): contiguous, measured faster
             const uint32_t k = strided ? tk.e0 + j + lane * nbatch : tk.e0 + 32u * j + lane;
-            const bool valid = k < tk.e1;
+            const bool valid = k < tk.e1 && (!kPick || fp.pend[k] == kEdgePending);
             uint32_t ub = 0, ue = 0, u = 0, du = 0;
             bool pruned = false;
             if (valid) {
@@ -915,9 +946,9 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
             if (lane == 0 && (words | nc)) {
                 atomicAdd(&ctr[0], (unsigned long long)words);
-                atomicAdd(&ctr[1], (unsigned long long)nc);
+                if (!kPick) atomicAdd(&ctr[1], (unsigned long long)nc);
             }
-            if (valid) cn[k] = cnt;
+            if (valid && (!kPick || !fp.sim)) cn[k] = cnt;
             if (fp.sim) fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, ve - vb, cnt, lane, nsim, ndis);
         }
         __syncthreads();

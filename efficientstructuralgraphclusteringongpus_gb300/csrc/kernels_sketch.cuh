@@ -1,0 +1,796 @@
+// Neighbourhood sketches: an upper bound on every edge's common-neighbour count from two
+// short bitmaps, before any neighbour list is read.
+//
+// A vertex of degree d >= 2 keeps its neighbours hashed into a bitmap of 2^L bits, L the
+// least with 2^L >= kSketchBits * d (at least 2^7, at most 2^20), and every fold of that
+// bitmap down to 2^7 bits: the fold of 2^l bits is the lower half OR the upper half of the
+// one of 2^(l+1), which is the bitmap the same hash gives with l bits.  So two vertices can
+// be compared at any size both have.  A bit set for u and clear for v is a neighbour of u
+// that v does not have, and distinct bits are distinct neighbours, so
+//     |N(u) & N(v)| <= d_u - popcount(bits_u & ~bits_v).
+// An edge whose count must reach tlo (count_floor) is decided, not similar, once more than
+// d_u - tlo such bits are seen; the rest are left to the list kernels (kernels_cn.cuh).
+//
+// Layout: the bitmaps of a vertex form a heap in 16-byte units: the fold of 2^l bits starts
+// 2^(l-7) units after the vertex's base and is 2^(l-7) units long, 2^(L-6) units in all (the
+// first is unused).  Bases are assigned by size class, largest first, so each heap is aligned
+// to its own size and a group of lanes reads whole 128-byte lines.  About as many bytes as
+// the adjacency itself (R-MAT s22: 523 MB against 513).
+#pragma once
+
+#include "device_common.cuh"
+#include "device_graph.h"
+#include "kernels_cn.cuh"
+
+namespace scan {
+
+constexpr uint32_t kSketchBits = 12;      // bits per neighbour, rounded up to a power of two
+constexpr int kSketchMinLog = 7;          // one 16-byte unit
+constexpr int kSketchMaxLog = 20;         // 128 KB: larger hubs share bits
+constexpr int kSketchClasses = kSketchMaxLog - kSketchMinLog + 1;
+constexpr int kSketchMidLog = 17;         // classes up to here are built by small CTAs, larger by whole-SM ones
+constexpr int kSketchWarpLog = 13;        // classes up to here are built by one warp
+
+// log2 of the bitmap size of a vertex of degree d >= 1.
+__host__ __device__ __forceinline__ int sketch_log(uint32_t d) {
+    if (d <= (1u << kSketchMinLog) / kSketchBits) return kSketchMinLog;
+    if (d >= (1u << kSketchMaxLog) / kSketchBits) return kSketchMaxLog;
+    const uint32_t x = kSketchBits * d - 1u;      // ceil(log2(x + 1)), x >= 127
+#ifdef __CUDA_ARCH__
+    return 32 - __clz(x);
+#else
+    return 32 - __builtin_clz(x);
+#endif
+}
+
+// Bit of neighbour w in a bitmap of 2^l bits: the low l bits.  The reversal puts the product's
+// well-mixed high bits lowest.
+__device__ __forceinline__ uint32_t sketch_hash(uint32_t w) { return __brev(w * 0x9E3779B1u); }
+
+// cls[c] = vertices of size class c (degree >= 2).
+__global__ void k_sketch_classes(uint32_t n, const uint32_t* __restrict__ off, uint32_t* __restrict__ cls) {
+    __shared__ uint32_t h[kSketchClasses];
+    if (threadIdx.x < kSketchClasses) h[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint64_t v0 = blockIdx.x * (uint64_t)blockDim.x; v0 < n; v0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = v0 + threadIdx.x;
+        const uint32_t d = v < n ? off[v + 1] - off[v] : 0u;
+        const int c = d >= 2 ? sketch_log(d) - kSketchMinLog : -1;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, c);
+        if (c >= 0 && (__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&h[c], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    if (threadIdx.x < kSketchClasses && h[threadIdx.x]) atomicAdd(&cls[threadIdx.x], h[threadIdx.x]);
+}
+
+// First unit of each class and the lists of the vertices that CTAs build.
+struct SketchPlan {
+    uint32_t base[kSketchClasses];    // first 16-byte unit of the class
+    uint32_t list_mid, list_hub;      // entries of the two lists
+};
+
+// info[v] = (first unit of v's heap, degree).  rank: one counter per class, then the mid and
+// hub list counters, all zero.  The order within a class is whatever the atomics give; nothing
+// depends on it.
+__global__ void k_sketch_assign(uint32_t n, const uint32_t* __restrict__ off, SketchPlan plan,
+                                uint32_t* __restrict__ rank, uint2* __restrict__ info, uint32_t* __restrict__ mid,
+                                uint32_t* __restrict__ hub) {
+    __shared__ uint32_t h[kSketchClasses], base[kSketchClasses];
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t v0 = blockIdx.x * (uint64_t)blockDim.x; v0 < n; v0 += (uint64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x < kSketchClasses) h[threadIdx.x] = 0;
+        __syncthreads();
+        const uint64_t v = v0 + threadIdx.x;
+        const uint32_t d = v < n ? off[v + 1] - off[v] : 0u;
+        const int c = d >= 2 ? sketch_log(d) - kSketchMinLog : -1;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, c);
+        const int lead = __ffs(peers) - 1;
+        uint32_t r = 0;
+        if (c >= 0 && lead == (int)lane) r = atomicAdd(&h[c], (uint32_t)__popc(peers));
+        r = __shfl_sync(0xFFFFFFFFu, r, lead) + __popc(peers & ((1u << lane) - 1u));
+        __syncthreads();
+        if (threadIdx.x < kSketchClasses)
+            base[threadIdx.x] = h[threadIdx.x] ? atomicAdd(&rank[threadIdx.x], h[threadIdx.x]) : 0u;
+        __syncthreads();
+        if (v < n) {
+            uint32_t unit = 0;
+            if (c >= 0) {
+                unit = plan.base[c] + ((base[c] + r) << (c + 1));
+                const int l = c + kSketchMinLog;
+                if (l > kSketchMidLog) {
+                    const uint32_t i = atomicAdd(&rank[kSketchClasses + 1], 1u);
+                    if (i < plan.list_hub) hub[i] = (uint32_t)v;
+                } else if (l > kSketchWarpLog) {
+                    const uint32_t i = atomicAdd(&rank[kSketchClasses], 1u);
+                    if (i < plan.list_mid) mid[i] = (uint32_t)v;
+                }
+            }
+            info[v] = make_uint2(unit, d);
+        }
+    }
+}
+
+// Vertices of the classes up to kSketchWarpLog, 32 per warp: those of the smallest class one
+// per lane (four words in registers), the others one after the other by the whole warp in
+// shared memory.
+constexpr int kSketchWarps = 8;
+__global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32_t n, const uint32_t* __restrict__ off,
+                                                                          const uint32_t* __restrict__ adj,
+                                                                          const uint2* __restrict__ info,
+                                                                          uint4* __restrict__ sk) {
+    __shared__ __align__(16) uint32_t smem[kSketchWarps][(1u << kSketchWarpLog) / 32];
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    uint32_t* bits = smem[wib];
+    uint4* bits4 = reinterpret_cast<uint4*>(bits);
+    const uint64_t step = (uint64_t)gridDim.x * kSketchWarps * 32;
+    for (uint64_t v0 = ((uint64_t)blockIdx.x * kSketchWarps + wib) * 32; v0 < n; v0 += step) {
+        const uint64_t v = v0 + lane;
+        const uint2 iv = v < n ? info[v] : make_uint2(0, 0);
+        const uint32_t b = v < n ? off[v] : 0u;
+        const int l = iv.y >= 2 ? sketch_log(iv.y) : 0;
+        if (l == kSketchMinLog) {
+            uint4 q = make_uint4(0, 0, 0, 0);
+            for (uint32_t j = 0; j < iv.y; ++j) {
+                const uint32_t h = sketch_hash(adj[b + j]) & 127u, bit = 1u << (h & 31u), w = h >> 5;
+                if (w == 0) q.x |= bit; else if (w == 1) q.y |= bit; else if (w == 2) q.z |= bit; else q.w |= bit;
+            }
+            sk[(uint64_t)iv.x + 1] = q;
+        }
+        uint32_t todo = __ballot_sync(0xFFFFFFFFu, l > kSketchMinLog && l <= kSketchWarpLog);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t d = __shfl_sync(0xFFFFFFFFu, iv.y, j), a = __shfl_sync(0xFFFFFFFFu, b, j);
+            const uint64_t unit = __shfl_sync(0xFFFFFFFFu, iv.x, j);
+            const int lj = __shfl_sync(0xFFFFFFFFu, l, j);
+            const uint32_t units = 1u << (lj - kSketchMinLog), mask = (1u << lj) - 1u;
+            for (uint32_t i = lane; i < units; i += 32) bits4[i] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            for (uint32_t i = lane; i < d; i += 32) {
+                const uint32_t h = sketch_hash(__ldg(adj + a + i)) & mask;
+                atomicOr(&bits[h >> 5], 1u << (h & 31u));
+            }
+            __syncwarp();
+            for (uint32_t i = lane; i < units; i += 32) sk[unit + units + i] = bits4[i];
+            for (uint32_t half = units >> 1; half; half >>= 1) {   // folds, in place
+                __syncwarp();
+                for (uint32_t i = lane; i < half; i += 32) {
+                    uint4 x = bits4[i];
+                    const uint4 y = bits4[i + half];
+                    x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
+                    bits4[i] = x;
+                    sk[unit + half + i] = x;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// The larger classes: one CTA per vertex of a list, the bitmap in dynamic shared memory.
+__global__ void k_sketch_build_cta(const uint32_t* __restrict__ list, uint32_t count, const uint32_t* __restrict__ off,
+                                   const uint32_t* __restrict__ adj, const uint2* __restrict__ info,
+                                   uint4* __restrict__ sk) {
+    extern __shared__ __align__(16) uint32_t sketch_smem[];
+    uint32_t* bits = sketch_smem;
+    uint4* bits4 = reinterpret_cast<uint4*>(bits);
+    for (uint32_t t = blockIdx.x; t < count; t += gridDim.x) {
+        const uint32_t v = list[t];
+        const uint2 iv = info[v];
+        const uint32_t b = off[v];
+        const int l = sketch_log(iv.y);
+        const uint32_t units = 1u << (l - kSketchMinLog), mask = (1u << l) - 1u;
+        for (uint32_t i = threadIdx.x; i < units; i += blockDim.x) bits4[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < iv.y; i += blockDim.x) {
+            const uint32_t h = sketch_hash(__ldg(adj + b + i)) & mask;
+            atomicOr(&bits[h >> 5], 1u << (h & 31u));
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < units; i += blockDim.x) sk[(uint64_t)iv.x + units + i] = bits4[i];
+        for (uint32_t half = units >> 1; half; half >>= 1) {
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
+                uint4 x = bits4[i];
+                const uint4 y = bits4[i + half];
+                x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
+                bits4[i] = x;
+                sk[(uint64_t)iv.x + half + i] = x;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---- the bound ------------------------------------------------------------------------------
+
+// Bitmap size to try first for an edge that needs `need` missing bits: the expected number of
+// bits of u that v lacks, were their lists unrelated, is about d_u exp(-(d_u / 2 + d_v) / 2^l)
+// (bits shared within u's list, and bits v has by chance); the least l at which that is
+// need / kSketchMargin.  0: even u's largest bitmap cannot be expected to decide the edge.
+// Only speed depends on this choice.
+constexpr float kSketchMargin = 0.9f;      // first try (R-MAT, SBM, power laws: 0.8-0.95 read about the same bytes)
+constexpr float kSketchLimit = 0.97f;      // whether to try at all
+__device__ __forceinline__ int sketch_level(uint32_t du, uint32_t dv, uint32_t need, int top) {
+    const float num = 0.5f * (float)du + (float)dv, inv = (float)du / (float)need;
+    const float g = __logf(kSketchMargin * inv);
+    const float cap = (float)(1u << top);
+    if (g <= 0.f || num > g * cap) return num < __logf(kSketchLimit * inv) * cap ? top : 0;
+    const uint32_t bits = (uint32_t)__fdividef(num, g);      // < 2^top
+    const int l = 32 - __clz(bits | ((1u << kSketchMinLog) - 1u));
+    return min(max(l, kSketchMinLog), top);
+}
+
+struct SketchSlot {      // one edge of a warp's batch that needs its bitmaps
+    uint32_t bu, bv;     // first units of the two heaps
+    uint32_t need;       // missing bits that decide it
+    uint32_t code;       // edge within the batch | level << 8 | top level << 16
+};
+__device__ __forceinline__ uint32_t slot_level(const SketchSlot& s) { return (s.code >> 8) & 0xFFu; }
+__device__ __forceinline__ uint32_t slot_top(const SketchSlot& s) { return (s.code >> 16) & 0xFFu; }
+
+__device__ __forceinline__ uint32_t missing_bits(const uint4 x, const uint4 y) {
+    return __popc(x.x & ~y.x) + __popc(x.y & ~y.y) + __popc(x.z & ~y.z) + __popc(x.w & ~y.w);
+}
+
+// Warps take `chunk` consecutive edges at a time from *queue and work through them in batches
+// of kSketchBatch.  Lane i reads edge i's endpoints and their (base, degree) pairs, prunes it
+// by the degrees and picks a bitmap size for what is left.  By that size:
+//   * up to kSketchLaneLog: one edge per lane, its few units read by that lane;
+//   * up to kSketchGroupLog: groups of G lanes take one edge each, compare G * U units at a
+//     time until it is decided, and move on to the next;
+//   * larger: the list of k_sketch_long, a warp per edge.  A hub's edges of this kind sit
+//     together in its list (low ids in power-law graphs), and the few warps that drew them
+//     would work on long after the others are done (power law, 57M edges: 4.35 -> 1.35 ms).
+// An edge that its size leaves undecided is tried once more at the lower endpoint's largest.
+// A pivot's bitmaps are shared by its consecutive edges and stay in L1.
+// sim[k] = kEdgePending for an edge the list kernels must count, 0 otherwise (decided: both
+// predicates reject it).  The pending work of pivots above small_deg goes to pivot[v] and, in
+// all, *total (see pending_work).
+// ctr[0] += units read of the lower endpoints' bitmaps, ctr[1] += edges not pruned.
+constexpr int kSketchBatch = 128;
+// Groups of 4 lanes x 4 units: R-MAT s20 / s22 0.39 / 1.85 ms against 0.41 / 1.95 with 4 x 2,
+// 0.47 / 2.42 against 0.51 / 2.64 (8 x 2) and 0.50 / 2.77 (2 x 4) before edges went to lanes.
+constexpr int kSketchGroup = 4, kSketchUnroll = 4;
+constexpr uint32_t kSketchLaneLog = 10;    // 8 units
+constexpr uint32_t kSketchGroupLog = 15;   // 256 units
+
+// List work of a pending edge: 1 + d_u / 64, so that a pivot's sum (at most its degree plus a
+// 64th of the adjacency) stays below 2^32.
+__device__ __forceinline__ uint32_t pending_work(uint32_t du) { return 1u + (du >> 6); }
+
+struct PendingWork {
+    uint32_t* pivot;                // n, zeroed: pending work per pivot above small_deg
+    unsigned long long* total;
+    uint32_t small_deg;
+};
+
+// Edge k found undecided after its bitmaps were read.
+__device__ __forceinline__ uint32_t edge_pending(uint8_t* sim, const PendingWork& pw,
+                                                 const uint32_t* __restrict__ lo_adj,
+                                                 const uint32_t* __restrict__ lo_src, const uint2* __restrict__ info,
+                                                 uint64_t k) {
+    sim[k] = kEdgePending;
+    const uint32_t v = lo_src[k];
+    if (info[v].y <= pw.small_deg) return 0;
+    const uint32_t w = pending_work(info[lo_adj[k]].y);
+    atomicAdd(&pw.pivot[v], w);
+    return w;
+}
+
+template <bool kPerGraph>
+__global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                                       const uint32_t* __restrict__ lo_src,
+                                                       const uint2* __restrict__ info, const uint4* __restrict__ sk,
+                                                       CnPrune pr, uint32_t chunk, uint32_t* queue,
+                                                       uint8_t* __restrict__ sim, PendingWork pw, LongEdges ll,
+                                                       unsigned long long* __restrict__ ctr) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    constexpr int G = kSketchGroup, U = kSketchUnroll;
+    constexpr uint32_t kGroups = 32 / G, kStep = G * U;
+    static_assert(kStep <= (2u << (kSketchLaneLog - kSketchMinLog)), "a group step must not exceed its smallest bitmap");
+    __shared__ SketchSlot slots[8][kSketchBatch];
+    const uint32_t lane = threadIdx.x & 31, gl = lane % G, gi = lane / G;
+    const uint32_t lower = (1u << lane) - 1u;
+    SketchSlot* slot = slots[threadIdx.x >> 5];
+    const uint64_t nchunks = (E + chunk - 1) / chunk;
+    uint32_t words = 0, counted = 0, pending = 0;
+    // A long edge for k_sketch_long; false when the list is full.
+    auto defer = [&](const SketchSlot& s, uint64_t k, uint32_t at) {
+        if (at >= ll.cap) return false;
+        ll.slot[at] = make_uint4(s.bu, s.bv, s.need, s.code);
+        ll.edge[at] = (uint32_t)k;
+        return true;
+    };
+    for (;;) {
+        uint32_t c = 0;
+        if (lane == 0) c = atomicAdd(queue, 1u);
+        c = __shfl_sync(kFull, c, 0);
+        if (c >= nchunks) break;
+        const uint64_t kend = min((uint64_t)E, (uint64_t)(c + 1ull) * chunk);
+        for (uint64_t kb = (uint64_t)c * chunk; kb < kend; kb += kSketchBatch) {
+            uint32_t groups = 0, lanes = 0;   // slots for the groups from the front, for the lanes from the back
+#pragma unroll
+            for (int q = 0; q < kSketchBatch / 32; ++q) {
+                const uint64_t k = kb + 32 * q + lane;
+                uint32_t l = 0;               // bitmap size, 0: none needed
+                SketchSlot s{0, 0, 0, 0};
+                if (k < kend) {
+                    const uint32_t u = __ldcs(lo_adj + k), v = __ldcs(lo_src + k);
+                    const uint2 iu = info[u], iv = info[v];
+                    float floor2 = pr.eps2_floor;
+                    double eps = pr.eps;
+                    if constexpr (kPerGraph) {
+                        const PredParams* g = pr.gpp + pr.vgid[v];
+                        floor2 = g->eps2_floor;
+                        eps = g->eps;
+                    }
+                    PivotTests pt;
+                    pt.np = 0;
+                    pt.tscale = floor2 * (float)(iv.y + 1u);
+                    uint8_t state = 0;
+                    // A margin above the float roundings: at or below it both predicates' degree
+                    // prune holds in exact arithmetic; an edge it misses only reads its bitmaps.
+                    if ((float)(iu.y + 1u) >= pt.tscale * 0.999999f) {
+                        ++counted;
+                        const uint32_t tlo = count_floor(iu.y, iv.y, pt, eps);
+                        if (tlo == 0) {
+                            state = kEdgePending;              // any count may be similar
+                        } else if (tlo <= iu.y) {
+                            const int top = sketch_log(iu.y);
+                            s.need = iu.y - tlo + 1;
+                            if (iu.y >= 2) l = sketch_level(iu.y, iv.y, s.need, top);
+                            if (l == 0) state = kEdgePending;
+                            s.bu = iu.x;
+                            s.bv = iv.x;
+                            s.code = (32 * q + lane) | l << 8 | (uint32_t)top << 16;
+                        }
+                    }
+                    sim[k] = state;
+                    if (state && iv.y > pw.small_deg) {
+                        const uint32_t w = pending_work(iu.y);
+                        atomicAdd(&pw.pivot[v], w);
+                        pending += w;
+                    }
+                }
+                const uint32_t large = __ballot_sync(kFull, l > kSketchGroupLog);
+                bool deferred = false;
+                if (large) {
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(ll.count, __popc(large));
+                    at = __shfl_sync(kFull, at, 0);
+                    if (l > kSketchGroupLog) deferred = defer(s, k, at + __popc(large & lower));
+                }
+                const bool by_lane = l > 0 && l <= kSketchLaneLog, by_group = l > kSketchLaneLog && !deferred;
+                const uint32_t ml = __ballot_sync(kFull, by_lane), mg = __ballot_sync(kFull, by_group);
+                if (by_lane) slot[kSketchBatch - 1 - lanes - __popc(ml & lower)] = s;
+                if (by_group) slot[groups + __popc(mg & lower)] = s;
+                lanes += __popc(ml);
+                groups += __popc(mg);
+            }
+            __syncwarp();
+            for (uint32_t i = lane; i < lanes; i += 32) {
+                const SketchSlot s = slot[kSketchBatch - 1 - i];
+                uint32_t l = slot_level(s);
+                const uint32_t top = slot_top(s);
+                for (;;) {
+                    const uint32_t units = 1u << (l - kSketchMinLog);
+                    const uint4* pu = sk + ((uint64_t)s.bu + units);
+                    const uint4* pv = sk + ((uint64_t)s.bv + units);
+                    uint32_t miss = 0, pos = 0;
+                    do {
+                        const bool two = units > 1;
+                        const uint4 x0 = __ldg(pu + pos), y0 = __ldg(pv + pos);
+                        uint4 x1 = make_uint4(0, 0, 0, 0), y1 = x1;
+                        if (two) {
+                            x1 = __ldg(pu + pos + 1);
+                            y1 = __ldg(pv + pos + 1);
+                        }
+                        miss += missing_bits(x0, y0) + missing_bits(x1, y1);
+                        pos += 2;
+                    } while (pos < units && miss < s.need);
+                    words += min(pos, units);
+                    if (miss >= s.need) break;
+                    if (l == top) {
+                        pending += edge_pending(sim, pw, lo_adj, lo_src, info, kb + (s.code & 0xFFu));
+                        break;
+                    }
+                    l = top;
+                }
+            }
+            if (groups) {
+                uint32_t mine = gi, next = kGroups;        // slot of this group, first slot not taken
+                bool on = mine < groups;
+                SketchSlot s{0, 0, 0, 0};
+                const uint4 *pu = sk, *pv = sk;            // a group without an edge reads unit 0 on
+                uint32_t left = 0, miss = 0;               // units left at this size
+                auto open = [&]() {
+                    left = 1u << (slot_level(s) - kSketchMinLog);
+                    pu = sk + ((uint64_t)s.bu + left + gl);
+                    pv = sk + ((uint64_t)s.bv + left + gl);
+                    miss = 0;
+                };
+                if (on) {
+                    s = slot[mine];
+                    open();
+                }
+                for (;;) {
+                    uint32_t m = 0;
+                    if (on) {
+                        uint4 x[U], y[U];
+#pragma unroll
+                        for (int q = 0; q < U; ++q) {
+                            x[q] = __ldg(pu + q * G);
+                            y[q] = __ldg(pv + q * G);
+                        }
+#pragma unroll
+                        for (int q = 0; q < U; ++q) m += missing_bits(x[q], y[q]);
+                    }
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) m += __shfl_xor_sync(kFull, m, o);
+                    pu += kStep;
+                    pv += kStep;
+                    left -= kStep;
+                    miss += m;
+                    bool done = on && (miss >= s.need || left == 0);
+                    if (!__any_sync(kFull, done)) continue;
+                    if (done) {
+                        if (gl == 0) words += (1u << (slot_level(s) - kSketchMinLog)) - left;
+                        if (miss < s.need) {
+                            const uint64_t k = kb + (s.code & 0xFFu);
+                            if (slot_level(s) < slot_top(s)) {     // the size chosen was too coarse: the largest
+                                s.code = (s.code & ~0xFF00u) | slot_top(s) << 8;
+                                bool deferred = false;
+                                if (slot_top(s) > kSketchGroupLog) {
+                                    if (gl == 0) deferred = defer(s, k, atomicAdd(ll.count, 1u));
+                                    deferred = __shfl_sync(((1u << G) - 1u) << (gi * G), deferred, gi * G);
+                                }
+                                if (!deferred) {
+                                    open();
+                                    done = false;
+                                }
+                            } else if (gl == 0) {
+                                pending += edge_pending(sim, pw, lo_adj, lo_src, info, k);
+                            }
+                        }
+                    }
+                    // groups that finished take the next slots in group order
+                    const uint32_t freed = __ballot_sync(kFull, done && gl == 0);
+                    if (done) {
+                        mine = next + __popc(freed & ((1u << (gi * G)) - 1u));
+                        on = mine < groups;
+                        if (on) {
+                            s = slot[mine];
+                            open();
+                        }
+                    }
+                    next += __popc(freed);
+                    if (!__any_sync(kFull, on)) break;
+                }
+            }
+            __syncwarp();                                  // slots are rewritten by the next batch
+        }
+    }
+    words = __reduce_add_sync(kFull, words);
+    counted = __reduce_add_sync(kFull, counted);
+    pending = __reduce_add_sync(kFull, pending);
+    if (lane == 0 && (words | counted)) {
+        atomicAdd(&ctr[0], (unsigned long long)words);
+        atomicAdd(&ctr[1], (unsigned long long)counted);
+        if (pending) atomicAdd(pw.total, (unsigned long long)pending);
+    }
+}
+
+// The long edges, one per warp, 128 units at a time; a CTA's warps take consecutive ones,
+// which mostly share their pivot and so its bitmaps in L1.
+__global__ void __launch_bounds__(256) k_sketch_long(LongEdges ll, const uint32_t* __restrict__ lo_adj,
+                                                     const uint32_t* __restrict__ lo_src,
+                                                     const uint2* __restrict__ info, const uint4* __restrict__ sk,
+                                                     uint8_t* __restrict__ sim, PendingWork pw,
+                                                     unsigned long long* __restrict__ ctr) {
+    static_assert(kSketchGroupLog + 1 - kSketchMinLog >= 7, "a long edge has whole steps of 128 units");
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t count = min(*ll.count, ll.cap);
+    uint32_t words = 0, pending = 0;
+    const uint32_t step = gridDim.x * (blockDim.x >> 5);
+    for (uint64_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < count; i += step) {
+        const uint4 e = ll.slot[i];
+        const SketchSlot s{e.x, e.y, e.z, e.w};
+        for (uint32_t level = slot_level(s);; level = slot_top(s)) {
+            const uint32_t units = 1u << (level - kSketchMinLog);
+            const uint4* pu = sk + ((uint64_t)s.bu + units + lane);
+            const uint4* pv = sk + ((uint64_t)s.bv + units + lane);
+            uint32_t miss = 0, left = units;
+            do {
+                uint4 x[4], y[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    x[q] = __ldg(pu + 32 * q);
+                    y[q] = __ldg(pv + 32 * q);
+                }
+                uint32_t m = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) m += missing_bits(x[q], y[q]);
+                miss += __reduce_add_sync(0xFFFFFFFFu, m);
+                pu += 128;
+                pv += 128;
+                left -= 128;
+            } while (left && miss < s.need);
+            if (lane == 0) words += units - left;
+            if (miss >= s.need) break;
+            if (level == slot_top(s)) {
+                if (lane == 0) pending += edge_pending(sim, pw, lo_adj, lo_src, info, ll.edge[i]);
+                break;
+            }
+        }
+    }
+    if (lane == 0 && words) {
+        atomicAdd(&ctr[0], (unsigned long long)words);
+        if (pending) atomicAdd(pw.total, (unsigned long long)pending);
+    }
+}
+
+// ---- pending edges of small pivots ------------------------------------------------------------
+
+// What the sketches left open, from the edge states: four edges per lane, pending ones as bits.
+__device__ __forceinline__ uint32_t pending_bits(const uint8_t* sim, uint64_t k, uint64_t E) {
+    if (k >= E) return 0;
+    // the scratch pads sim to 256 bytes; states: 0, 1, kEdgePending = 2
+    const uint32_t p = (*reinterpret_cast<const uint32_t*>(sim + k) >> 1) & 0x01010101u;
+    const uint32_t bits = (p | p >> 7 | p >> 14 | p >> 21) & 0xFu;
+    return k + 4 > E ? bits & ((1u << (uint32_t)(E - k)) - 1u) : bits;
+}
+
+// The predicate of one pending edge with count t; lanes of a warp take different edges.
+// Writes the edge's final state; the similar-degree counts are added by the caller's warp.
+__device__ __forceinline__ bool settle_edge(const CnPrune& P, uint32_t t, uint32_t du, uint32_t dv,
+                                            unsigned long long& nsim, unsigned long long& ndis) {
+    const PivotTests pt{0, P.eps2_floor * (float)(dv + 1ull)};
+    if (t < count_floor(du, dv, pt, P.eps)) return false;      // both predicates reject it
+    const bool r = ref_f64_similar(t, du, dv, P.eps), x = exact_similar(t, du, dv, P.p, P.q);
+    const bool s = P.mode ? r : x;
+    ndis += r != x;
+    nsim += s;
+    return s;
+}
+
+__device__ __forceinline__ void add_similar(int32_t* sd, bool s, uint32_t u, uint32_t v, uint32_t lane) {
+    if (s) atomicAdd(&sd[u], 1);
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, s ? v : kEmpty);
+    if (s && (__ffs(peers) - 1) == (int)lane) atomicAdd(&sd[v], __popc(peers));
+}
+
+// Pending edges whose pivot has at most small_deg neighbours, in tiles of consecutive edges, so
+// that those of one pivot come in runs.  A run of kTableRun edges and more is counted against
+// a bucketed table of the pivot's list, a shorter one by binary search in the list itself
+// (which stays in L1): either way groups of eight lanes take an edge each and read 32 entries
+// of its lower list per round.  The predicate runs afterwards with an edge per lane, so its
+// double arithmetic is not paid at an eighth of the width.
+constexpr uint32_t kTableRun = 4;
+constexpr int kSmallTile = 128;    // edges a warp takes at a time
+
+template <bool kPerGraph>
+__global__ void __launch_bounds__(256) k_cn_pending_small(uint64_t E, uint32_t small_deg,
+                                                          const uint32_t* __restrict__ lo_adj,
+                                                          const uint32_t* __restrict__ lo_src,
+                                                          const uint32_t* __restrict__ off,
+                                                          const uint32_t* __restrict__ adj, CnPrune pr,
+                                                          uint8_t* sim, int32_t* sd, RunCounters* rc,
+                                                          unsigned long long* ctr) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    __shared__ uint32_t slots[8][kSmallTile];      // edge within the tile | count << 16
+    const uint32_t lane = threadIdx.x & 31, gl = lane & 7u, gi = lane >> 3, lower = (1u << lane) - 1u;
+    __shared__ __align__(16) uint32_t tabs[8][4 * kSmallDeg];
+    uint32_t* slot = slots[threadIdx.x >> 5];
+    __shared__ uint8_t lones[8][kSmallTile];       // slots of the edges counted by search
+    uint8_t* lone = lones[threadIdx.x >> 5];
+    uint32_t* tab = tabs[threadIdx.x >> 5];
+    uint4* tab4 = reinterpret_cast<uint4*>(tab);
+    const uint64_t ntiles = (E + kSmallTile - 1) / kSmallTile;
+    const uint64_t warp0 = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    const uint64_t nwarps = gridDim.x * (uint64_t)(blockDim.x >> 5);
+    unsigned long long nsim = 0, ndis = 0;
+    uint32_t words = 0;
+    for (uint64_t tile = warp0; tile < ntiles; tile += nwarps) {
+        const uint64_t kb = tile * kSmallTile;
+        uint32_t bits = pending_bits(sim, kb + 4 * lane, E);
+        if (!__any_sync(kFull, bits)) continue;
+        uint32_t incl = __popc(bits);
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, s);
+            if ((int)lane >= s) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        for (uint32_t at = incl - __popc(bits); bits; bits &= bits - 1, ++at) slot[at] = 4 * lane + __ffs(bits) - 1;
+        __syncwarp();
+        uint32_t nlone = 0;
+        for (uint32_t at = 0; at < total; at += 32) {          // 32 slots; runs of one pivot within them
+            const bool in = at + lane < total;
+            const uint64_t k = kb + (in ? slot[at + lane] : 0u);
+            const uint32_t v = in ? lo_src[k] : kEmpty;
+            uint32_t vb = 0, dv = 0, ub = 0, ue = 0;
+            if (in) {
+                const uint32_t u = lo_adj[k];
+                vb = off[v];
+                dv = off[v + 1] - vb;
+                ub = off[u];
+                ue = off[u + 1];
+            }
+            const bool here = in && dv <= small_deg;
+            const uint32_t before = __shfl_up_sync(kFull, v, 1);
+            const uint32_t heads = __ballot_sync(kFull, lane == 0 || v != before);
+            const uint32_t head = 31 - __clz(heads & (lower << 1 | 1u));
+            const uint32_t rest = lane == 31 ? 0u : heads >> (lane + 1);
+            const uint32_t end = rest ? lane + __ffs(rest) : 32u;
+            const bool single = here && end - head < kTableRun;
+            const uint32_t ms = __ballot_sync(kFull, single);
+            if (single) lone[nlone + __popc(ms & lower)] = (uint8_t)(at + lane);
+            nlone += __popc(ms);
+            uint32_t mc = here ? 0u : 0xFFFFu;                 // 0xFFFF: not counted here
+            uint32_t runs = __ballot_sync(kFull, here && !single && head == lane);
+            while (runs) {
+                const uint32_t h = __ffs(runs) - 1;
+                runs &= runs - 1;
+                const uint32_t stop = __shfl_sync(kFull, end, h), b0 = __shfl_sync(kFull, vb, h);
+                const uint32_t d0 = __shfl_sync(kFull, dv, h);
+                for (uint32_t i = lane; i < d0; i += 32) tab4[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+                __syncwarp();
+                for (uint32_t i = lane; i < d0; i += 32) bucket_insert(tab, d0, __ldg(adj + b0 + i));
+                __syncwarp();
+                for (uint32_t j0 = h; j0 < stop; j0 += 4) {
+                    const uint32_t j = min(j0 + gi, 31u);
+                    const uint32_t b = __shfl_sync(kFull, ub, j), e = __shfl_sync(kFull, ue, j);
+                    uint32_t c = 0;
+                    if (j0 + gi < stop)
+                        for (uint32_t p = (b & ~3u) + 4 * gl; p < e; p += 32) {
+                            c += probe_word(__ldg(reinterpret_cast<const uint4*>(adj + p)), p, b, e, tab, d0);
+                            ++words;
+                        }
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+                    const uint32_t mine = __shfl_sync(kFull, c, 8 * ((lane - j0) & 3u));
+                    if (lane - j0 < 4u && lane < stop) mc = mine;
+                }
+                __syncwarp();                                  // the table is rebuilt for the next run
+            }
+            if (in) slot[at + lane] |= mc << 16;
+        }
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < nlone; i0 += 4) {
+            const uint32_t i = i0 + gi;
+            uint32_t c = 0;
+            if (i < nlone) {
+                const uint64_t k = kb + slot[lone[i]];
+                const uint32_t u = lo_adj[k], v = lo_src[k];
+                const uint32_t ub = off[u], ue = off[u + 1], vb = off[v], dv = off[v + 1] - vb;
+                const uint32_t* list = adj + vb;
+                const uint32_t half = 1u << (31 - __clz(dv));
+                for (uint32_t p = (ub & ~3u) + 4 * gl; p < ue; p += 32) {
+                    const uint4 x = __ldg(reinterpret_cast<const uint4*>(adj + p));
+                    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+                    uint32_t n[4] = {0, 0, 0, 0};              // entries of the pivot known to be <= w
+                    for (uint32_t s = half; s; s >>= 1) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (n[q] + s <= dv && __ldg(list + n[q] + s - 1) <= w[q]) n[q] += s;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) c += p + q >= ub && p + q < ue && n[q] && __ldg(list + n[q] - 1) == w[q];
+                    ++words;
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+            if (i < nlone && gl == 0) slot[lone[i]] |= c << 16;
+        }
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            bool s = false;
+            uint32_t u = 0, v = 0;
+            if (i < total) {
+                const uint32_t t = slot[i] >> 16;
+                if (t != 0xFFFFu) {
+                    const uint64_t k = kb + (slot[i] & 0xFFFFu);
+                    u = lo_adj[k];
+                    v = lo_src[k];
+                    CnPrune Pg;
+                    if constexpr (kPerGraph) Pg = prune_of_graph(pr, v);
+                    const CnPrune& P = kPerGraph ? Pg : pr;
+                    s = settle_edge(P, t, off[u + 1] - off[u], off[v + 1] - off[v], nsim, ndis);
+                    sim[k] = s;
+                }
+            }
+            add_similar(sd, s, u, v, lane);
+        }
+        __syncwarp();                                          // slots are rewritten by the next tile
+    }
+    fused_totals(FusedPred{sim, sd, rc, nullptr}, lane, nsim, ndis);
+    words = __reduce_add_sync(kFull, words);
+    if (lane == 0 && words) atomicAdd(&ctr[0], (unsigned long long)words);
+}
+
+// Plans with split pivots: the list kernels leave cn[] of the pending edges, whose predicate
+// runs here (one byte per edge is read; k_predicate would read every edge, its count and both
+// degrees: 1.03 ms on a power law of 57M edges).
+__global__ void __launch_bounds__(256) k_predicate_pending(uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                                           const uint32_t* __restrict__ lo_src,
+                                                           const uint32_t* __restrict__ off,
+                                                           const uint32_t* __restrict__ cn, CnPrune pr, uint8_t* sim,
+                                                           int32_t* sd, RunCounters* rc) {
+    const uint32_t lane = threadIdx.x & 31;
+    unsigned long long nsim = 0, ndis = 0;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x * 4;
+    for (uint64_t k0 = ((uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 4; k0 < E; k0 += step) {
+        const uint64_t kb = k0 + 4 * lane;
+        uint32_t bits = pending_bits(sim, kb, E);
+        while (__any_sync(0xFFFFFFFFu, bits)) {
+            bool s = false;
+            uint32_t u = 0, v = 0;
+            if (bits) {
+                const uint64_t k = kb + __ffs(bits) - 1;
+                bits &= bits - 1;
+                u = lo_adj[k];
+                v = lo_src[k];
+                s = settle_edge(pr, cn[k], off[u + 1] - off[u], off[v + 1] - off[v], nsim, ndis);
+                sim[k] = s;
+            }
+            add_similar(sd, s, u, v, lane);
+        }
+    }
+    fused_totals(FusedPred{sim, sd, rc, nullptr}, lane, nsim, ndis);
+}
+
+// ---- pending edges of larger pivots -----------------------------------------------------------
+
+// The tasks of the plan whose pivot has a pending edge, cut into slices of about equal pending
+// work: the plan's tasks are sized for counting every edge, and a hub with a few hundred
+// pending edges would keep one CTA busy after all others are done (R-MAT s21, eps 0.2: hub
+// kernels 2.7 -> 1.2 ms).  Per task list, entries of TaskPick::order; counts[c] hash class c,
+// counts[kNumBigClasses] the larger hubs, counts[1 + kNumBigClasses] the mid hubs.
+constexpr int kPendingLists = kNumBigClasses + 2;
+constexpr uint32_t kPendingSlices = 8;        // slices aimed at per SM, over all lists
+constexpr uint32_t kPendingMinWork = 512;     // 32K list entries: a slice stages its pivot again
+struct PendingLists {
+    const CnTask* tasks[kPendingLists];
+    uint32_t count[kPendingLists];
+    uint2* out[kPendingLists];                // count + kPendingSlices per SM entries
+};
+
+__global__ void k_pending_tasks(PendingLists pl, PendingWork pw, const uint32_t* __restrict__ off,
+                                const uint32_t* __restrict__ lo_off, uint32_t slices, uint32_t* __restrict__ counts) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t even = (uint32_t)min(*pw.total / slices + 1, 0x7FFFFFFFull);
+    for (int a = 0; a < kPendingLists; ++a) {
+        const uint32_t cnt = pl.count[a];
+        for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < cnt; i0 += (uint64_t)gridDim.x * blockDim.x) {
+            const uint64_t i = i0 + threadIdx.x;
+            uint32_t n = 0;
+            if (i < cnt) {
+                const CnTask t = pl.tasks[a][i];
+                const uint32_t work = pw.pivot[t.v];
+                if (work) {
+                    const uint32_t dv = off[t.v + 1] - off[t.v], edges = lo_off[t.v + 1] - lo_off[t.v];
+                    const uint64_t mine = (uint64_t)work * (t.e1 - t.e0) / edges;        // the task's share
+                    const uint32_t aim = max(even, max(kPendingMinWork, dv / 16));       // 4 d_v entries at least
+                    n = (uint32_t)min(mine / aim + 1, (uint64_t)min((t.e1 - t.e0 + 31) / 32, 0xFFFFu));
+                    n = max(n, 1u);
+                }
+            }
+            uint32_t incl = n;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, s);
+                if (lane >= (uint32_t)s) incl += y;
+            }
+            uint32_t at = 0;
+            if (lane == 31 && incl) at = atomicAdd(&counts[a], incl);
+            at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - n;
+            for (uint32_t q = 0; q < n; ++q) pl.out[a][at + q] = make_uint2((uint32_t)i, q | n << 16);
+        }
+    }
+}
+
+}  // namespace scan

@@ -32,6 +32,7 @@
 #include "kernels_cluster.cuh"
 #include "kernels_cn.cuh"
 #include "kernels_orient.cuh"
+#include "kernels_sketch.cuh"
 
 namespace scan {
 
@@ -308,6 +309,9 @@ size_t run_scratch_bytes(uint32_t n, uint64_t E) {
            align256(4 * kMaxJumpRounds);
 }
 
+// The run counters and, after them, the round flags of a RunScratch.
+static size_t run_counter_bytes() { return align256(sizeof(RunCounters)) + 4 * kMaxJumpRounds; }
+
 // The order is relied on: role follows label, and the round flags follow the counters
 // (each padded to 256 bytes), so the serving loop copies each pair back in one transfer.
 void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E) {
@@ -402,6 +406,13 @@ scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
     SCAN_TRY(ensure(&d->hubs, &d->cap_hubs, d->nhmid + d->nbmp));   // mid hubs, then the larger hubs
     d->hmid = d->hubs;
     d->bmp = d->hubs + d->nhmid;
+    if (d->sk) {
+        uint64_t total = (uint64_t)d->nhmid + d->nbmp;
+        for (int c = 0; c < kNumBigClasses; ++c) total += d->nbig[c];
+        if (total)
+            SCAN_TRY(ensure(&d->pend_lists, &d->cap_pend,
+                            (uint32_t)(total + (uint64_t)kPendingLists * kPendingSlices * d->num_sms)));
+    }
     SCAN_CUDA(cudaMemsetAsync(counts, 0, sizeof(hc), s));
     k_plan<<<pg, 256, 0, s>>>(d->n, d->off, d->lo_off, d->work, d->tailc, pp, counts, d->small_piv, d->big[0],
                               d->big[1], d->big[2], d->bmp, d->hmid);
@@ -410,8 +421,41 @@ scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
     return SCAN_OK;
 }
 
-scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_host, bool off64,
-                          const uint32_t* adj_host, DeviceGraph** out, scan_stats* st, bool adj_in_host_memory) {
+// Graphs of fewer edges go without sketches: their list kernels finish in a few launches.
+constexpr uint64_t kSketchMinEdges = 1u << 12;
+// The same below this with no larger pivot: k_cn_small alone is one launch (a run on
+// communities of 100K edges 205 us, with sketches 216; a batch of 450K 332 and 358; a run on
+// 2M 593 and 480).
+constexpr uint64_t kSketchSmallEdges = 1u << 19;
+// Task counts per list of k_pending_tasks, then the filter's queue counter and the length of
+// the long-edge list.
+constexpr int kPendCounts = kPendingLists + 2;
+// Counters of one kind share 256 bytes, different kinds do not: with the totals and the task
+// queues in one line their atomics waited for one another (k_cn_small 0.105 -> 0.155 ms).
+constexpr int kCounterSpan = 64, kStageCounters = 3 * kCounterSpan;
+
+// Bases and bitmaps of every vertex's sketch, from the resident adjacency, on d->stream.
+static scan_status build_sketches(DeviceGraph* d, const SketchPlan& plan, uint32_t* rank, uint32_t* mid, uint32_t* hub) {
+    cudaStream_t s = d->stream;
+    k_sketch_assign<<<grid_for(d, d->n, 256), 256, 0, s>>>(d->n, d->off, plan, rank, d->sk_info, mid, hub);
+    k_sketch_build_small<<<grid_for(d, d->n, kSketchWarps * 32), kSketchWarps * 32, 0, s>>>(d->n, d->off, d->adj,
+                                                                                         d->sk_info, d->sk);
+    constexpr int kMidSmem = (1 << kSketchMidLog) / 8, kHubSmem = (1 << kSketchMaxLog) / 8;
+    if (plan.list_mid)
+        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_mid, (uint64_t)d->num_sms * 8), 256, kMidSmem, s>>>(
+            mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk);
+    if (plan.list_hub) {
+        SCAN_CUDA(cudaFuncSetAttribute(k_sketch_build_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubSmem));
+        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_hub, (uint64_t)d->num_sms), 1024, kHubSmem, s>>>(
+            hub, plan.list_hub, d->off, d->adj, d->sk_info, d->sk);
+    }
+    SCAN_CUDA(cudaGetLastError());
+    return SCAN_OK;
+}
+
+static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* off_host, bool off64,
+                               const uint32_t* adj_host, DeviceGraph** out, scan_stats* st, bool adj_in_host_memory,
+                               uint64_t sketch_budget) {
     if (n == 0 || n >= 0xFFFFFFFFull) return fail(SCAN_ERR_INVALID_ARG, "vertex count must be in [1, 2^32-1)");
     if (m >= 0xFFFFFFF0ull) return fail(SCAN_ERR_TOO_LARGE, "m >= 2^32 directed entries");
     SCAN_CUDA(cudaSetDevice(device));
@@ -454,6 +498,14 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
     } else {
         SCAN_CUDA(cudaMemcpyAsync(d->off, off_host, (n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     }
+    // Counters of the similarity stage, cleared together: list words, edges counted and pending
+    // work (64 bits each), the kernels' task queues, the pending lists.
+    static_assert(2 * kCounterSpan + kPendCounts <= kStageCounters, "similarity-stage counters");
+    uint32_t* stage = nullptr;
+    SCAN_TRY(dalloc(d.get(), &stage, kStageCounters));
+    d->cn_ctr = reinterpret_cast<unsigned long long*>(stage);
+    d->task_queue = stage + kCounterSpan;
+    d->pend_counts = stage + 2 * kCounterSpan;
     // The offsets are checked first (every later kernel indexes lists by them), with the
     // degree histogram of the hot-id assignment; both need only the offsets, so the host
     // waits for those alone.
@@ -474,10 +526,52 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
         k_deg_hist<<<grid_for(d.get(), n, 256), 256, 0, s>>>(d->n, d->off, hist);
         SCAN_CUDA(cudaMemcpyAsync(h.data(), hist, kDegBins * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     }
+    // Sketches for the one-shot runs: their size follows from the degrees.
+    uint32_t* sk_cls = nullptr;
+    std::vector<uint32_t> hcls(kSketchClasses, 0);
+    const bool want_sketch = m >= 2 * kSketchMinEdges;
+    if (want_sketch) {
+        SCAN_TRY(dalloc(d.get(), &sk_cls, 2 * kSketchClasses + 2));   // class sizes; then assignment counters
+        SCAN_CUDA(cudaMemsetAsync(sk_cls, 0, (2 * kSketchClasses + 2) * sizeof(uint32_t), s));
+        k_sketch_classes<<<grid_for(d.get(), n, 256), 256, 0, s>>>(d->n, d->off, sk_cls);
+        SCAN_CUDA(cudaMemcpyAsync(hcls.data(), sk_cls, kSketchClasses * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    }
     uint32_t bad = 0;
     SCAN_CUDA(cudaMemcpyAsync(&bad, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     SCAN_CUDA(cudaStreamSynchronize(s));
     if (bad) return fail(SCAN_ERR_FORMAT, "offsets are not a non-decreasing sequence from 0 to m");
+    SketchPlan sk_plan{};
+    uint64_t sk_units = 0;
+    uint32_t *sk_mid = nullptr, *sk_hub = nullptr;
+    bool use_sketch = want_sketch && sketch_budget != kNoSketches;
+    if (use_sketch && m < 2 * kSketchSmallEdges) {
+        use_sketch = false;
+        for (int c = sketch_log(kSmallDeg) + 1 - kSketchMinLog; c < kSketchClasses; ++c) use_sketch |= hcls[c] > 0;
+    }
+    if (use_sketch) {
+        for (int c = kSketchClasses; c-- > 0;) {   // largest heaps first: each aligned to its size
+            sk_plan.base[c] = (uint32_t)sk_units;
+            sk_units += (uint64_t)hcls[c] << (c + 1);
+            const int l = c + kSketchMinLog;
+            if (l > kSketchMidLog) sk_plan.list_hub += hcls[c];
+            else if (l > kSketchWarpLog) sk_plan.list_mid += hcls[c];
+        }
+        if (sk_units && sk_units < 0xFFFFFFF0ull && (!sketch_budget || sk_units * 16 + 13 * n <= sketch_budget)) {
+            SCAN_TRY(dalloc(d.get(), &d->sk, sk_units));
+            SCAN_TRY(dalloc(d.get(), &d->sk_info, n));
+            SCAN_TRY(dalloc(d.get(), &d->pend_pivot, n));   // 4 bytes a vertex
+            LongEdges& ll = d->long_edges;
+            ll.count = d->pend_counts + kPendCounts - 1;
+            for (int c = kSketchGroupLog + 1 - kSketchMinLog; c < kSketchClasses; ++c)
+                if (hcls[c]) ll.cap = (uint32_t)std::max<uint64_t>(m / 32, 4096);
+            if (ll.cap) {   // a sixteenth of the edges; what finds no room has a slower path
+                SCAN_TRY(dalloc(d.get(), &ll.slot, ll.cap));
+                SCAN_TRY(dalloc(d.get(), &ll.edge, ll.cap));
+            }
+            SCAN_TRY(dalloc(d.get(), &sk_mid, sk_plan.list_mid));
+            SCAN_TRY(dalloc(d.get(), &sk_hub, sk_plan.list_hub));
+        }
+    }
     uint32_t min_bin = 1;                            // isolated vertices are never hot
     if (bitmap_path) {
         uint64_t acc = 0;
@@ -585,6 +679,7 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
         k_fill_tiles<<<grid_for(d.get(), fill_tiles * kFillThreads, kFillThreads), kFillThreads, 0, s>>>(
             d->n, m, (uint32_t)d->E, d->off, d->adj, tile_v, lowbits, wpre, d->lo_adj, d->lo_src);
     }
+    if (d->sk) SCAN_TRY(build_sketches(d.get(), sk_plan, sk_cls + kSketchClasses, sk_mid, sk_hub));
     SCAN_CUDA(cudaGetLastError());
 
     // Task plan.
@@ -600,8 +695,6 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
 
     // Result and scratch arrays.
     SCAN_TRY(dalloc(d.get(), &d->cn, d->E));
-    SCAN_TRY(dalloc(d.get(), &d->cn_ctr, 2));
-    SCAN_TRY(dalloc(d.get(), &d->task_queue, 8));
     SCAN_TRY(dalloc(d.get(), &d->np_tab, kPruneTable));
     uint8_t* rs_mem = nullptr;
     SCAN_TRY(dalloc(d.get(), &rs_mem, run_scratch_bytes(d->n, d->E)));
@@ -620,12 +713,26 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
     return SCAN_OK;
 }
 
+scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_host, bool off64,
+                          const uint32_t* adj_host, DeviceGraph** out, scan_stats* st, bool adj_in_host_memory,
+                          uint64_t sketch_budget) {
+    scan_status rc = upload_once(device, n, m, off_host, off64, adj_host, out, st, adj_in_host_memory, sketch_budget);
+    // The sketches are an aid: a graph that does not fit with them is uploaded without.
+    if (rc == SCAN_ERR_OUT_OF_MEMORY && sketch_budget != kNoSketches) {
+        if (st) std::memset(st, 0, sizeof(*st));
+        clear_error();
+        rc = upload_once(device, n, m, off_host, off64, adj_host, out, st, adj_in_host_memory, kNoSketches);
+    }
+    return rc;
+}
+
 // Kernel attributes and occupancies, found once per device (so capturing launch_cn into a
 // CUDA graph queries nothing).  [g] is 1 for the instantiations with per-graph parameters.
-static bool g_attr_set[64] = {};
-static bool g_attr_bitmap[64][2] = {};
+static bool g_attr_set[64][2] = {};         // k_cn_big: [after the sketches]
+static bool g_attr_bitmap[64][2][2] = {};   // [g][after the sketches]
 static bool g_attr_filter[64][2][2] = {};   // [g][mid hubs]
-static int g_per_sm[64][kNumBigClasses] = {};               // k_cn_big, each hash class
+static int g_per_sm[64][2][kNumBigClasses] = {};            // k_cn_big, [after the sketches][hash class]
+static int g_per_sm_sketch[64][2] = {};                      // k_sketch_filter
 static int g_per_sm_hub_filter[64][2] = {};                 // k_cn_filter on the mid hubs
 static int g_per_sm_filter[64][2][kNumBigClasses][2] = {};  // k_cn_filter, [g][class][largest class 2
                                                             // at the default chunk, or at the cap]
@@ -640,15 +747,79 @@ static uint32_t spread_stride(uint32_t n) {
     return (uint32_t)st;
 }
 
+// A prime: i * kSpreadPrime mod n visits 0..n-1 once each for every n below it (the order of
+// spread_stride for a task list whose length only the device knows).
+constexpr uint32_t kSpreadPrime = 2654435761u;
+
+// Every edge of a one-shot run through the sketches: edge states to sim, pending pivots to
+// d->pend_pivot.
 template <bool kPerGraph>
-static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPrune& pr, const FusedPred& fp) {
+static scan_status launch_sketch_filter(DeviceGraph* d, uint32_t* launches, const CnPrune& pr, uint8_t* sim,
+                                        const PendingWork& pw) {
+    cudaStream_t s = d->stream;
+    // (the pivots' work is read only where there are task lists to pick from)
+    if (d->cap_pend) SCAN_CUDA(cudaMemsetAsync(d->pend_pivot, 0, d->n * sizeof(uint32_t), s));
+    if (!d->E) return SCAN_OK;
+    constexpr int kThreads = 256;
+    auto* kernel = k_sketch_filter<kPerGraph>;
+    int& per_sm = g_per_sm_sketch[d->device][kPerGraph ? 1 : 0];
+    if (per_sm == 0) {
+        SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+        per_sm = std::max(per_sm, 1);
+    }
+    // Edges a warp takes at a time: one batch, or less where that leaves warps without work.
+    const uint64_t warps = (uint64_t)d->num_sms * per_sm * (kThreads / 32);
+    const uint64_t chunk = std::min<uint64_t>(kSketchBatch, std::max<uint64_t>(32, d->E / (warps * 8) / 32 * 32));
+    const uint64_t blocks = (d->E + chunk * (kThreads / 32) - 1) / (chunk * (kThreads / 32));
+    const unsigned grid = (unsigned)std::min<uint64_t>(blocks, (uint64_t)d->num_sms * per_sm);
+    kernel<<<grid, kThreads, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->sk_info, d->sk, pr, (uint32_t)chunk,
+                                     d->pend_counts + kPendCounts - 2, sim, pw, d->long_edges, d->cn_ctr);
+    ++*launches;
+    if (d->long_edges.cap) {
+        k_sketch_long<<<d->num_sms * 6, kThreads, 0, s>>>(d->long_edges, d->lo_adj, d->lo_src, d->sk_info, d->sk, sim,
+                                                          pw, d->cn_ctr);
+        ++*launches;
+    }
+    return SCAN_OK;
+}
+
+template <bool kPerGraph, bool kPick>
+static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPrune& pr, const FusedPred& fp,
+                                  const RunScratch& run) {
     cudaStream_t s = d->stream;
     const int g = kPerGraph ? 1 : 0;
+    // The sketches first: they settle most edges, and the list kernels below then work on the
+    // tasks with a pending edge only (pick; the counts stay on the device).
+    TaskPick pick_class[kNumBigClasses] = {}, pick_bmp{}, pick_mid{};
+    if constexpr (kPick) {
+        const PendingWork pw{d->pend_pivot, d->cn_ctr + 2, d->plan.small_deg};
+        SCAN_TRY(launch_sketch_filter<kPerGraph>(d, launches, pr, const_cast<uint8_t*>(fp.pend), pw));
+        PendingLists pl{};
+        uint2* out = d->pend_lists;
+        uint32_t longest = 0;
+        auto list = [&](int a, uint32_t count, const CnTask* tasks) {
+            pl.tasks[a] = tasks;
+            pl.count[a] = count;
+            pl.out[a] = out;
+            const TaskPick pick{out, d->pend_counts + a};
+            if (count) out += count + kPendingSlices * d->num_sms;
+            longest = std::max(longest, count);
+            return pick;
+        };
+        for (int c = 0; c < kNumBigClasses; ++c) pick_class[c] = list(c, d->nbig[c], d->big[c]);
+        pick_bmp = list(kNumBigClasses, d->nbmp, d->bmp);
+        pick_mid = list(1 + kNumBigClasses, d->nhmid, d->hmid);
+        if (longest) {
+            k_pending_tasks<<<grid_for(d, longest, 256, 4), 256, 0, s>>>(pl, pw, d->off, d->lo_off,
+                                                                         kPendingSlices * d->num_sms, d->pend_counts);
+            ++*launches;
+        }
+    }
     SCAN_CUDA(cudaEventRecord(d->ev[7], s));
-    if (!g_attr_set[d->device]) {
-        SCAN_CUDA(cudaFuncSetAttribute(k_cn_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (!g_attr_set[d->device][kPick]) {
+        SCAN_CUDA(cudaFuncSetAttribute(k_cn_big<kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(big_class_slots(kNumBigClasses - 1) * sizeof(uint32_t))));
-        g_attr_set[d->device] = true;
+        g_attr_set[d->device][kPick] = true;
     }
     // One-shot fused runs (every pivot unsplit) decide most edges from an upper bound on
     // their count (k_cn_filter); full counts and split plans use the bucketed table.
@@ -666,33 +837,37 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     // another, and the CTAs of one fill the SMs that another's last tasks leave idle.  Run one
     // after the other, those tails added up (R-MAT s22 over the stage: 14.56 ms in sequence,
     // 13.3 ms on two streams; the larger hubs first: eps 0.2, mu 2 30.6 -> 29.8 ms).
-    cudaStream_t sh = d->side;
-    SCAN_CUDA(cudaEventRecord(d->fork, s));
-    SCAN_CUDA(cudaStreamWaitEvent(sh, d->fork, 0));
+    // work items of a task list: after the sketches, slices of its tasks
+    auto items = [&](uint64_t tasks) { return fp.pend ? tasks + kPendingSlices * d->num_sms : tasks; };
+    const bool hubs = d->nbmp || d->nhmid;
+    cudaStream_t sh = hubs ? d->side : s;
+    if (hubs) {
+        SCAN_CUDA(cudaEventRecord(d->fork, s));
+        SCAN_CUDA(cudaStreamWaitEvent(sh, d->fork, 0));
+    }
     // Hubs.  The mid hubs of a one-shot run go to k_cn_filter like the hash classes; the
     // larger hubs, and every hub when counting in full, to the hot-id bitmap kernel (full
     // counts: one launch over both task lists, d->hmid being followed by d->bmp in one array).
     // Hubs above kHubFilterMax stay off k_cn_filter: edges between two hubs of degree above
     // 46,339 have no early-stop threshold (the reference's int square may wrap), so the
     // filter would end in an exact recount by binary search over the whole list.
-    uint32_t nbitmap = d->nbmp;
-    const CnTask* bitmap_tasks = d->bmp;
     const bool mid_on_filter = filter && d->nhmid;
-    if (!mid_on_filter) {
-        nbitmap += d->nhmid;
-        bitmap_tasks = d->hmid;
-    }
-    if (nbitmap) {
+    // With split pivots and sketches the two hub lists are picked separately: two launches.
+    for (int part = 0; part < (mid_on_filter || !fp.pend ? 1 : 2); ++part) {
+        const bool both = !mid_on_filter && !fp.pend;
+        const uint32_t nbitmap = both ? d->nbmp + d->nhmid : part == 0 ? d->nbmp : d->nhmid;
+        const CnTask* bitmap_tasks = both || part == 1 ? d->hmid : d->bmp;
+        if (!nbitmap) continue;
         const size_t smem = (kHotBits / 32 + kTailSlots) * sizeof(uint32_t);
-        if (!g_attr_bitmap[d->device][g]) {
-            SCAN_CUDA(cudaFuncSetAttribute(k_cn_bitmap<kPerGraph>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (!g_attr_bitmap[d->device][g][kPick]) {
+            SCAN_CUDA(cudaFuncSetAttribute(k_cn_bitmap<kPerGraph, kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem));
-            g_attr_bitmap[d->device][g] = true;
+            g_attr_bitmap[d->device][g][kPick] = true;
         }
-        const uint64_t grid = std::min<uint64_t>(nbitmap, (uint64_t)d->num_sms);
-        k_cn_bitmap<kPerGraph><<<(unsigned)grid, kBitmapThreads, smem, sh>>>(
-            bitmap_tasks, nbitmap, d->task_queue + 3, d->off, d->radj, d->lo_adj, d->cn, d->long_words, pr,
-            d->cn_ctr, fp, pr.on);
+        const uint64_t grid = std::min<uint64_t>(items(nbitmap), (uint64_t)d->num_sms);
+        k_cn_bitmap<kPerGraph, kPick><<<(unsigned)grid, kBitmapThreads, smem, sh>>>(
+            bitmap_tasks, nbitmap, d->task_queue + (part == 0 ? 3 : 4), d->off, d->radj, d->lo_adj, d->cn,
+            d->long_words, pr, d->cn_ctr, fp, pr.on, part == 0 ? pick_bmp : pick_mid);
         ++*launches;
     }
     if (mid_on_filter) {
@@ -703,10 +878,10 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
             SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_filter<kPerGraph>, threads, smem));
             per_sm = std::max(per_sm, 1);
         }
-        const uint64_t grid = std::min<uint64_t>(d->nhmid, (uint64_t)d->num_sms * per_sm);
+        const uint64_t grid = std::min<uint64_t>(items(d->nhmid), (uint64_t)d->num_sms * per_sm);
         k_cn_filter<kPerGraph><<<(unsigned)grid, threads, smem, sh>>>(
             d->hmid, d->nhmid, kHubFilterMax, d->task_queue + 4, d->off, d->adj,
-            d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 1u);   // hubs: strided batches
+            d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 1u, pick_mid);   // hubs: strided batches
         ++*launches;
     }
     for (int c = kNumBigClasses - 1; c >= 0; --c) {   // longest tasks first
@@ -722,29 +897,36 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
                                                                             threads, smem));
                     per_sm = std::max(per_sm, 1);
                 }
-                const uint64_t grid = std::min<uint64_t>(d->nbig[c], (uint64_t)d->num_sms * per_sm);
+                const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
                 k_cn_filter_classes<kPerGraph><<<(unsigned)grid, threads, smem, s>>>(
                     d->big[c], d->nbig[c], entries, d->task_queue + c, d->off, d->adj,
-                    d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 0u);
+                    d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 0u, pick_class[c]);
             } else {
                 const size_t smem = big_class_slots(c) * sizeof(uint32_t);
-                int& per_sm = g_per_sm[d->device][c];
+                int& per_sm = g_per_sm[d->device][kPick][c];
                 if (per_sm == 0) {
-                    SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_big, threads, smem));
+                    SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_big<kPick>, threads, smem));
                     per_sm = std::max(per_sm, 1);
                 }
-                const uint64_t grid = std::min<uint64_t>(d->nbig[c], (uint64_t)d->num_sms * per_sm);
-                k_cn_big<<<(unsigned)grid, threads, smem, s>>>(d->big[c], d->nbig[c], big_class_slots(c),
+                const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
+                k_cn_big<kPick><<<(unsigned)grid, threads, smem, s>>>(d->big[c], d->nbig[c], big_class_slots(c),
                                                                 d->task_queue + c, d->off,
                                                                 d->adj, d->lo_adj, d->cn, d->long_words, pr,
                                                                 d->cn_ctr, pr.on ? d->miss : nullptr, d->nmiss,
-                                                                pr.on && d->nmiss ? spread_stride(d->nbig[c]) : 0u);
+                                                                !pr.on || !d->nmiss ? 0u
+                                                                : fp.pend ? kSpreadPrime : spread_stride(d->nbig[c]),
+                                                                fp.pend, pick_class[c]);
             }
             ++*launches;
         }
         SCAN_CUDA(cudaEventRecord(d->ev[9 + c], s));
     }
-    if (d->nsmall) {
+    if (d->nsmall && fp.pend) {
+        const unsigned grid = (unsigned)grid_for(d, (d->E + kSmallTile - 1) / kSmallTile * 32, 256, 8);
+        k_cn_pending_small<kPerGraph><<<grid, 256, 0, s>>>(d->E, d->plan.small_deg, d->lo_adj, d->lo_src, d->off,
+                                                           d->adj, pr, run.sim, run.sd, run.ctr, d->cn_ctr);
+        ++*launches;
+    } else if (d->nsmall) {
         constexpr int kWpb = 8;
         const unsigned grid = (unsigned)grid_for(d, (uint64_t)d->nsmall * 32, kWpb * 32, 16);
         auto launch_small = [&](auto strategy) {
@@ -758,16 +940,23 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
         ++*launches;
     }
     SCAN_CUDA(cudaEventRecord(d->ev[8], s));
-    SCAN_CUDA(cudaEventRecord(d->ev[15], sh));
-    SCAN_CUDA(cudaEventRecord(d->join, sh));
-    SCAN_CUDA(cudaStreamWaitEvent(s, d->join, 0));
+    if (hubs) {
+        SCAN_CUDA(cudaEventRecord(d->ev[15], sh));
+        SCAN_CUDA(cudaEventRecord(d->join, sh));
+        SCAN_CUDA(cudaStreamWaitEvent(s, d->join, 0));
+    }
+    if (fp.pend && !fp.sim && d->E) {   // split pivots: the pending edges' counts are complete now
+        k_predicate_pending<<<grid_for(d, (d->E + 3) / 4, 256), 256, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->off,
+                                                                               d->cn, pr, run.sim, run.sd, run.ctr);
+        ++*launches;
+    }
     SCAN_CUDA(cudaEventRecord(d->ev[12], s));
     SCAN_CUDA(cudaGetLastError());
     return SCAN_OK;
 }
 
 // cn for every edge (the similarity stage); events 7..12 bracket its kernels.
-scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune, const RunScratch* fused,
+scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune, const RunScratch* run,
                       const BatchParams* bp) {
     if (d->device < 0 || d->device >= 64) return fail(SCAN_ERR_INVALID_ARG, "device index must be < 64");
     CnPrune pr{0.0, 0, 1, 0u, 0, nullptr, nullptr, 0.0, 0.f, nullptr};
@@ -778,13 +967,19 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
         pr.gpp = bp->gpp;
         pr.vgid = bp->vgid;
     }
-    FusedPred fp{nullptr, nullptr, nullptr};
-    if (fused && prune && !d->has_split) fp = FusedPred{fused->sim, fused->sd, fused->ctr};
+    FusedPred fp{nullptr, nullptr, nullptr, nullptr};
+    const bool fused = run && prune && !d->has_split;
+    if (fused) fp = FusedPred{run->sim, run->sd, run->ctr, nullptr};
+    if (run && prune && d->sk) fp.pend = run->sim;
     if (per_graph && !fp.sim) return fail(SCAN_ERR_INVALID_ARG, "per-graph parameters need the fused one-shot path");
     cudaStream_t s = d->stream;
-    SCAN_CUDA(cudaMemsetAsync(d->cn, 0, d->E * sizeof(uint32_t), s));
-    SCAN_CUDA(cudaMemsetAsync(d->cn_ctr, 0, 2 * sizeof(unsigned long long), s));
-    SCAN_CUDA(cudaMemsetAsync(d->task_queue, 0, 8 * sizeof(uint32_t), s));
+    if (!fused || !fp.pend) SCAN_CUDA(cudaMemsetAsync(d->cn, 0, d->E * sizeof(uint32_t), s));
+    if (fused || fp.pend) {
+        if (!fp.pend) SCAN_CUDA(cudaMemsetAsync(run->sim, 0, d->E, s));
+        SCAN_CUDA(cudaMemsetAsync(run->sd, 0, d->n * sizeof(int32_t), s));
+        SCAN_CUDA(cudaMemsetAsync(run->ctr, 0, run_counter_bytes(), s));   // and the round flags
+    }
+    SCAN_CUDA(cudaMemsetAsync(d->cn_ctr, 0, kStageCounters * sizeof(uint32_t), s));
     if (prune && d->nmiss) SCAN_CUDA(cudaMemsetAsync(d->miss, 0, (size_t)d->nmiss * sizeof(uint32_t), s));
     if (prune && !per_graph) {
         k_prune_table<<<kPruneTable / 256, 256, 0, s>>>(pr, d->np_tab);
@@ -795,8 +990,18 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
         pr.np_tab = bp->np_tabs;
         ++*launches;
     }
-    return per_graph ? launch_cn_impl<true>(d, launches, pr, fp) : launch_cn_impl<false>(d, launches, pr, fp);
+    const RunScratch r = run ? *run : RunScratch{};
+    if (fp.pend)
+        return per_graph ? launch_cn_impl<true, true>(d, launches, pr, fp, r)
+                         : launch_cn_impl<false, true>(d, launches, pr, fp, r);
+    return per_graph ? launch_cn_impl<true, false>(d, launches, pr, fp, r)
+                     : launch_cn_impl<false, false>(d, launches, pr, fp, r);
 }
+
+// A one-shot launch_cn also runs the predicate: with no split pivot the counting kernels do
+// (each count is final in the lane that computes it), and after the sketches the few edges of
+// split pivots take a pass of their own.
+bool one_shot_predicate(const DeviceGraph* d) { return !d->has_split || d->sk; }
 
 // Autotuner: a coordinate search over the plan, each setting timed on this graph with
 // `stage` (the similarity stage as the caller runs it; null: full counts).  In order:
@@ -864,13 +1069,13 @@ scan_status autotune_similarity(DeviceGraph* d, float* best_ms, const std::funct
     return SCAN_OK;
 }
 
-// Main stream: ev[7] (stage start), class 2 -> ev[11], class 1 -> ev[10], class 0 -> ev[9],
+// Main stream: ev[7] (the list kernels' start, after the sketches of a one-shot run), class 2 -> ev[11], class 1 -> ev[10], class 0 -> ev[9],
 // small pivots -> ev[8]; side stream: the hubs from ev[7] to ev[15].
 static void cn_kernel_times(DeviceGraph* d, scan_stats* st) {
     st->ms_cn_kernel[0] = ev_ms(d->ev[9], d->ev[8]);
     for (int c = 0; c < kNumBigClasses; ++c)
         st->ms_cn_kernel[1 + c] = ev_ms(c == kNumBigClasses - 1 ? d->ev[7] : d->ev[10 + c], d->ev[9 + c]);
-    st->ms_cn_kernel[4] = ev_ms(d->ev[7], d->ev[15]);
+    st->ms_cn_kernel[4] = d->nbmp || d->nhmid ? ev_ms(d->ev[7], d->ev[15]) : 0.0;
     st->cn_work_items[0] = d->nsmall;
     for (int c = 0; c < kNumBigClasses; ++c) st->cn_work_items[1 + c] = d->nbig[c];
     st->cn_work_items[4] = d->nbmp + d->nhmid;
@@ -884,11 +1089,10 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     const uint32_t n = d->n;
     const int sms = d->num_sms, T = 256;
     const int ge = grid_for_n(sms, E, T), gn = grid_for_n(sms, n, T);
-    k_cluster_reset<<<gn, T, 0, s>>>(n, predicate_done ? nullptr : r.sd, predicate_done ? nullptr : r.ctr,
-                                     r.jump_flags, kMaxJumpRounds);
-    ++*launches;
     const uint32_t* vgid = bp ? bp->vgid : nullptr;
-    if (!predicate_done) {
+    if (!predicate_done) {   // a one-shot launch_cn has cleared them
+        k_cluster_reset<<<gn, T, 0, s>>>(n, r.sd, r.ctr, r.jump_flags, kMaxJumpRounds);
+        ++*launches;
         if (d->tau && !bp && d->cn_valid)
             k_predicate_tau<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, d->off, d->cn, d->tau, pp, r.sim, r.sd, r.ctr);
         else
@@ -968,17 +1172,10 @@ static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bo
     SCAN_CUDA(cudaEventRecord(d->ev[3], s));
     d->cn_valid_before = d->cn_valid;
     const bool count = !(reuse_cn && d->cn_valid);
-    // With no split pivot, the counting kernels also run the predicate (each count is final
-    // in the lane that computes it).
-    const bool fused = count && !d->has_split;
+    const bool fused = count && one_shot_predicate(d);
     if (count) {
         d->cn_valid = false;
-        if (fused) {
-            SCAN_CUDA(cudaMemsetAsync(d->rs.sim, 0, d->E, s));
-            SCAN_CUDA(cudaMemsetAsync(d->rs.sd, 0, d->n * sizeof(int32_t), s));
-            SCAN_CUDA(cudaMemsetAsync(d->rs.ctr, 0, sizeof(RunCounters), s));
-        }
-        SCAN_TRY(launch_cn(d, &launches, &pp, fused ? &d->rs : nullptr));
+        SCAN_TRY(launch_cn(d, &launches, &pp, &d->rs));
     }
     SCAN_CUDA(cudaEventRecord(d->ev[4], s));
     SCAN_TRY(launch_cluster(d, d->rs, s, pp, mu, &launches, nullptr, fused));
@@ -1049,7 +1246,17 @@ scan_status scan_graph_upload_streamed(scan_graph* g, int device, uint64_t devic
         return fail(SCAN_ERR_OUT_OF_MEMORY, "streamed graph needs about " + std::to_string(est >> 20) +
                                                 " MiB of device memory, above the budget of " +
                                                 std::to_string(device_budget_bytes >> 20) + " MiB");
-    SCAN_TRY(device_upload(device, g->n, g->m, g->off.data(), true, g->adj.data(), &g->dev, nullptr, true));
+    // What the estimate leaves of the budget may hold the sketches, but for the orientation's
+    // bit words and their prefix; a graph that then exceeds the budget goes without them.
+    const uint64_t spare = device_budget_bytes > est + g->m / 4 ? device_budget_bytes - est - g->m / 4 : kNoSketches;
+    SCAN_TRY(device_upload(device, g->n, g->m, g->off.data(), true, g->adj.data(), &g->dev, nullptr, true,
+                           device_budget_bytes ? spare : 0));
+    if (device_budget_bytes && g->dev->device_bytes > device_budget_bytes && g->dev->sk) {
+        device_graph_free(g->dev);
+        g->dev = nullptr;
+        SCAN_TRY(device_upload(device, g->n, g->m, g->off.data(), true, g->adj.data(), &g->dev, nullptr, true,
+                               kNoSketches));
+    }
     if (device_bytes_used) *device_bytes_used = g->dev->device_bytes;
     if (device_budget_bytes && g->dev->device_bytes > device_budget_bytes) {
         const uint64_t used = g->dev->device_bytes;

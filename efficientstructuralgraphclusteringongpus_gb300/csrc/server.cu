@@ -364,7 +364,8 @@ scan_status scan_server_add_graph(scan_server* s, const scan_graph* g, uint32_t*
     clear_error();
     if (!s || !g || !graph_id) return fail(SCAN_ERR_INVALID_ARG, "null argument");
     DeviceGraph* d = nullptr;
-    scan_status st = device_upload(s->device, g->n, g->m, g->off.data(), true, g->adj.data(), &d, nullptr);
+    scan_status st = device_upload(s->device, g->n, g->m, g->off.data(), true, g->adj.data(), &d, nullptr, false,
+                                   kNoSketches);
     if (st != SCAN_OK) return st;
     uint32_t launches = 0;
     st = launch_cn(d, &launches);
