@@ -249,6 +249,30 @@ __device__ __forceinline__ void fused_totals(const FusedPred& fp, uint32_t lane,
     }
 }
 
+// A CTA's totals of list words read and edges counted, kept in shared memory and added to the
+// run's once per CTA: with an atomic per batch or small pivot on the one pair of global
+// counters, those atomics were what k_cn_small waited for.
+struct CtaTotals {
+    unsigned long long words, counted;
+};
+
+__device__ __forceinline__ void totals_clear(CtaTotals* t) {   // the caller's next CTA barrier publishes it
+    if (threadIdx.x == 0) *t = CtaTotals{0, 0};
+}
+
+__device__ __forceinline__ void totals_add(CtaTotals* t, uint32_t words, uint32_t counted) {   // one lane per warp
+    if (words) atomicAdd(&t->words, (unsigned long long)words);
+    if (counted) atomicAdd(&t->counted, (unsigned long long)counted);
+}
+
+__device__ __forceinline__ void totals_flush(CtaTotals* t, unsigned long long* ctr) {   // every thread, at the end
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (t->words) atomicAdd(&ctr[0], t->words);
+        if (t->counted) atomicAdd(&ctr[1], t->counted);
+    }
+}
+
 // First position in adj[b, e) whose value is >= key (scalar, uniform across the warp).
 __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__ adj, uint32_t b, uint32_t e,
                                                     uint32_t key) {
@@ -482,6 +506,9 @@ k_cn_small(const uint32_t* __restrict__ pivots, uint32_t npiv, const uint32_t* _
            const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t* queue) {
     __shared__ uint32_t tabs[kWarpsPerBlock][kSmallSlots];
+    __shared__ CtaTotals totals;
+    totals_clear(&totals);
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint32_t* tab = tabs[wib];
     unsigned long long nsim = 0, ndis = 0;
@@ -548,13 +575,11 @@ k_cn_small(const uint32_t* __restrict__ pivots, uint32_t npiv, const uint32_t* _
                 fused_predicate<false>(fp, P, vk, pruned || mc < count_floor(du, e - b, pt, P.eps), kk, u, v, du, e - b, mc, lane, nsim,
                                 ndis);
         }
-        if (lane == 0 && counted) {
-            atomicAdd(&ctr[0], (unsigned long long)words);
-            atomicAdd(&ctr[1], (unsigned long long)counted);
-        }
+        if (lane == 0) totals_add(&totals, words, counted);
         __syncwarp();
     }
     fused_totals(fp, lane, nsim, ndis);
+    totals_flush(&totals, ctr);
 }
 
 // Next task of a persistent CTA: from the launch's queue counter (dynamic: a CTA that drew
@@ -577,6 +602,8 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
     if constexpr (kPick) ntasks = *pick.count;
     extern __shared__ __align__(16) uint32_t tab[];
     __shared__ uint32_t next_batch, task_slot;
+    __shared__ CtaTotals totals;
+    totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nb = cap / 4;
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
@@ -643,10 +670,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                                                                  return probe_word(x, p, lb, le, tab, nb);
                                                              });
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, counted));
-            if (lane == 0 && (words | nc)) {
-                atomicAdd(&ctr[0], (unsigned long long)words);
-                if (!kPick) atomicAdd(&ctr[1], (unsigned long long)nc);
-            }
+            if (lane == 0) totals_add(&totals, words, kPick ? 0u : nc);   // else k_sketch_filter counted them
             if (valid) {
                 if (!tk.chunked) {
                     cn[k] = cnt;
@@ -663,6 +687,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         }
         __syncthreads();
     }
+    totals_flush(&totals, ctr);
 }
 
 // One-shot runs on the hash classes (no split pivot, predicate fused): nearly every counted
@@ -759,6 +784,8 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
     uint32_t* bits = smem;
     uint32_t* list = smem + nwords;
     __shared__ uint32_t next_batch, task_slot;
+    __shared__ CtaTotals totals;
+    totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long nsim = 0, ndis = 0;
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
@@ -817,16 +844,14 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
                 if ((int)lane == j) cnt = c;
             }
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
-            if (lane == 0 && (words | nc)) {
-                atomicAdd(&ctr[0], (unsigned long long)words);
-                if (!fp.pend) atomicAdd(&ctr[1], (unsigned long long)nc);
-            }
+            if (lane == 0) totals_add(&totals, words, fp.pend ? 0u : nc);
             if (valid && !fp.pend) cn[k] = cnt;
             fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, dv, cnt, lane, nsim, ndis);
         }
         __syncthreads();
     }
     fused_totals(fp, lane, nsim, ndis);
+    totals_flush(&totals, ctr);
 }
 
 
@@ -889,6 +914,8 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
     uint32_t* bits = smem;                              // kHotBits / 32 words
     uint32_t* tail = smem + kHotBits / 32;              // kTailSlots words
     __shared__ uint32_t next_batch, task_slot;
+    __shared__ CtaTotals totals;
+    totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long nsim = 0, ndis = 0;
     for (uint32_t i = threadIdx.x; i < kHotBits / 128; i += blockDim.x)
@@ -944,10 +971,7 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
                                                                                                 tail, ntb);
                                                                    });
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
-            if (lane == 0 && (words | nc)) {
-                atomicAdd(&ctr[0], (unsigned long long)words);
-                if (!kPick) atomicAdd(&ctr[1], (unsigned long long)nc);
-            }
+            if (lane == 0) totals_add(&totals, words, kPick ? 0u : nc);
             if (valid && (!kPick || !fp.sim)) cn[k] = cnt;
             if (fp.sim) fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, ve - vb, cnt, lane, nsim, ndis);
         }
@@ -959,6 +983,7 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
         __syncthreads();
     }
     fused_totals(fp, lane, nsim, ndis);
+    totals_flush(&totals, ctr);
 }
 
 // Task planner.  Pass 1 (outputs null) counts tasks per class; pass 2 writes them.
