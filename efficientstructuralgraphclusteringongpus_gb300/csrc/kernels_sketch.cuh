@@ -110,23 +110,29 @@ __global__ void k_sketch_assign(uint32_t n, const uint32_t* __restrict__ off, Sk
     }
 }
 
-// Vertices of the classes up to kSketchWarpLog, 32 per warp: those of the smallest class one
-// per lane (four words in registers), the others one after the other by the whole warp in
-// shared memory.
+// Vertices [v_begin, v_end) of the classes up to kSketchWarpLog, 32 per warp: those of the
+// smallest class one per lane (four words in registers), up to kSketchOctetLog four at a time
+// by eight lanes each (folds by shuffle), the others one after the other by the whole warp in
+// shared memory.  Latency bounds it (a list load, the shared atomics, the folds), so several
+// loads are in flight per lane (R-MAT s22: 0.87 ms with a warp per vertex, now 0.66 in eight
+// parts, of which all but the last run while the adjacency arrives).
 constexpr int kSketchWarps = 8;
-__global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32_t n, const uint32_t* __restrict__ off,
+constexpr int kSketchOctetLog = 10;    // 8 units, up to 85 neighbours
+__global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32_t v_begin, uint32_t v_end,
+                                                                          const uint32_t* __restrict__ off,
                                                                           const uint32_t* __restrict__ adj,
                                                                           const uint2* __restrict__ info,
                                                                           uint4* __restrict__ sk) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
     __shared__ __align__(16) uint32_t smem[kSketchWarps][(1u << kSketchWarpLog) / 32];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, gl = lane & 7u, gi = lane >> 3;
     uint32_t* bits = smem[wib];
     uint4* bits4 = reinterpret_cast<uint4*>(bits);
     const uint64_t step = (uint64_t)gridDim.x * kSketchWarps * 32;
-    for (uint64_t v0 = ((uint64_t)blockIdx.x * kSketchWarps + wib) * 32; v0 < n; v0 += step) {
+    for (uint64_t v0 = v_begin + ((uint64_t)blockIdx.x * kSketchWarps + wib) * 32; v0 < v_end; v0 += step) {
         const uint64_t v = v0 + lane;
-        const uint2 iv = v < n ? info[v] : make_uint2(0, 0);
-        const uint32_t b = v < n ? off[v] : 0u;
+        const uint2 iv = v < v_end ? info[v] : make_uint2(0, 0);
+        const uint32_t b = v < v_end ? off[v] : 0u;
         const int l = iv.y >= 2 ? sketch_log(iv.y) : 0;
         if (l == kSketchMinLog) {
             uint4 q = make_uint4(0, 0, 0, 0);
@@ -136,19 +142,69 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
             }
             sk[(uint64_t)iv.x + 1] = q;
         }
-        uint32_t todo = __ballot_sync(0xFFFFFFFFu, l > kSketchMinLog && l <= kSketchWarpLog);
+        uint32_t octets = __ballot_sync(kFull, l > kSketchMinLog && l <= kSketchOctetLog);
+        while (octets) {
+            // the gi-th of the lowest four set bits
+            uint32_t rest = octets;
+            for (uint32_t i = 0; i < gi; ++i) rest &= rest - 1;
+            const int j = rest ? __ffs(rest) - 1 : 0;
+            for (int i = 0; i < 4; ++i) octets &= octets - 1;
+            const uint32_t dj = __shfl_sync(kFull, iv.y, j), a = __shfl_sync(kFull, b, j);
+            const uint64_t unit = __shfl_sync(kFull, iv.x, j);
+            const int lj = __shfl_sync(kFull, l, j);
+            const uint32_t d = rest ? dj : 0u;
+            const uint32_t units = rest ? 1u << (lj - kSketchMinLog) : 0u, mask = rest ? (1u << lj) - 1u : 0u;
+            uint32_t* mine = bits + 32 * gi;               // 8 units
+            reinterpret_cast<uint4*>(mine)[gl] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            for (uint32_t i = gl; i < d; i += 48) {
+                uint32_t w[6];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) w[q] = i + 8 * q < d ? __ldg(adj + a + i + 8 * q) : 0u;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if (i + 8 * q < d) {
+                        const uint32_t h = sketch_hash(w[q]) & mask;
+                        atomicOr(&mine[h >> 5], 1u << (h & 31u));
+                    }
+            }
+            __syncwarp();
+            uint4 x = reinterpret_cast<uint4*>(mine)[gl];
+            if (gl < units) sk[unit + units + gl] = x;
+#pragma unroll
+            for (uint32_t half = 4; half; half >>= 1) {    // folds below 2 * half units
+                uint4 y;
+                y.x = __shfl_down_sync(kFull, x.x, half, 8);
+                y.y = __shfl_down_sync(kFull, x.y, half, 8);
+                y.z = __shfl_down_sync(kFull, x.z, half, 8);
+                y.w = __shfl_down_sync(kFull, x.w, half, 8);
+                if (half < units) {
+                    x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
+                    if (gl < half) sk[unit + half + gl] = x;
+                }
+            }
+            __syncwarp();
+        }
+        uint32_t todo = __ballot_sync(kFull, l > kSketchOctetLog && l <= kSketchWarpLog);
         while (todo) {
             const int j = __ffs(todo) - 1;
             todo &= todo - 1;
-            const uint32_t d = __shfl_sync(0xFFFFFFFFu, iv.y, j), a = __shfl_sync(0xFFFFFFFFu, b, j);
-            const uint64_t unit = __shfl_sync(0xFFFFFFFFu, iv.x, j);
-            const int lj = __shfl_sync(0xFFFFFFFFu, l, j);
+            const uint32_t d = __shfl_sync(kFull, iv.y, j), a = __shfl_sync(kFull, b, j);
+            const uint64_t unit = __shfl_sync(kFull, iv.x, j);
+            const int lj = __shfl_sync(kFull, l, j);
             const uint32_t units = 1u << (lj - kSketchMinLog), mask = (1u << lj) - 1u;
             for (uint32_t i = lane; i < units; i += 32) bits4[i] = make_uint4(0, 0, 0, 0);
             __syncwarp();
-            for (uint32_t i = lane; i < d; i += 32) {
-                const uint32_t h = sketch_hash(__ldg(adj + a + i)) & mask;
-                atomicOr(&bits[h >> 5], 1u << (h & 31u));
+            for (uint32_t i = lane; i < d; i += 256) {
+                uint32_t w[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) w[q] = i + 32 * q < d ? __ldg(adj + a + i + 32 * q) : 0u;
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (i + 32 * q < d) {
+                        const uint32_t h = sketch_hash(w[q]) & mask;
+                        atomicOr(&bits[h >> 5], 1u << (h & 31u));
+                    }
             }
             __syncwarp();
             for (uint32_t i = lane; i < units; i += 32) sk[unit + units + i] = bits4[i];

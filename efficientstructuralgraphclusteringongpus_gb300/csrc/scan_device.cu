@@ -245,8 +245,10 @@ void device_graph_free(DeviceGraph* d) {
     int prev = -1;
     cudaGetDevice(&prev);
     if (d->device >= 0) cudaSetDevice(d->device);
-    // the aux and side streams' last work is joined into the main stream
-    const bool idle = d->stream && cudaStreamSynchronize(d->stream) == cudaSuccess;
+    // The side stream's last work is joined into the main stream, and so is the aux stream's
+    // unless an upload gave up in between.
+    bool idle = d->stream && cudaStreamSynchronize(d->stream) == cudaSuccess;
+    idle = idle && d->aux && cudaStreamSynchronize(d->aux) == cudaSuccess;
     for (auto& a : d->allocs) cache_give(d->device, a.first, a.second);
     if (d->adj_host) cudaFreeHost(d->adj_host);
     const StreamSet x = streams_of(d);
@@ -434,21 +436,18 @@ constexpr int kPendCounts = kPendingLists + 2;
 // queues in one line their atomics waited for one another (k_cn_small 0.105 -> 0.155 ms).
 constexpr int kCounterSpan = 64, kStageCounters = 3 * kCounterSpan;
 
-// Bases and bitmaps of every vertex's sketch, from the resident adjacency, on d->stream.
-static scan_status build_sketches(DeviceGraph* d, const SketchPlan& plan, uint32_t* rank, uint32_t* mid, uint32_t* hub) {
-    cudaStream_t s = d->stream;
-    k_sketch_assign<<<grid_for(d, d->n, 256), 256, 0, s>>>(d->n, d->off, plan, rank, d->sk_info, mid, hub);
-    k_sketch_build_small<<<grid_for(d, d->n, kSketchWarps * 32), kSketchWarps * 32, 0, s>>>(d->n, d->off, d->adj,
-                                                                                         d->sk_info, d->sk);
+// The bitmaps of the larger vertices (lists from k_sketch_assign), on stream s.
+static scan_status build_large_sketches(DeviceGraph* d, const SketchPlan& plan, const uint32_t* mid,
+                                        const uint32_t* hub, cudaStream_t s) {
     constexpr int kMidSmem = (1 << kSketchMidLog) / 8, kHubSmem = (1 << kSketchMaxLog) / 8;
-    if (plan.list_mid)
-        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_mid, (uint64_t)d->num_sms * 8), 256, kMidSmem, s>>>(
-            mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk);
     if (plan.list_hub) {
         SCAN_CUDA(cudaFuncSetAttribute(k_sketch_build_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubSmem));
         k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_hub, (uint64_t)d->num_sms), 1024, kHubSmem, s>>>(
             hub, plan.list_hub, d->off, d->adj, d->sk_info, d->sk);
     }
+    if (plan.list_mid)
+        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_mid, (uint64_t)d->num_sms * 8), 256, kMidSmem,
+                             s>>>(mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk);
     SCAN_CUDA(cudaGetLastError());
     return SCAN_OK;
 }
@@ -626,6 +625,9 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         if (bitmap_path)
             k_hot_assign<<<grid_for(d.get(), n, 256), 256, 0, s2>>>(d->n, d->off, min_bin, kHotBits, d->hot,
                                                                   hist + kDegBins);
+        if (d->sk)
+            k_sketch_assign<<<grid_for(d.get(), n, 256), 256, 0, s2>>>(d->n, d->off, sk_plan, sk_cls + kSketchClasses,
+                                                                     d->sk_info, sk_mid, sk_hub);
         if (adj_in_host_memory) {
             std::memcpy(d->adj_host, adj_host, m * sizeof(uint32_t));
             std::memset(d->adj_host + m, 0, kAdjPad * sizeof(uint32_t));
@@ -646,11 +648,20 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
                     lowbits, flags, kBadId, kBadSelfLoop, kBadOrder);
                 ++orient_launches;
             }
+            if (c == chunks - 1) {
+                if (bitmap_path) SCAN_CUDA(cudaMemsetAsync(d->radj + m, 0, kAdjPad * sizeof(uint32_t), s2));
+                SCAN_CUDA(cudaEventRecord(ev_chunk[kMaxChunks], s2));
+            }
+            if (d->sk && vcut[c + 1] > vcut[c])
+                k_sketch_build_small<<<grid_for(d.get(), vcut[c + 1] - vcut[c], kSketchWarps * 32), kSketchWarps * 32, 0,
+                                       s2>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk);
         }
         SCAN_CUDA(cudaEventRecord(d->ev[1], s));   // end of the copies
-        if (bitmap_path) SCAN_CUDA(cudaMemsetAsync(d->radj + m, 0, kAdjPad * sizeof(uint32_t), s2));
-        SCAN_CUDA(cudaEventRecord(ev_chunk[kMaxChunks], s2));
-        SCAN_CUDA(cudaStreamWaitEvent(s, ev_chunk[kMaxChunks], 0));   // back to one stream
+        // The orientation continues on s; the larger vertices' bitmaps are built beside it and
+        // joined at the end.
+        SCAN_CUDA(cudaStreamWaitEvent(s, ev_chunk[kMaxChunks], 0));
+        if (d->sk) SCAN_TRY(build_large_sketches(d.get(), sk_plan, sk_mid, sk_hub, s2));
+        SCAN_CUDA(cudaEventRecord(d->join, s2));
         return SCAN_OK;
     };
     ost = enqueue();
@@ -679,7 +690,6 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         k_fill_tiles<<<grid_for(d.get(), fill_tiles * kFillThreads, kFillThreads), kFillThreads, 0, s>>>(
             d->n, m, (uint32_t)d->E, d->off, d->adj, tile_v, lowbits, wpre, d->lo_adj, d->lo_src);
     }
-    if (d->sk) SCAN_TRY(build_sketches(d.get(), sk_plan, sk_cls + kSketchClasses, sk_mid, sk_hub));
     SCAN_CUDA(cudaGetLastError());
 
     // Task plan.
@@ -699,6 +709,7 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     uint8_t* rs_mem = nullptr;
     SCAN_TRY(dalloc(d.get(), &rs_mem, run_scratch_bytes(d->n, d->E)));
     run_scratch_bind(&d->rs, rs_mem, d->n, d->E);
+    SCAN_CUDA(cudaStreamWaitEvent(s, d->join, 0));   // the bitmaps: one stream again
     SCAN_CUDA(cudaEventRecord(d->ev[2], s));
     SCAN_CUDA(cudaEventSynchronize(d->ev[2]));
     if (st) {
