@@ -15,12 +15,19 @@
 
 namespace scan {
 struct CnTask;
+struct TaskSlice;
+
+// First 16-byte unit of the array of each bitmap size (kernels_sketch.cuh).
+constexpr int kSketchClasses = 14;
+struct SketchLevels {
+    uint32_t base[kSketchClasses];
+};
 
 // The edges between larger vertices, for a kernel with a warp per edge: a hub's edges of this
 // kind sit together in its list (low ids in power-law graphs), and the few warps that drew
 // them would work on long after the others are done.
 struct LongEdges {
-    uint4* slot;         // bitmaps, bits that decide the edge, sizes (kernels_sketch.cuh: SketchSlot)
+    uint4* slot;         // ranks, bits that decide the edge, sizes (kernels_sketch.cuh: SketchSlot)
     uint32_t* edge;      // edge id
     uint32_t* count;     // edges offered (may exceed cap)
     uint32_t cap;
@@ -89,19 +96,18 @@ struct DeviceGraph {
     uint32_t* hot = nullptr;       // n: hot id or kHotBits + v
     uint32_t* radj = nullptr;      // m + pad: adjacency mapped through hot[]
     uint32_t* tailc = nullptr;     // n: non-hot neighbours per vertex
-    scan::CnTask* hubs = nullptr;  // hub tasks: hmid then bmp, one array
-    scan::CnTask* hmid = nullptr;  // mid hubs (plan.bitmap_min_deg, kHubFilterMax]
-    uint32_t nhmid = 0;
-    scan::CnTask* bmp = nullptr;   // hubs above kHubFilterMax
-    uint32_t nbmp = 0;
+    scan::CnTask* hubs = nullptr;  // hub tasks (pivots above plan.bitmap_min_deg)
+    uint32_t nhub = 0;
     uint32_t cap_small = 0, cap_big[scan::kNumBigClasses] = {}, cap_hubs = 0;   // task array capacities
     scan::PlanParams plan{};
     uint32_t long_words = 32;      // lists of >= long_words 16-byte words get a whole warp
     // neighbourhood sketches (kernels_sketch.cuh; null when off)
-    uint2* sk_info = nullptr;          // n: first 16-byte unit of the vertex's bitmaps, degree
+    uint2* sk_info = nullptr;          // n: rank, degree
     uint4* sk = nullptr;               // the bitmaps
+    scan::SketchLevels sk_levels{};
     uint32_t* pend_pivot = nullptr;    // n: one-shot runs, list work of the edges the sketches leave open
-    uint2* pend_lists = nullptr;       // slices of those pivots' tasks (one array, the task lists' order), ...
+    uint32_t* pend_edges = nullptr;    // E: those edges, gathered per task (cn's memory unless pivots are split)
+    scan::TaskSlice* pend_lists = nullptr;   // slices of those tasks (one array, the task lists' order), ...
     uint32_t* pend_counts = nullptr;   // ... their number per list, and the filter's queue counter
     uint32_t cap_pend = 0;
     scan::LongEdges long_edges{};

@@ -6,7 +6,7 @@
 // once, grouped by its higher endpoint v (the pivot):
 //   1. the pivot's list N(v) (or one id-range chunk of it) is staged in shared memory: a
 //      per-warp hash table for small pivots, and per CTA task a hashed bitmap plus a sorted
-//      copy (one-shot runs, k_cn_filter), a bucketed hash table (full counts, k_cn_big) or
+//      copy (one-shot runs, k_cn_filter_classes), a bucketed hash table (full counts, k_cn_big) or
 //      a bitmap of hot ids (hubs, k_cn_bitmap);
 //   2. warps stream the lower endpoints' lists N(u) with 16-byte loads and probe each
 //      element against it; ballots and warp reductions give the counts;
@@ -46,10 +46,6 @@ constexpr uint32_t kTailMax = kTailSlots / 2;
 // SM: a bitmap task of a mid-size pivot leaves most of its 32 warps waiting at the task
 // barrier (R-MAT s22, eps 0.5: 33.0 ms against 38.3 ms with the threshold at 1024).
 constexpr uint32_t kBitmapMinDeg = kChunkMax;
-// Hubs up to kHubFilterMax entries (the "mid hubs") get their own task list: one-shot runs
-// count them with k_cn_filter (a 2^19-bit filter, <= 1/42 false positives, plus the sorted
-// copy: 112 KB, two CTAs per SM), full counts with k_cn_bitmap like the larger hubs.
-constexpr uint32_t kHubFilterMax = kChunkMaxCap;
 constexpr int kBitmapThreads = 1024;
 __host__ __device__ constexpr uint32_t big_class_entries(int c) { return c == 0 ? 1024u : c == 1 ? 4096u : kChunkMax; }
 __host__ __device__ constexpr uint32_t big_class_slots(int c) { return 4u * big_class_entries(c); }   // load <= 1/4
@@ -200,13 +196,37 @@ struct FusedPred {
 // Edge states k_sketch_filter leaves in sim[]: pending, or 0 (decided: not similar).
 constexpr uint8_t kEdgePending = 2;
 
-// The part of a task list that a launch works on: order[0, *count) are slices of tasks with
-// pending edges, (index into the list, slice | slices << 16); slice i of a task takes every
-// slices-th batch of its edges from the i-th on.  Null: the whole list, tasks undivided.
+// One-shot runs after the sketches: slices of the tasks with pending edges.  edges[e0, e0 +
+// count) of a task {.., e0, ..} are its pending edges; order[0, *count) name the slices.
+struct TaskSlice {
+    uint32_t task;       // index into the task list
+    uint32_t first, step;   // pending edges first, first + step, ... of the task
+    uint32_t count;      // the task's pending edges
+};
 struct TaskPick {
-    const uint2* order;
+    const TaskSlice* order;
     const uint32_t* count;
-    __device__ __forceinline__ uint2 at(uint32_t t) const { return order ? order[t] : make_uint2(t, 1u << 16); }
+    const uint32_t* edges;
+};
+
+// How a slice's edges are dealt to warps: batches small enough that every warp of the CTA has
+// one (a warp streams the long lists of its batch one after the other), at most 32.
+struct SliceBatches {
+    uint32_t edges, size, batches;
+    __device__ __forceinline__ explicit SliceBatches(const TaskSlice& t) {
+        const uint32_t warps = blockDim.x >> 5;
+        edges = (t.count - t.first + t.step - 1) / t.step;
+        size = min(32u, max(1u, (edges + warps - 1) / warps));
+        batches = (edges + size - 1) / size;
+    }
+    // edge of lane i in batch j (strided: the expensive lists of a pivot sit together)
+    __device__ __forceinline__ bool edge(const TaskPick& pick, const TaskSlice& t, uint32_t e0, uint32_t j,
+                                         uint32_t lane, uint32_t* k) const {
+        const uint32_t i = j + lane * batches;
+        if (lane >= size || i >= edges) return false;
+        *k = pick.edges[e0 + t.first + i * t.step];
+        return true;
+    }
 };
 
 // Warp-wide (holds a ballot): every lane calls it; lanes with valid set test edge k
@@ -298,9 +318,6 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* __restrict__
 //     counts (0..8).
 constexpr uint32_t kLongWordsDefault = 32;   // lists of >= 128 entries take the whole warp (tunable)
 constexpr int kWordsInFlight = 2;        // hash and class kernels (48+ registers would cost occupancy)
-constexpr int kWordsInFlightMidHub = 3;  // k_cn_filter on mid hubs: two CTAs per SM by shared memory, so 64
-                                         // registers cost nothing (R-MAT s22: 11.87 -> 11.73 ms; 3 in the
-                                         // class kernels too: 12.11 ms)
 constexpr int kWordsInFlightBitmap = 6;  // bitmap kernel: one CTA per SM, 64 registers at 6 (s22: -0.6 ms against 4)
 
 __device__ __forceinline__ uint32_t lane_range_mask(int lo, int hi) {
@@ -592,13 +609,17 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* queue, uint32_t prev, bo
     return *slot;
 }
 
-// kPick: a one-shot run after the sketches (pend and pick given); full counts keep the plain form.
-template <bool kPick>
+// kPick: a one-shot run after the sketches (pick given); full counts keep the plain form.  The
+// edges the sketches leave open are similar or close to it, so they are counted exactly at
+// once; k_cn_filter_classes' bound and then its recount by binary search took longer (whole
+// runs at eps 0.3: R-MAT of 16,384 vertices 553 -> 369 us, of 65,536 536 -> 405).  fp.sim null:
+// plans with split pivots, counts only.
+template <bool kPerGraph, bool kPick>
 __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32_t* queue,
                          const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                          const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn, uint32_t long_words,
                          CnPrune pr, unsigned long long* __restrict__ ctr, uint32_t* __restrict__ miss,
-                         uint32_t nmiss, uint32_t stride, const uint8_t* pend, TaskPick pick) {
+                         uint32_t nmiss, uint32_t stride, FusedPred fp, TaskPick pick) {
     if constexpr (kPick) ntasks = *pick.count;
     extern __shared__ __align__(16) uint32_t tab[];
     __shared__ uint32_t next_batch, task_slot;
@@ -606,14 +627,17 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
     totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nb = cap / 4;
+    unsigned long long nsim = 0, ndis = 0;
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
         // stride (coprime to ntasks, 0: in order): the i-th task drawn is i * stride mod ntasks,
         // so the chunks of one split pivot, adjacent in the array, run spread over the launch
         // and the misses of the early ones can decide edges for the later ones
         const uint32_t ti = stride ? (uint32_t)((uint64_t)t * stride % ntasks) : t;
-        const uint2 slice = kPick ? pick.at(ti) : make_uint2(ti, 1u << 16);
-        const CnTask tk = tasks[slice.x];
+        TaskSlice slice{ti, 0, 1, 1};
+        if constexpr (kPick) slice = pick.order[ti];
+        const SliceBatches sb(slice);
+        const CnTask tk = tasks[slice.task];
         for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x)
             reinterpret_cast<uint4*>(tab)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
         if (threadIdx.x == 0) next_batch = 0;
@@ -621,17 +645,24 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         for (uint32_t j = tk.cb + threadIdx.x; j < tk.ce; j += blockDim.x) bucket_insert(tab, nb, adj[j]);
         __syncthreads();
         const uint32_t vb = off[tk.v], ve = off[tk.v + 1];
-        const PivotTests pt = pivot_tests(ve - vb, pr);   // np = 0 when counting in full
+        CnPrune Pg;
+        if constexpr (kPerGraph) Pg = prune_of_graph(pr, tk.v);
+        const CnPrune& P = kPerGraph ? Pg : pr;
+        const PivotTests pt = pivot_tests(ve - vb, P);   // np = 0 when counting in full
         const uint32_t lo_id = (tk.cb > vb) ? adj[tk.cb] : 0u;          // chunk id range
         const uint32_t hi_id = (tk.ce < ve) ? adj[tk.ce - 1] : kEmpty;
         for (;;) {
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
             const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
-            const uint32_t kb = tk.e0 + 32u * (kPick ? (slice.y & 0xFFFFu) + j * (slice.y >> 16) : j);
-            if (kb >= tk.e1) break;
-            const uint32_t k = kb + lane;
-            const bool valid = k < tk.e1 && (!kPick || pend[k] == kEdgePending);
+            uint32_t k = tk.e0 + 32u * j + lane;
+            bool valid = k < tk.e1;
+            if constexpr (kPick) {
+                if (j >= sb.batches) break;
+                valid = sb.edge(pick, slice, tk.e0, j, lane, &k);
+            } else if (tk.e0 + 32u * j >= tk.e1) {
+                break;
+            }
             uint32_t ub = 0, ue = 0, u = 0, du = 0, tlo = 0, mi = 0xFFFFFFFFu;
             bool counted = false;
             if (valid) {
@@ -641,7 +672,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                 du = ue - ub;
                 if (edge_pruned(du, pt)) ue = ub;
                 counted = ue > ub && tk.cb == vb;               // once per edge: in its first chunk
-                if (pr.on && ue > ub) tlo = count_floor(du, ve - vb, pt, pr.eps);
+                if (P.on && ue > ub) tlo = count_floor(du, ve - vb, pt, P.eps);
                 if (tk.chunked && ue > ub) {
                     // One-shot runs: the misses found by the edge's other chunks so far bound
                     // its count by du - misses; once that is below tlo the edge is decided and
@@ -671,7 +702,10 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                                                              });
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, counted));
             if (lane == 0) totals_add(&totals, words, kPick ? 0u : nc);   // else k_sketch_filter counted them
-            if (valid) {
+            if (kPick && fp.sim) {                              // no split pivot
+                const bool decided = edge_pruned(du, pt) || cnt < count_floor(du, ve - vb, pt, P.eps);
+                fused_predicate(fp, P, valid, decided, k, u, tk.v, du, ve - vb, cnt, lane, nsim, ndis);
+            } else if (valid) {
                 if (!tk.chunked) {
                     cn[k] = cnt;
                 } else {
@@ -687,6 +721,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         }
         __syncthreads();
     }
+    if constexpr (kPick) fused_totals(fp, lane, nsim, ndis);
     totals_flush(&totals, ctr);
 }
 
@@ -748,7 +783,7 @@ __device__ __forceinline__ uint32_t sorted_count(const uint32_t* list, uint32_t 
     return __reduce_add_sync(0xFFFFFFFFu, c);
 }
 
-// Shared memory of k_cn_filter for a class of up to `entries` pivot entries.
+// Shared memory of k_cn_filter_classes for a class of up to `entries` pivot entries.
 __host__ __device__ constexpr uint32_t filter_log2bits(uint32_t entries) {
     uint32_t l = 10;
     while ((1u << l) < 32u * entries) ++l;
@@ -761,23 +796,14 @@ __host__ __device__ constexpr size_t filter_smem_bytes(uint32_t entries) {
 // list_entries: capacity of the shared sorted copy (pivots hold at most that many entries);
 // the bitmap size follows from it in the kernel (R-MAT s22: passing the bit count as a
 // kernel parameter instead measured 0.9 ms slower over the stage).
-// strided: lane i of batch j takes edge e0 + j + i * nbatch instead of e0 + 32 j + i, so
-// every batch samples the whole slice.  Lower edges are stored in id order, and a hub's
-// expensive lower lists (those of high-degree neighbours, the ones the degree prune leaves)
-// have low ids in R-MAT-like graphs: contiguous batches would hand them to a few warps while
-// the rest finish the cheap batches and wait at the task barrier.
-// Two entry points share the body: k_cn_filter_classes (hash classes) is launch-bounded to
-// three 512-thread CTAs per SM, which holds it to 40 registers (R-MAT s22: the 4,096-entry
-// class 4.67 -> 4.25 ms; two CTAs at 60 registers: slower again); k_cn_filter (mid hubs,
-// held to two CTAs per SM by their 112 KB of shared memory) is left unbounded and streams
-// three words per lane (64 registers; a bound measured slower there).
-template <bool kPerGraph, int W>
-__device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t list_entries,
-                            uint32_t* queue, const uint32_t* __restrict__ off,
-                            const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
-                            uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
-    if (pick.count) ntasks = *pick.count;
+// Launch-bounded to three 512-thread CTAs per SM, which holds it to 40 registers (R-MAT s22:
+// the 4,096-entry class 4.67 -> 4.25 ms; two CTAs at 60 registers: slower again).
+template <bool kPerGraph>
+__global__ void __launch_bounds__(512, 3)
+k_cn_filter_classes(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t list_entries, uint32_t* queue,
+                    const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
+                    const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
+                    unsigned long long* __restrict__ ctr, FusedPred fp) {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t log2bits = filter_log2bits(list_entries);
     const uint32_t nwords = (1u << log2bits) >> 5;
@@ -790,8 +816,7 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
     unsigned long long nsim = 0, ndis = 0;
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
-        const uint2 slice = pick.at(t);
-        const CnTask tk = tasks[slice.x];
+        const CnTask tk = tasks[t];
         CnPrune Pg;
         if constexpr (kPerGraph) Pg = prune_of_graph(pr, tk.v);
         const CnPrune& P = kPerGraph ? Pg : pr;
@@ -812,10 +837,10 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
             const uint32_t nbatch = (tk.e1 - tk.e0 + 31u) >> 5;
-            const uint32_t j = (slice.y & 0xFFFFu) + __shfl_sync(0xFFFFFFFFu, bidx, 0) * (slice.y >> 16);
+            const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
             if (j >= nbatch) break;
-            const uint32_t k = strided ? tk.e0 + j + lane * nbatch : tk.e0 + 32u * j + lane;
-            const bool valid = k < tk.e1 && (!fp.pend || fp.pend[k] == kEdgePending);
+            const uint32_t k = tk.e0 + 32u * j + lane;
+            const bool valid = k < tk.e1;
             uint32_t ub = 0, ue = 0, u = 0, du = 0, tlo = 0;
             bool pruned = false;
             if (valid) {
@@ -830,7 +855,7 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
             // tlo = 0: any count may be similar, so the bound decides nothing; count exactly
             const bool bound_scan = ue > ub && tlo > 0;
             uint32_t words = 0;
-            uint32_t cnt = count_batch<W>(adj, lane, ub, bound_scan ? ue : ub, tlo, long_words, words,
+            uint32_t cnt = count_batch<kWordsInFlight>(adj, lane, ub, bound_scan ? ue : ub, tlo, long_words, words,
                                                        [&](uint4 x, uint32_t p, uint32_t lb, uint32_t le) {
                                                            return filter_probe_word(x, p, lb, le, bits, log2bits);
                                                        });
@@ -844,35 +869,14 @@ __device__ __forceinline__ void cn_filter_body(const CnTask* __restrict__ tasks,
                 if ((int)lane == j) cnt = c;
             }
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
-            if (lane == 0) totals_add(&totals, words, fp.pend ? 0u : nc);
-            if (valid && !fp.pend) cn[k] = cnt;
-            fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, dv, cnt, lane, nsim, ndis);
+            if (lane == 0) totals_add(&totals, words, nc);
+            if (valid) cn[k] = cnt;
+            fused_predicate<false>(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, dv, cnt, lane, nsim, ndis);
         }
         __syncthreads();
     }
     fused_totals(fp, lane, nsim, ndis);
     totals_flush(&totals, ctr);
-}
-
-
-template <bool kPerGraph>
-__global__ void __launch_bounds__(512, 3) k_cn_filter_classes(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t list_entries,
-                            uint32_t* queue, const uint32_t* __restrict__ off,
-                            const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
-                            uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
-    cn_filter_body<kPerGraph, kWordsInFlight>(tasks, ntasks, list_entries, queue, off, adj, lo_adj, cn, long_words, pr, ctr, fp,
-                              strided, pick);
-}
-
-template <bool kPerGraph>
-__global__ void k_cn_filter(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t list_entries,
-                            uint32_t* queue, const uint32_t* __restrict__ off,
-                            const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
-                            uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr,
-                            unsigned long long* __restrict__ ctr, FusedPred fp, uint32_t strided, TaskPick pick) {
-    cn_filter_body<kPerGraph, kWordsInFlightMidHub>(tasks, ntasks, list_entries, queue, off, adj, lo_adj, cn, long_words, pr, ctr, fp,
-                              strided, pick);
 }
 
 // Bitmap path: one CTA of kBitmapThreads per task (pivot, edge slice), one CTA per SM.
@@ -922,8 +926,10 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
         reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
-        const uint2 slice = kPick ? pick.at(t) : make_uint2(t, 1u << 16);
-        const CnTask tk = tasks[slice.x];
+        TaskSlice slice{t, 0, 1, 1};
+        if constexpr (kPick) slice = pick.order[t];
+        const SliceBatches sb(slice);
+        const CnTask tk = tasks[slice.task];
         CnPrune Pg;
         if constexpr (kPerGraph) Pg = prune_of_graph(pr, tk.v);
         const CnPrune& P = kPerGraph ? Pg : pr;
@@ -936,6 +942,7 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             reinterpret_cast<uint4*>(tail)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
         if (threadIdx.x == 0) next_batch = 0;
         __syncthreads();
+#pragma unroll 4
         for (uint32_t j = vb + threadIdx.x; j < ve; j += blockDim.x) {
             const uint32_t w = radj[j];
             if (w < kHotBits) atomicOr(&bits[w >> 5], 1u << (w & 31u));
@@ -946,13 +953,21 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             uint32_t bidx = 0;
             if (lane == 0) bidx = atomicAdd(&next_batch, 1u);
             const uint32_t nbatch = (tk.e1 - tk.e0 + 31u) >> 5;
-            const uint32_t b = __shfl_sync(0xFFFFFFFFu, bidx, 0);
-            const uint32_t j = kPick ? (slice.y & 0xFFFFu) + b * (slice.y >> 16) : b;
-            if (j >= nbatch) break;
-            // one-shot runs: strided, as k_cn_filter's hub launch; full counts (every edge
-            // counted, no pruned majority): contiguous, measured faster
-            const uint32_t k = strided ? tk.e0 + j + lane * nbatch : tk.e0 + 32u * j + lane;
-            const bool valid = k < tk.e1 && (!kPick || fp.pend[k] == kEdgePending);
+            const uint32_t j = __shfl_sync(0xFFFFFFFFu, bidx, 0);
+            // One-shot runs: strided, lane i of batch j takes edge e0 + j + i * nbatch.  Lower
+            // edges are stored in id order, and a hub's expensive lower lists (those of
+            // high-degree neighbours, the ones the degree prune leaves) have low ids in
+            // R-MAT-like graphs: contiguous batches would hand them to a few warps while the
+            // rest wait at the task barrier.  Full counts (every edge counted, no pruned
+            // majority): contiguous, measured faster.
+            uint32_t k = strided ? tk.e0 + j + lane * nbatch : tk.e0 + 32u * j + lane;
+            bool valid = k < tk.e1;
+            if constexpr (kPick) {
+                if (j >= sb.batches) break;
+                valid = sb.edge(pick, slice, tk.e0, j, lane, &k);
+            } else if (j >= nbatch) {
+                break;
+            }
             uint32_t ub = 0, ue = 0, u = 0, du = 0;
             bool pruned = false;
             if (valid) {
@@ -976,6 +991,7 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             if (fp.sim) fused_predicate(fp, P, valid, pruned || cnt < tlo, k, u, tk.v, du, ve - vb, cnt, lane, nsim, ndis);
         }
         __syncthreads();
+#pragma unroll 4
         for (uint32_t j = vb + threadIdx.x; j < ve; j += blockDim.x) {   // clear this pivot's bits
             const uint32_t w = radj[j];
             if (w < kHotBits) bits[w >> 5] = 0u;
@@ -987,9 +1003,8 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
 }
 
 // Task planner.  Pass 1 (outputs null) counts tasks per class; pass 2 writes them.
-// counts[0] small pivots, counts[1 + c] tasks of hash class c, counts[4] bitmap tasks of
-// hubs above kHubFilterMax, counts[5] bitmap tasks of the mid hubs, counts[6] (pass 1 only)
-// pivots split into chunks.
+// counts[0] small pivots, counts[1 + c] tasks of hash class c, counts[4] hub
+// tasks, counts[5] (pass 1 only) pivots split into chunks.
 // tail (may be null: bitmap path off) holds each vertex's count of non-hot neighbours.
 // (PlanParams: device_graph.h.)
 
@@ -997,8 +1012,8 @@ __global__ void k_plan(uint32_t n, const uint32_t* __restrict__ off, const uint3
                        const unsigned long long* __restrict__ work, const uint32_t* __restrict__ tail,
                        PlanParams pp, uint32_t* __restrict__ counts, uint32_t* __restrict__ small_out,
                        CnTask* __restrict__ big0, CnTask* __restrict__ big1, CnTask* __restrict__ big2,
-                       CnTask* __restrict__ bmp, CnTask* __restrict__ hmid) {
-    constexpr int kClasses = 3 + kNumBigClasses;   // small, hash classes, big hubs, mid hubs
+                       CnTask* __restrict__ hubs) {
+    constexpr int kClasses = 2 + kNumBigClasses;   // small, hash classes, hubs
     __shared__ uint32_t blk[kClasses];
     __shared__ uint32_t base[kClasses];
     if (threadIdx.x < kClasses) blk[threadIdx.x] = 0;
@@ -1014,7 +1029,7 @@ __global__ void k_plan(uint32_t n, const uint32_t* __restrict__ off, const uint3
                 cls = 0;
                 ntask = 1;
             } else if (tail && dv > pp.bitmap_min_deg && tail[v] <= kTailMax) {
-                cls = dv <= kHubFilterMax ? 2 + kNumBigClasses : 1 + kNumBigClasses;
+                cls = 1 + kNumBigClasses;
                 nch = 1;
                 unsigned long long s = (work[v] + pp.target_probes_bitmap - 1) / pp.target_probes_bitmap;
                 const uint32_t smax = (L + pp.min_slice_edges - 1) / pp.min_slice_edges;
@@ -1047,7 +1062,7 @@ __global__ void k_plan(uint32_t n, const uint32_t* __restrict__ off, const uint3
         small_out[pos] = v;
         return;
     }
-    CnTask* out = cls == 1 ? big0 : cls == 2 ? big1 : cls == 3 ? big2 : cls == 4 ? bmp : hmid;
+    CnTask* out = cls == 1 ? big0 : cls == 2 ? big1 : cls == 3 ? big2 : hubs;
     const uint32_t vb = off[v], e0 = lo_off[v];
     const uint32_t mbase = nch > 1 ? atomicAdd(&counts[kClasses + 1], L) : 0u;   // this pivot's miss counters
     uint32_t i = 0;

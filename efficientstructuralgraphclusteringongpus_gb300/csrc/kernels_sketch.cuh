@@ -2,20 +2,21 @@
 // short bitmaps, before any neighbour list is read.
 //
 // A vertex of degree d >= 2 keeps its neighbours hashed into a bitmap of 2^L bits, L the
-// least with 2^L >= kSketchBits * d (at least 2^7, at most 2^20), and every fold of that
-// bitmap down to 2^7 bits: the fold of 2^l bits is the lower half OR the upper half of the
-// one of 2^(l+1), which is the bitmap the same hash gives with l bits.  So two vertices can
-// be compared at any size both have.  A bit set for u and clear for v is a neighbour of u
-// that v does not have, and distinct bits are distinct neighbours, so
+// least with 2^L >= 12 d (16 d above 85 neighbours; at least 2^7, at most 2^20), and every
+// fold of that bitmap down to 2^7 bits: the fold of 2^l bits is the lower half OR the upper
+// half of the one of 2^(l+1), which is the bitmap the same hash gives with l bits.  So two
+// vertices can be compared at any size both have.  A bit set for u and clear for v is a
+// neighbour of u that v does not have, and distinct bits are distinct neighbours, so
 //     |N(u) & N(v)| <= d_u - popcount(bits_u & ~bits_v).
 // An edge whose count must reach tlo (count_floor) is decided, not similar, once more than
 // d_u - tlo such bits are seen; the rest are left to the list kernels (kernels_cn.cuh).
 //
-// Layout: the bitmaps of a vertex form a heap in 16-byte units: the fold of 2^l bits starts
-// 2^(l-7) units after the vertex's base and is 2^(l-7) units long, 2^(L-6) units in all (the
-// first is unused).  Bases are assigned by size class, largest first, so each heap is aligned
-// to its own size and a group of lanes reads whole 128-byte lines.  About as many bytes as
-// the adjacency itself (R-MAT s22: 523 MB against 513).
+// Layout, in 16-byte units: all bitmaps of 2^l bits are one array, 2^(l-7) units each, in the
+// order of the vertices' ranks; ranks descend by L, so the vertices that have a size are the
+// first ones.  Every bitmap is aligned to its own size (up to 128 bytes), and what a run reads
+// (mostly one or two sizes per vertex) lies together: with each vertex's sizes side by side
+// instead, the similarity stage of R-MAT s22 at eps 0.5 took 2.06 ms, so 1.87.  All arrays
+// together are about as large as the adjacency.
 #pragma once
 
 #include "device_common.cuh"
@@ -24,18 +25,22 @@
 
 namespace scan {
 
-constexpr uint32_t kSketchBits = 12;      // bits per neighbour, rounded up to a power of two
+// Bits per neighbour, rounded up to a power of two.  More decide more edges at low eps and are
+// read only where fewer cannot; longer lists cost more to count when left open (R-MAT s21 at
+// eps 0.2, whole run: 6.0 ms with 12 throughout, 5.0 with 16 above 85 neighbours, 5.95 with 24
+// above 682).
+constexpr uint32_t kSketchBits = 12, kSketchBitsLarge = 16, kSketchLargeDeg = 85;
 constexpr int kSketchMinLog = 7;          // one 16-byte unit
 constexpr int kSketchMaxLog = 20;         // 128 KB: larger hubs share bits
-constexpr int kSketchClasses = kSketchMaxLog - kSketchMinLog + 1;
+static_assert(kSketchClasses == kSketchMaxLog - kSketchMinLog + 1, "bitmap sizes");
 constexpr int kSketchMidLog = 17;         // classes up to here are built by small CTAs, larger by whole-SM ones
 constexpr int kSketchWarpLog = 13;        // classes up to here are built by one warp
 
 // log2 of the bitmap size of a vertex of degree d >= 1.
 __host__ __device__ __forceinline__ int sketch_log(uint32_t d) {
     if (d <= (1u << kSketchMinLog) / kSketchBits) return kSketchMinLog;
-    if (d >= (1u << kSketchMaxLog) / kSketchBits) return kSketchMaxLog;
-    const uint32_t x = kSketchBits * d - 1u;      // ceil(log2(x + 1)), x >= 127
+    if (d >= (1u << kSketchMaxLog) / kSketchBitsLarge) return kSketchMaxLog;
+    const uint32_t x = (d > kSketchLargeDeg ? kSketchBitsLarge : kSketchBits) * d - 1u;   // ceil(log2(x + 1))
 #ifdef __CUDA_ARCH__
     return 32 - __clz(x);
 #else
@@ -63,13 +68,18 @@ __global__ void k_sketch_classes(uint32_t n, const uint32_t* __restrict__ off, u
     if (threadIdx.x < kSketchClasses && h[threadIdx.x]) atomicAdd(&cls[threadIdx.x], h[threadIdx.x]);
 }
 
-// First unit of each class and the lists of the vertices that CTAs build.
+// First rank of each class and the lists of the vertices that CTAs build.
 struct SketchPlan {
-    uint32_t base[kSketchClasses];    // first 16-byte unit of the class
+    uint32_t first[kSketchClasses];
     uint32_t list_mid, list_hub;      // entries of the two lists
 };
 
-// info[v] = (first unit of v's heap, degree).  rank: one counter per class, then the mid and
+// The bitmap of 2^l bits of the vertex of a rank: its first unit.
+__device__ __forceinline__ uint32_t sketch_unit(const SketchLevels& lv, int l, uint32_t rank) {
+    return lv.base[l - kSketchMinLog] + (rank << (l - kSketchMinLog));
+}
+
+// info[v] = (rank, degree).  rank: one counter per class, then the mid and
 // hub list counters, all zero.  The order within a class is whatever the atomics give; nothing
 // depends on it.
 __global__ void k_sketch_assign(uint32_t n, const uint32_t* __restrict__ off, SketchPlan plan,
@@ -93,9 +103,9 @@ __global__ void k_sketch_assign(uint32_t n, const uint32_t* __restrict__ off, Sk
             base[threadIdx.x] = h[threadIdx.x] ? atomicAdd(&rank[threadIdx.x], h[threadIdx.x]) : 0u;
         __syncthreads();
         if (v < n) {
-            uint32_t unit = 0;
+            uint32_t place = 0;
             if (c >= 0) {
-                unit = plan.base[c] + ((base[c] + r) << (c + 1));
+                place = plan.first[c] + base[c] + r;
                 const int l = c + kSketchMinLog;
                 if (l > kSketchMidLog) {
                     const uint32_t i = atomicAdd(&rank[kSketchClasses + 1], 1u);
@@ -105,7 +115,7 @@ __global__ void k_sketch_assign(uint32_t n, const uint32_t* __restrict__ off, Sk
                     if (i < plan.list_mid) mid[i] = (uint32_t)v;
                 }
             }
-            info[v] = make_uint2(unit, d);
+            info[v] = make_uint2(place, d);
         }
     }
 }
@@ -122,7 +132,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
                                                                           const uint32_t* __restrict__ off,
                                                                           const uint32_t* __restrict__ adj,
                                                                           const uint2* __restrict__ info,
-                                                                          uint4* __restrict__ sk) {
+                                                                          uint4* __restrict__ sk, SketchLevels lv) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     __shared__ __align__(16) uint32_t smem[kSketchWarps][(1u << kSketchWarpLog) / 32];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, gl = lane & 7u, gi = lane >> 3;
@@ -140,7 +150,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
                 const uint32_t h = sketch_hash(adj[b + j]) & 127u, bit = 1u << (h & 31u), w = h >> 5;
                 if (w == 0) q.x |= bit; else if (w == 1) q.y |= bit; else if (w == 2) q.z |= bit; else q.w |= bit;
             }
-            sk[(uint64_t)iv.x + 1] = q;
+            sk[sketch_unit(lv, kSketchMinLog, iv.x)] = q;
         }
         uint32_t octets = __ballot_sync(kFull, l > kSketchMinLog && l <= kSketchOctetLog);
         while (octets) {
@@ -150,7 +160,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
             const int j = rest ? __ffs(rest) - 1 : 0;
             for (int i = 0; i < 4; ++i) octets &= octets - 1;
             const uint32_t dj = __shfl_sync(kFull, iv.y, j), a = __shfl_sync(kFull, b, j);
-            const uint64_t unit = __shfl_sync(kFull, iv.x, j);
+            const uint32_t rank = __shfl_sync(kFull, iv.x, j);
             const int lj = __shfl_sync(kFull, l, j);
             const uint32_t d = rest ? dj : 0u;
             const uint32_t units = rest ? 1u << (lj - kSketchMinLog) : 0u, mask = rest ? (1u << lj) - 1u : 0u;
@@ -170,9 +180,10 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
             }
             __syncwarp();
             uint4 x = reinterpret_cast<uint4*>(mine)[gl];
-            if (gl < units) sk[unit + units + gl] = x;
+            if (gl < units) sk[sketch_unit(lv, lj, rank) + gl] = x;
 #pragma unroll
-            for (uint32_t half = 4; half; half >>= 1) {    // folds below 2 * half units
+            for (int f = 2; f >= 0; --f) {                 // the fold of 2^f units
+                const uint32_t half = 1u << f;
                 uint4 y;
                 y.x = __shfl_down_sync(kFull, x.x, half, 8);
                 y.y = __shfl_down_sync(kFull, x.y, half, 8);
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
                 y.w = __shfl_down_sync(kFull, x.w, half, 8);
                 if (half < units) {
                     x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
-                    if (gl < half) sk[unit + half + gl] = x;
+                    if (gl < half) sk[sketch_unit(lv, kSketchMinLog + f, rank) + gl] = x;
                 }
             }
             __syncwarp();
@@ -190,7 +201,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
             const int j = __ffs(todo) - 1;
             todo &= todo - 1;
             const uint32_t d = __shfl_sync(kFull, iv.y, j), a = __shfl_sync(kFull, b, j);
-            const uint64_t unit = __shfl_sync(kFull, iv.x, j);
+            const uint32_t rank = __shfl_sync(kFull, iv.x, j);
             const int lj = __shfl_sync(kFull, l, j);
             const uint32_t units = 1u << (lj - kSketchMinLog), mask = (1u << lj) - 1u;
             for (uint32_t i = lane; i < units; i += 32) bits4[i] = make_uint4(0, 0, 0, 0);
@@ -207,15 +218,17 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
                     }
             }
             __syncwarp();
-            for (uint32_t i = lane; i < units; i += 32) sk[unit + units + i] = bits4[i];
-            for (uint32_t half = units >> 1; half; half >>= 1) {   // folds, in place
+            const uint32_t at = sketch_unit(lv, lj, rank);
+            for (uint32_t i = lane; i < units; i += 32) sk[at + i] = bits4[i];
+            for (int f = lj - 1; f >= kSketchMinLog; --f) {        // folds, in place
+                const uint32_t half = 1u << (f - kSketchMinLog), to = sketch_unit(lv, f, rank);
                 __syncwarp();
                 for (uint32_t i = lane; i < half; i += 32) {
                     uint4 x = bits4[i];
                     const uint4 y = bits4[i + half];
                     x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
                     bits4[i] = x;
-                    sk[unit + half + i] = x;
+                    sk[to + i] = x;
                 }
             }
             __syncwarp();
@@ -226,7 +239,7 @@ __global__ void __launch_bounds__(kSketchWarps * 32) k_sketch_build_small(uint32
 // The larger classes: one CTA per vertex of a list, the bitmap in dynamic shared memory.
 __global__ void k_sketch_build_cta(const uint32_t* __restrict__ list, uint32_t count, const uint32_t* __restrict__ off,
                                    const uint32_t* __restrict__ adj, const uint2* __restrict__ info,
-                                   uint4* __restrict__ sk) {
+                                   uint4* __restrict__ sk, SketchLevels lv) {
     extern __shared__ __align__(16) uint32_t sketch_smem[];
     uint32_t* bits = sketch_smem;
     uint4* bits4 = reinterpret_cast<uint4*>(bits);
@@ -244,15 +257,17 @@ __global__ void k_sketch_build_cta(const uint32_t* __restrict__ list, uint32_t c
             atomicOr(&bits[h >> 5], 1u << (h & 31u));
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < units; i += blockDim.x) sk[(uint64_t)iv.x + units + i] = bits4[i];
-        for (uint32_t half = units >> 1; half; half >>= 1) {
+        const uint32_t at = sketch_unit(lv, l, iv.x);
+        for (uint32_t i = threadIdx.x; i < units; i += blockDim.x) sk[at + i] = bits4[i];
+        for (int f = l - 1; f >= kSketchMinLog; --f) {
+            const uint32_t half = 1u << (f - kSketchMinLog), to = sketch_unit(lv, f, iv.x);
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
                 uint4 x = bits4[i];
                 const uint4 y = bits4[i + half];
                 x.x |= y.x; x.y |= y.y; x.z |= y.z; x.w |= y.w;
                 bits4[i] = x;
-                sk[(uint64_t)iv.x + half + i] = x;
+                sk[to + i] = x;
             }
         }
         __syncthreads();
@@ -279,7 +294,7 @@ __device__ __forceinline__ int sketch_level(uint32_t du, uint32_t dv, uint32_t n
 }
 
 struct SketchSlot {      // one edge of a warp's batch that needs its bitmaps
-    uint32_t bu, bv;     // first units of the two heaps
+    uint32_t ru, rv;     // ranks of the endpoints
     uint32_t need;       // missing bits that decide it
     uint32_t code;       // edge within the batch | level << 8 | top level << 16
 };
@@ -299,7 +314,8 @@ __device__ __forceinline__ uint32_t missing_bits(const uint4 x, const uint4 y) {
 //   * larger: the list of k_sketch_long, a warp per edge.  A hub's edges of this kind sit
 //     together in its list (low ids in power-law graphs), and the few warps that drew them
 //     would work on long after the others are done (power law, 57M edges: 4.35 -> 1.35 ms).
-// An edge that its size leaves undecided is tried once more at the lower endpoint's largest.
+// An edge that its size leaves undecided is tried again at four times that, up to the lower
+// endpoint's largest.
 // A pivot's bitmaps are shared by its consecutive edges and stay in L1.
 // sim[k] = kEdgePending for an edge the list kernels must count, 0 otherwise (decided: both
 // predicates reject it).  The pending work of pivots above small_deg goes to pivot[v] and, in
@@ -339,7 +355,7 @@ template <bool kPerGraph>
 __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint32_t* __restrict__ lo_adj,
                                                        const uint32_t* __restrict__ lo_src,
                                                        const uint2* __restrict__ info, const uint4* __restrict__ sk,
-                                                       CnPrune pr, uint32_t chunk, uint32_t* queue,
+                                                       SketchLevels levels, CnPrune pr, uint32_t chunk, uint32_t* queue,
                                                        uint8_t* __restrict__ sim, PendingWork pw, LongEdges ll,
                                                        unsigned long long* __restrict__ ctr) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
@@ -347,6 +363,9 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
     constexpr uint32_t kGroups = 32 / G, kStep = G * U;
     static_assert(kStep <= (2u << (kSketchLaneLog - kSketchMinLog)), "a group step must not exceed its smallest bitmap");
     __shared__ SketchSlot slots[8][kSketchBatch];
+    __shared__ SketchLevels lv;               // indexed by lane: shared memory, not a parameter
+    if (threadIdx.x < kSketchClasses) lv.base[threadIdx.x] = levels.base[threadIdx.x];
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31, gl = lane % G, gi = lane / G;
     const uint32_t lower = (1u << lane) - 1u;
     SketchSlot* slot = slots[threadIdx.x >> 5];
@@ -355,7 +374,7 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
     // A long edge for k_sketch_long; false when the list is full.
     auto defer = [&](const SketchSlot& s, uint64_t k, uint32_t at) {
         if (at >= ll.cap) return false;
-        ll.slot[at] = make_uint4(s.bu, s.bv, s.need, s.code);
+        ll.slot[at] = make_uint4(s.ru, s.rv, s.need, s.code);
         ll.edge[at] = (uint32_t)k;
         return true;
     };
@@ -398,8 +417,8 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                             s.need = iu.y - tlo + 1;
                             if (iu.y >= 2) l = sketch_level(iu.y, iv.y, s.need, top);
                             if (l == 0) state = kEdgePending;
-                            s.bu = iu.x;
-                            s.bv = iv.x;
+                            s.ru = iu.x;
+                            s.rv = iv.x;
                             s.code = (32 * q + lane) | l << 8 | (uint32_t)top << 16;
                         }
                     }
@@ -432,8 +451,8 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                 const uint32_t top = slot_top(s);
                 for (;;) {
                     const uint32_t units = 1u << (l - kSketchMinLog);
-                    const uint4* pu = sk + ((uint64_t)s.bu + units);
-                    const uint4* pv = sk + ((uint64_t)s.bv + units);
+                    const uint4* pu = sk + sketch_unit(lv, l, s.ru);
+                    const uint4* pv = sk + sketch_unit(lv, l, s.rv);
                     uint32_t miss = 0, pos = 0;
                     do {
                         const bool two = units > 1;
@@ -452,7 +471,7 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                         pending += edge_pending(sim, pw, lo_adj, lo_src, info, kb + (s.code & 0xFFu));
                         break;
                     }
-                    l = top;
+                    l = min(l + 2, top);
                 }
             }
             if (groups) {
@@ -463,8 +482,8 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                 uint32_t left = 0, miss = 0;               // units left at this size
                 auto open = [&]() {
                     left = 1u << (slot_level(s) - kSketchMinLog);
-                    pu = sk + ((uint64_t)s.bu + left + gl);
-                    pv = sk + ((uint64_t)s.bv + left + gl);
+                    pu = sk + sketch_unit(lv, slot_level(s), s.ru) + gl;
+                    pv = sk + sketch_unit(lv, slot_level(s), s.rv) + gl;
                     miss = 0;
                 };
                 if (on) {
@@ -495,10 +514,10 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                         if (gl == 0) words += (1u << (slot_level(s) - kSketchMinLog)) - left;
                         if (miss < s.need) {
                             const uint64_t k = kb + (s.code & 0xFFu);
-                            if (slot_level(s) < slot_top(s)) {     // the size chosen was too coarse: the largest
-                                s.code = (s.code & ~0xFF00u) | slot_top(s) << 8;
+                            if (slot_level(s) < slot_top(s)) {     // the size chosen was too coarse
+                                s.code = (s.code & ~0xFF00u) | min(slot_level(s) + 2, slot_top(s)) << 8;
                                 bool deferred = false;
-                                if (slot_top(s) > kSketchGroupLog) {
+                                if (slot_level(s) > kSketchGroupLog) {
                                     if (gl == 0) deferred = defer(s, k, atomicAdd(ll.count, 1u));
                                     deferred = __shfl_sync(((1u << G) - 1u) << (gi * G), deferred, gi * G);
                                 }
@@ -543,7 +562,7 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
 __global__ void __launch_bounds__(256) k_sketch_long(LongEdges ll, const uint32_t* __restrict__ lo_adj,
                                                      const uint32_t* __restrict__ lo_src,
                                                      const uint2* __restrict__ info, const uint4* __restrict__ sk,
-                                                     uint8_t* __restrict__ sim, PendingWork pw,
+                                                     SketchLevels lv, uint8_t* __restrict__ sim, PendingWork pw,
                                                      unsigned long long* __restrict__ ctr) {
     static_assert(kSketchGroupLog + 1 - kSketchMinLog >= 7, "a long edge has whole steps of 128 units");
     const uint32_t lane = threadIdx.x & 31;
@@ -553,10 +572,10 @@ __global__ void __launch_bounds__(256) k_sketch_long(LongEdges ll, const uint32_
     for (uint64_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < count; i += step) {
         const uint4 e = ll.slot[i];
         const SketchSlot s{e.x, e.y, e.z, e.w};
-        for (uint32_t level = slot_level(s);; level = slot_top(s)) {
+        for (uint32_t level = slot_level(s);; level = min(level + 2, slot_top(s))) {
             const uint32_t units = 1u << (level - kSketchMinLog);
-            const uint4* pu = sk + ((uint64_t)s.bu + units + lane);
-            const uint4* pv = sk + ((uint64_t)s.bv + units + lane);
+            const uint4* pu = sk + sketch_unit(lv, level, s.ru) + lane;
+            const uint4* pv = sk + sketch_unit(lv, level, s.rv) + lane;
             uint32_t miss = 0, left = units;
             do {
                 uint4 x[4], y[4];
@@ -801,52 +820,116 @@ __global__ void __launch_bounds__(256) k_predicate_pending(uint64_t E, const uin
 
 // ---- pending edges of larger pivots -----------------------------------------------------------
 
-// The tasks of the plan whose pivot has a pending edge, cut into slices of about equal pending
-// work: the plan's tasks are sized for counting every edge, and a hub with a few hundred
-// pending edges would keep one CTA busy after all others are done (R-MAT s21, eps 0.2: hub
-// kernels 2.7 -> 1.2 ms).  Per task list, entries of TaskPick::order; counts[c] hash class c,
-// counts[kNumBigClasses] the larger hubs, counts[1 + kNumBigClasses] the mid hubs.
-constexpr int kPendingLists = kNumBigClasses + 2;
+// The pending edges of every task of the plan, gathered at the task's place in edges[] (of E
+// entries), and the task cut into slices of about equal pending work: the plan's tasks are
+// sized for counting every edge, so a hub's few pending edges would be sought among all of
+// its edges and keep one CTA busy after the others are done.  Per task list, entries of
+// TaskPick::order; counts[c] hash class c, counts[kNumBigClasses] the hubs.
+constexpr int kPendingLists = kNumBigClasses + 1;
 constexpr uint32_t kPendingSlices = 8;        // slices aimed at per SM, over all lists
 constexpr uint32_t kPendingMinWork = 512;     // 32K list entries: a slice stages its pivot again
 struct PendingLists {
     const CnTask* tasks[kPendingLists];
     uint32_t count[kPendingLists];
-    uint2* out[kPendingLists];                // count + kPendingSlices per SM entries
+    TaskSlice* out[kPendingLists];            // count + kPendingSlices per SM entries
 };
 
-__global__ void k_pending_tasks(PendingLists pl, PendingWork pw, const uint32_t* __restrict__ off,
-                                const uint32_t* __restrict__ lo_off, uint32_t slices, uint32_t* __restrict__ counts) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t even = (uint32_t)min(*pw.total / slices + 1, 0x7FFFFFFFull);
-    for (int a = 0; a < kPendingLists; ++a) {
-        const uint32_t cnt = pl.count[a];
-        for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < cnt; i0 += (uint64_t)gridDim.x * blockDim.x) {
-            const uint64_t i = i0 + threadIdx.x;
-            uint32_t n = 0;
-            if (i < cnt) {
-                const CnTask t = pl.tasks[a][i];
-                const uint32_t work = pw.pivot[t.v];
-                if (work) {
-                    const uint32_t dv = off[t.v + 1] - off[t.v], edges = lo_off[t.v + 1] - lo_off[t.v];
-                    const uint64_t mine = (uint64_t)work * (t.e1 - t.e0) / edges;        // the task's share
-                    const uint32_t aim = max(even, max(kPendingMinWork, dv / 16));       // 4 d_v entries at least
-                    n = (uint32_t)min(mine / aim + 1, (uint64_t)min((t.e1 - t.e0 + 31) / 32, 0xFFFFu));
-                    n = max(n, 1u);
-                }
-            }
-            uint32_t incl = n;
+// The pending edges of [e0, e1) in order to edges[e0...]; returns their number.  In order: the
+// chunk tasks of a split pivot gather the same edges at the same place, perhaps at the same
+// time.
+__device__ __forceinline__ uint32_t warp_exclusive(uint32_t n, uint32_t lane, uint32_t* total) {
+    uint32_t incl = n;
 #pragma unroll
-            for (int s = 1; s < 32; s <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, s);
-                if (lane >= (uint32_t)s) incl += y;
-            }
-            uint32_t at = 0;
-            if (lane == 31 && incl) at = atomicAdd(&counts[a], incl);
-            at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - n;
-            for (uint32_t q = 0; q < n; ++q) pl.out[a][at + q] = make_uint2((uint32_t)i, q | n << 16);
-        }
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, s);
+        if (lane >= (uint32_t)s) incl += y;
     }
+    *total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    return incl - n;
+}
+
+__device__ __forceinline__ uint32_t gather_pending_warp(const uint8_t* sim, uint32_t e0, uint32_t e1,
+                                                        uint32_t* __restrict__ edges, uint32_t lane) {
+    uint32_t found = 0;
+    for (uint64_t s0 = e0 & ~3ull; s0 < e1; s0 += 128) {
+        const uint64_t k = s0 + 4 * lane;
+        uint32_t bits = pending_bits(sim, k, e1);
+        if (k < e0) bits &= 0xFu << (e0 - (uint32_t)k);    // the first word may start before the task
+        uint32_t total;
+        uint32_t at = e0 + found + warp_exclusive(__popc(bits), lane, &total);
+        for (; bits; bits &= bits - 1) edges[at++] = (uint32_t)k + __ffs(bits) - 1;
+        found += total;
+    }
+    return found;
+}
+
+__device__ __forceinline__ uint32_t gather_pending_cta(const uint8_t* sim, uint32_t e0, uint32_t e1,
+                                                       uint32_t* __restrict__ edges, uint32_t lane,
+                                                       uint32_t* warp_sums) {
+    uint32_t found = 0;
+    const uint32_t wib = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (uint64_t s0 = e0 & ~15ull; s0 < e1; s0 += 16ull * blockDim.x) {
+        const uint64_t k = s0 + 16ull * threadIdx.x;
+        uint32_t bits = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bits |= pending_bits(sim, k + 4 * q, e1) << (4 * q);
+        if (k < e0) bits &= 0xFFFFu << (e0 - (uint32_t)k);
+        uint32_t total;
+        const uint32_t before = warp_exclusive(__popc(bits), lane, &total);
+        if (lane == 0) warp_sums[wib] = total;
+        __syncthreads();
+        uint32_t at = e0 + found + before;
+        for (uint32_t w = 0; w < warps; ++w) {
+            if (w < wib) at += warp_sums[w];
+            found += warp_sums[w];
+        }
+        for (; bits; bits &= bits - 1) edges[at++] = (uint32_t)k + __ffs(bits) - 1;
+        __syncthreads();
+    }
+    return found;
+}
+
+// Lists of hubs and of the largest class: a CTA per task; the others: a warp per task.
+__global__ void __launch_bounds__(256) k_pending_tasks(PendingLists pl, PendingWork pw,
+                                                       const uint32_t* __restrict__ off,
+                                                       const uint32_t* __restrict__ lo_off, const uint8_t* sim,
+                                                       uint32_t slices, uint32_t* __restrict__ edges,
+                                                       uint32_t* __restrict__ counts) {
+    __shared__ uint32_t warp_sums[8], place;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t even = (uint32_t)min(*pw.total / slices + 1, 0x7FFFFFFFull);
+    // slices for `found` pending edges of task t
+    auto cut = [&](const CnTask& t, uint32_t work, uint32_t found) {
+        const uint32_t dv = off[t.v + 1] - off[t.v], all = lo_off[t.v + 1] - lo_off[t.v];
+        const uint64_t mine = (uint64_t)work * (t.e1 - t.e0) / all;          // the task's share of its pivot's
+        const uint32_t aim = max(even, max(kPendingMinWork, dv / 16));       // 4 d_v entries at least
+        return (uint32_t)min(mine / aim + 1, (uint64_t)((found + 7) / 8));
+    };
+    for (int a = 2; a < kPendingLists; ++a)
+        for (uint32_t i = blockIdx.x; i < pl.count[a]; i += gridDim.x) {
+            const CnTask t = pl.tasks[a][i];
+            const uint32_t work = pw.pivot[t.v];
+            if (!work) continue;                                             // the same in every thread
+            const uint32_t found = gather_pending_cta(sim, t.e0, t.e1, edges, lane, warp_sums);
+            const uint32_t n = cut(t, work, found);
+            if (threadIdx.x == 0 && n) place = atomicAdd(&counts[a], n);
+            __syncthreads();
+            for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) pl.out[a][place + q] = TaskSlice{i, q, n, found};
+            __syncthreads();
+        }
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + wib, warps = gridDim.x * (blockDim.x >> 5);
+    for (int a = 0; a < 2; ++a)
+        for (uint32_t i = warp; i < pl.count[a]; i += warps) {
+            const CnTask t = pl.tasks[a][i];
+            const uint32_t work = pw.pivot[t.v];
+            if (!work) continue;
+            const uint32_t found = gather_pending_warp(sim, t.e0, t.e1, edges, lane);
+            const uint32_t n = cut(t, work, found);
+            uint32_t at = 0;
+            if (lane == 0 && n) at = atomicAdd(&counts[a], n);
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            for (uint32_t q = lane; q < n; q += 32) pl.out[a][at + q] = TaskSlice{i, q, n, found};
+        }
 }
 
 }  // namespace scan

@@ -381,10 +381,10 @@ scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
     cudaStream_t s = d->stream;
     uint32_t* counts = d->dflags + 1;
     const unsigned pg = (unsigned)((d->n + 255) / 256);
-    SCAN_CUDA(cudaMemsetAsync(counts, 0, (5 + kNumBigClasses) * sizeof(uint32_t), s));
+    SCAN_CUDA(cudaMemsetAsync(counts, 0, (4 + kNumBigClasses) * sizeof(uint32_t), s));
     k_plan<<<pg, 256, 0, s>>>(d->n, d->off, d->lo_off, d->work, d->tailc, pp, counts, nullptr, nullptr, nullptr,
-                              nullptr, nullptr, nullptr);
-    uint32_t hc[5 + kNumBigClasses];
+                              nullptr, nullptr);
+    uint32_t hc[4 + kNumBigClasses];
     SCAN_CUDA(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s));
     SCAN_CUDA(cudaStreamSynchronize(s));
     // task arrays: reuse the current ones when large enough
@@ -400,24 +400,25 @@ scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
         d->nbig[c] = hc[1 + c];
         SCAN_TRY(ensure(&d->big[c], &d->cap_big[c], d->nbig[c]));
     }
-    d->nbmp = hc[1 + kNumBigClasses];
-    d->nhmid = hc[2 + kNumBigClasses];
-    d->has_split = hc[3 + kNumBigClasses] > 0;
-    d->nmiss = hc[4 + kNumBigClasses];               // lower edges of split pivots
+    d->nhub = hc[1 + kNumBigClasses];
+    d->has_split = hc[2 + kNumBigClasses] > 0;
+    d->nmiss = hc[3 + kNumBigClasses];               // lower edges of split pivots
     if (d->nmiss) SCAN_TRY(ensure(&d->miss, &d->cap_miss, d->nmiss));
-    SCAN_TRY(ensure(&d->hubs, &d->cap_hubs, d->nhmid + d->nbmp));   // mid hubs, then the larger hubs
-    d->hmid = d->hubs;
-    d->bmp = d->hubs + d->nhmid;
+    SCAN_TRY(ensure(&d->hubs, &d->cap_hubs, d->nhub));
     if (d->sk) {
-        uint64_t total = (uint64_t)d->nhmid + d->nbmp;
+        uint64_t total = d->nhub;
         for (int c = 0; c < kNumBigClasses; ++c) total += d->nbig[c];
+        // Fused runs leave cn alone, so its memory holds the pending edges; with split pivots the
+        // list kernels still put their counts there.
+        if (d->has_split && (!d->pend_edges || d->pend_edges == d->cn)) SCAN_TRY(dalloc(d, &d->pend_edges, d->E));
+        if (!d->pend_edges) d->pend_edges = d->cn;
         if (total)
             SCAN_TRY(ensure(&d->pend_lists, &d->cap_pend,
                             (uint32_t)(total + (uint64_t)kPendingLists * kPendingSlices * d->num_sms)));
     }
     SCAN_CUDA(cudaMemsetAsync(counts, 0, sizeof(hc), s));
     k_plan<<<pg, 256, 0, s>>>(d->n, d->off, d->lo_off, d->work, d->tailc, pp, counts, d->small_piv, d->big[0],
-                              d->big[1], d->big[2], d->bmp, d->hmid);
+                              d->big[1], d->big[2], d->hubs);
     SCAN_CUDA(cudaGetLastError());
     d->plan = pp;
     return SCAN_OK;
@@ -443,11 +444,11 @@ static scan_status build_large_sketches(DeviceGraph* d, const SketchPlan& plan, 
     if (plan.list_hub) {
         SCAN_CUDA(cudaFuncSetAttribute(k_sketch_build_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubSmem));
         k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_hub, (uint64_t)d->num_sms), 1024, kHubSmem, s>>>(
-            hub, plan.list_hub, d->off, d->adj, d->sk_info, d->sk);
+            hub, plan.list_hub, d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
     }
     if (plan.list_mid)
         k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_mid, (uint64_t)d->num_sms * 8), 256, kMidSmem,
-                             s>>>(mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk);
+                             s>>>(mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
     SCAN_CUDA(cudaGetLastError());
     return SCAN_OK;
 }
@@ -548,12 +549,18 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         for (int c = sketch_log(kSmallDeg) + 1 - kSketchMinLog; c < kSketchClasses; ++c) use_sketch |= hcls[c] > 0;
     }
     if (use_sketch) {
-        for (int c = kSketchClasses; c-- > 0;) {   // largest heaps first: each aligned to its size
-            sk_plan.base[c] = (uint32_t)sk_units;
-            sk_units += (uint64_t)hcls[c] << (c + 1);
+        uint32_t ranked = 0;
+        uint32_t holders[kSketchClasses];                  // vertices that have a bitmap of the size
+        for (int c = kSketchClasses; c-- > 0;) {           // ranks descend by size
+            sk_plan.first[c] = ranked;
+            holders[c] = ranked += hcls[c];
             const int l = c + kSketchMinLog;
             if (l > kSketchMidLog) sk_plan.list_hub += hcls[c];
             else if (l > kSketchWarpLog) sk_plan.list_mid += hcls[c];
+        }
+        for (int c = 0; c < kSketchClasses; ++c) {         // arrays on 128-byte boundaries
+            d->sk_levels.base[c] = (uint32_t)sk_units;
+            sk_units += (((uint64_t)holders[c] << c) + 7) & ~7ull;
         }
         if (sk_units && sk_units < 0xFFFFFFF0ull && (!sketch_budget || sk_units * 16 + 13 * n <= sketch_budget)) {
             SCAN_TRY(dalloc(d.get(), &d->sk, sk_units));
@@ -654,7 +661,7 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
             }
             if (d->sk && vcut[c + 1] > vcut[c])
                 k_sketch_build_small<<<grid_for(d.get(), vcut[c + 1] - vcut[c], kSketchWarps * 32), kSketchWarps * 32, 0,
-                                       s2>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk);
+                                       s2>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
         }
         SCAN_CUDA(cudaEventRecord(d->ev[1], s));   // end of the copies
         // The orientation continues on s; the larger vertices' bitmaps are built beside it and
@@ -701,10 +708,10 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     pp.small_deg = kSmallDeg;
     pp.small_strategy = kSmallSerial;
     pp.bitmap_min_deg = kBitmapMinDeg;
+    SCAN_TRY(dalloc(d.get(), &d->cn, d->E));
     SCAN_TRY(plan_tasks(d.get(), pp));
 
     // Result and scratch arrays.
-    SCAN_TRY(dalloc(d.get(), &d->cn, d->E));
     SCAN_TRY(dalloc(d.get(), &d->np_tab, kPruneTable));
     uint8_t* rs_mem = nullptr;
     SCAN_TRY(dalloc(d.get(), &rs_mem, run_scratch_bytes(d->n, d->E)));
@@ -739,14 +746,13 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
 
 // Kernel attributes and occupancies, found once per device (so capturing launch_cn into a
 // CUDA graph queries nothing).  [g] is 1 for the instantiations with per-graph parameters.
-static bool g_attr_set[64][2] = {};         // k_cn_big: [after the sketches]
+static bool g_attr_set[64][2][2] = {};      // k_cn_big, [g][after the sketches]
 static bool g_attr_bitmap[64][2][2] = {};   // [g][after the sketches]
-static bool g_attr_filter[64][2][2] = {};   // [g][mid hubs]
-static int g_per_sm[64][2][kNumBigClasses] = {};            // k_cn_big, [after the sketches][hash class]
+static bool g_attr_filter[64][2] = {};      // k_cn_filter_classes, [g]
+static int g_per_sm[64][2][2][kNumBigClasses] = {};         // k_cn_big, [g][after the sketches][hash class]
 static int g_per_sm_sketch[64][2] = {};                      // k_sketch_filter
-static int g_per_sm_hub_filter[64][2] = {};                 // k_cn_filter on the mid hubs
-static int g_per_sm_filter[64][2][kNumBigClasses][2] = {};  // k_cn_filter, [g][class][largest class 2
-                                                            // at the default chunk, or at the cap]
+static int g_per_sm_filter[64][2][kNumBigClasses][2] = {};  // k_cn_filter_classes, [g][class][largest class at
+                                                            // the default chunk, or at the cap]
 
 // A stride coprime to n near n / golden ratio: i * stride mod n visits 0..n-1 once each,
 // consecutive draws far apart in the array (k_cn_big's order for split pivots).
@@ -783,11 +789,11 @@ static scan_status launch_sketch_filter(DeviceGraph* d, uint32_t* launches, cons
     const uint64_t chunk = std::min<uint64_t>(kSketchBatch, std::max<uint64_t>(32, d->E / (warps * 8) / 32 * 32));
     const uint64_t blocks = (d->E + chunk * (kThreads / 32) - 1) / (chunk * (kThreads / 32));
     const unsigned grid = (unsigned)std::min<uint64_t>(blocks, (uint64_t)d->num_sms * per_sm);
-    kernel<<<grid, kThreads, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->sk_info, d->sk, pr, (uint32_t)chunk,
+    kernel<<<grid, kThreads, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->sk_info, d->sk, d->sk_levels, pr, (uint32_t)chunk,
                                      d->pend_counts + kPendCounts - 2, sim, pw, d->long_edges, d->cn_ctr);
     ++*launches;
     if (d->long_edges.cap) {
-        k_sketch_long<<<d->num_sms * 6, kThreads, 0, s>>>(d->long_edges, d->lo_adj, d->lo_src, d->sk_info, d->sk, sim,
+        k_sketch_long<<<d->num_sms * 6, kThreads, 0, s>>>(d->long_edges, d->lo_adj, d->lo_src, d->sk_info, d->sk, d->sk_levels, sim,
                                                           pw, d->cn_ctr);
         ++*launches;
     }
@@ -801,98 +807,73 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     const int g = kPerGraph ? 1 : 0;
     // The sketches first: they settle most edges, and the list kernels below then work on the
     // tasks with a pending edge only (pick; the counts stay on the device).
-    TaskPick pick_class[kNumBigClasses] = {}, pick_bmp{}, pick_mid{};
+    TaskPick pick_class[kNumBigClasses] = {}, pick_hub{};
     if constexpr (kPick) {
         const PendingWork pw{d->pend_pivot, d->cn_ctr + 2, d->plan.small_deg};
         SCAN_TRY(launch_sketch_filter<kPerGraph>(d, launches, pr, const_cast<uint8_t*>(fp.pend), pw));
         PendingLists pl{};
-        uint2* out = d->pend_lists;
+        TaskSlice* out = d->pend_lists;
         uint32_t longest = 0;
         auto list = [&](int a, uint32_t count, const CnTask* tasks) {
             pl.tasks[a] = tasks;
             pl.count[a] = count;
             pl.out[a] = out;
-            const TaskPick pick{out, d->pend_counts + a};
+            const TaskPick pick{out, d->pend_counts + a, d->pend_edges};
             if (count) out += count + kPendingSlices * d->num_sms;
             longest = std::max(longest, count);
             return pick;
         };
         for (int c = 0; c < kNumBigClasses; ++c) pick_class[c] = list(c, d->nbig[c], d->big[c]);
-        pick_bmp = list(kNumBigClasses, d->nbmp, d->bmp);
-        pick_mid = list(1 + kNumBigClasses, d->nhmid, d->hmid);
+        pick_hub = list(kNumBigClasses, d->nhub, d->hubs);
         if (longest) {
-            k_pending_tasks<<<grid_for(d, longest, 256, 4), 256, 0, s>>>(pl, pw, d->off, d->lo_off,
-                                                                         kPendingSlices * d->num_sms, d->pend_counts);
+            const unsigned grid = (unsigned)grid_for(d, (uint64_t)longest * 32, 256, 8);
+            k_pending_tasks<<<grid, 256, 0, s>>>(pl, pw, d->off, d->lo_off, run.sim, kPendingSlices * d->num_sms,
+                                                 d->pend_edges, d->pend_counts);
             ++*launches;
         }
     }
     SCAN_CUDA(cudaEventRecord(d->ev[7], s));
-    if (!g_attr_set[d->device][kPick]) {
-        SCAN_CUDA(cudaFuncSetAttribute(k_cn_big<kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (!g_attr_set[d->device][g][kPick]) {
+        SCAN_CUDA(cudaFuncSetAttribute(k_cn_big<kPerGraph, kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(big_class_slots(kNumBigClasses - 1) * sizeof(uint32_t))));
-        g_attr_set[d->device][kPick] = true;
+        g_attr_set[d->device][g][kPick] = true;
     }
-    // One-shot fused runs (every pivot unsplit) decide most edges from an upper bound on
-    // their count (k_cn_filter); full counts and split plans use the bucketed table.
-    const bool filter = fp.sim != nullptr;
-    if (filter && !g_attr_filter[d->device][g][0]) {
+    // One-shot fused runs without sketches (every pivot unsplit) decide most edges from an upper
+    // bound on their count (k_cn_filter_classes); the others use the bucketed table.
+    const bool filter = fp.sim != nullptr && !kPick;
+    if (filter && !g_attr_filter[d->device][g]) {
         SCAN_CUDA(cudaFuncSetAttribute(k_cn_filter_classes<kPerGraph>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)filter_smem_bytes(kChunkMaxCap)));
-        SCAN_CUDA(cudaFuncSetAttribute(k_cn_filter<kPerGraph>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)filter_smem_bytes(kHubFilterMax)));
-        g_attr_filter[d->device][g][0] = true;
+        g_attr_filter[d->device][g] = true;
     }
-    // The hub kernels run on the side stream (larger hubs, then mid hubs) while the hash
-    // classes and the small pivots run on the main one, longest tasks first.  Every kernel is
-    // persistent over its own task queue and writes its own edges' counts, so none waits on
-    // another, and the CTAs of one fill the SMs that another's last tasks leave idle.  Run one
-    // after the other, those tails added up (R-MAT s22 over the stage: 14.56 ms in sequence,
-    // 13.3 ms on two streams; the larger hubs first: eps 0.2, mu 2 30.6 -> 29.8 ms).
+    // The hub kernel runs on the side stream while the hash classes and the small pivots run
+    // on the main one, longest tasks first.  Every kernel is persistent over its own task queue
+    // and writes its own edges' counts, so none waits on another, and the CTAs of one fill the
+    // SMs that another's last tasks leave idle.  Run one after the other, those tails added up
+    // (R-MAT s22, full counts: 71.7 ms in sequence, 66.6 on two streams).
     // work items of a task list: after the sketches, slices of its tasks
     auto items = [&](uint64_t tasks) { return fp.pend ? tasks + kPendingSlices * d->num_sms : tasks; };
-    const bool hubs = d->nbmp || d->nhmid;
+    const bool hubs = d->nhub > 0;
     cudaStream_t sh = hubs ? d->side : s;
     if (hubs) {
         SCAN_CUDA(cudaEventRecord(d->fork, s));
         SCAN_CUDA(cudaStreamWaitEvent(sh, d->fork, 0));
     }
-    // Hubs.  The mid hubs of a one-shot run go to k_cn_filter like the hash classes; the
-    // larger hubs, and every hub when counting in full, to the hot-id bitmap kernel (full
-    // counts: one launch over both task lists, d->hmid being followed by d->bmp in one array).
-    // Hubs above kHubFilterMax stay off k_cn_filter: edges between two hubs of degree above
-    // 46,339 have no early-stop threshold (the reference's int square may wrap), so the
-    // filter would end in an exact recount by binary search over the whole list.
-    const bool mid_on_filter = filter && d->nhmid;
-    // With split pivots and sketches the two hub lists are picked separately: two launches.
-    for (int part = 0; part < (mid_on_filter || !fp.pend ? 1 : 2); ++part) {
-        const bool both = !mid_on_filter && !fp.pend;
-        const uint32_t nbitmap = both ? d->nbmp + d->nhmid : part == 0 ? d->nbmp : d->nhmid;
-        const CnTask* bitmap_tasks = both || part == 1 ? d->hmid : d->bmp;
-        if (!nbitmap) continue;
+    // Hubs stay off the filter kernel: what the sketches leave open there is close to its
+    // threshold, where the filter's bound decides little and ends in an exact recount by binary
+    // search (hubs of 6,145-12,288 entries, R-MAT s20 at eps 0.2: 3.66 ms, on the bitmap kernel
+    // 0.9).
+    if (d->nhub) {
         const size_t smem = (kHotBits / 32 + kTailSlots) * sizeof(uint32_t);
         if (!g_attr_bitmap[d->device][g][kPick]) {
             SCAN_CUDA(cudaFuncSetAttribute(k_cn_bitmap<kPerGraph, kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem));
             g_attr_bitmap[d->device][g][kPick] = true;
         }
-        const uint64_t grid = std::min<uint64_t>(items(nbitmap), (uint64_t)d->num_sms);
+        const uint64_t grid = std::min<uint64_t>(items(d->nhub), (uint64_t)d->num_sms);
         k_cn_bitmap<kPerGraph, kPick><<<(unsigned)grid, kBitmapThreads, smem, sh>>>(
-            bitmap_tasks, nbitmap, d->task_queue + (part == 0 ? 3 : 4), d->off, d->radj, d->lo_adj, d->cn,
-            d->long_words, pr, d->cn_ctr, fp, pr.on, part == 0 ? pick_bmp : pick_mid);
-        ++*launches;
-    }
-    if (mid_on_filter) {
-        const int threads = 512;
-        const size_t smem = filter_smem_bytes(kHubFilterMax);
-        int& per_sm = g_per_sm_hub_filter[d->device][g];
-        if (per_sm == 0) {
-            SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_filter<kPerGraph>, threads, smem));
-            per_sm = std::max(per_sm, 1);
-        }
-        const uint64_t grid = std::min<uint64_t>(items(d->nhmid), (uint64_t)d->num_sms * per_sm);
-        k_cn_filter<kPerGraph><<<(unsigned)grid, threads, smem, sh>>>(
-            d->hmid, d->nhmid, kHubFilterMax, d->task_queue + 4, d->off, d->adj,
-            d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 1u, pick_mid);   // hubs: strided batches
+            d->hubs, d->nhub, d->task_queue + 3, d->off, d->radj, d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp,
+            pr.on, pick_hub);
         ++*launches;
     }
     for (int c = kNumBigClasses - 1; c >= 0; --c) {   // longest tasks first
@@ -911,22 +892,22 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
                 const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
                 k_cn_filter_classes<kPerGraph><<<(unsigned)grid, threads, smem, s>>>(
                     d->big[c], d->nbig[c], entries, d->task_queue + c, d->off, d->adj,
-                    d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp, 0u, pick_class[c]);
+                    d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp);
             } else {
                 const size_t smem = big_class_slots(c) * sizeof(uint32_t);
-                int& per_sm = g_per_sm[d->device][kPick][c];
+                int& per_sm = g_per_sm[d->device][g][kPick][c];
                 if (per_sm == 0) {
-                    SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_big<kPick>, threads, smem));
+                    SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_big<kPerGraph, kPick>, threads, smem));
                     per_sm = std::max(per_sm, 1);
                 }
                 const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
-                k_cn_big<kPick><<<(unsigned)grid, threads, smem, s>>>(d->big[c], d->nbig[c], big_class_slots(c),
+                k_cn_big<kPerGraph, kPick><<<(unsigned)grid, threads, smem, s>>>(d->big[c], d->nbig[c], big_class_slots(c),
                                                                 d->task_queue + c, d->off,
                                                                 d->adj, d->lo_adj, d->cn, d->long_words, pr,
                                                                 d->cn_ctr, pr.on ? d->miss : nullptr, d->nmiss,
                                                                 !pr.on || !d->nmiss ? 0u
                                                                 : fp.pend ? kSpreadPrime : spread_stride(d->nbig[c]),
-                                                                fp.pend, pick_class[c]);
+                                                                fp, pick_class[c]);
             }
             ++*launches;
         }
@@ -1086,10 +1067,10 @@ static void cn_kernel_times(DeviceGraph* d, scan_stats* st) {
     st->ms_cn_kernel[0] = ev_ms(d->ev[9], d->ev[8]);
     for (int c = 0; c < kNumBigClasses; ++c)
         st->ms_cn_kernel[1 + c] = ev_ms(c == kNumBigClasses - 1 ? d->ev[7] : d->ev[10 + c], d->ev[9 + c]);
-    st->ms_cn_kernel[4] = d->nbmp || d->nhmid ? ev_ms(d->ev[7], d->ev[15]) : 0.0;
+    st->ms_cn_kernel[4] = d->nhub ? ev_ms(d->ev[7], d->ev[15]) : 0.0;
     st->cn_work_items[0] = d->nsmall;
     for (int c = 0; c < kNumBigClasses; ++c) st->cn_work_items[1 + c] = d->nbig[c];
-    st->cn_work_items[4] = d->nbmp + d->nhmid;
+    st->cn_work_items[4] = d->nhub;
 }
 
 // predicate -> cores -> union-find -> attach -> classify, on cached cn.  Queued on s with
