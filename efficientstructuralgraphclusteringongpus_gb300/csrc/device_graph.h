@@ -80,6 +80,8 @@ struct DeviceGraph {
     uint32_t* lo_off = nullptr;
     uint32_t* lo_adj = nullptr;
     uint32_t* lo_src = nullptr;
+    uint32_t* lowbits = nullptr;   // m / 32 words: entry j is a lower neighbour (null when m = 0)
+    uint32_t* wpre = nullptr;      // exclusive prefix of their popcounts
     unsigned long long* work = nullptr;
     unsigned long long* cn_ctr = nullptr;
     uint32_t* task_queue = nullptr;        // launch_cn: one task counter per similarity kernel
@@ -152,6 +154,10 @@ struct BatchParams;
 scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune = nullptr,
                       const RunScratch* run = nullptr, const BatchParams* bp = nullptr);
 bool one_shot_predicate(const DeviceGraph* d);
+// Counts of every edge into d->cn by triangles (kernels_tri.cuh), on d->stream, waiting for it.
+// The counts in the reference's order are copied to out_host unless it is null.  Working
+// memory comes from the device-buffer cache; where there is none left, by launch_cn.
+scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host);
 // Rebuild the similarity tasks for plan parameters pp.
 scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp);
 // Time the similarity stage under plan settings (small-pivot strategy and degree cut, task

@@ -33,6 +33,7 @@
 #include "kernels_cn.cuh"
 #include "kernels_orient.cuh"
 #include "kernels_sketch.cuh"
+#include "kernels_tri.cuh"
 
 namespace scan {
 
@@ -74,24 +75,18 @@ __global__ void k_fill_u32(uint32_t* p, uint64_t n, uint32_t x) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) p[i] = x;
 }
 
-// Reference edge order (GPUSCAN++/Graph.cpp:87-111): edge {u lower, v higher} has id
-// P[u] + (rank of v among the higher neighbours of u), P = prefix of higher-neighbour
-// counts.  Used to return cn[] in the order the reference's Edge_u/Edge_v use.
-__global__ void k_higher_count(uint32_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ lo_off,
-                               uint32_t* __restrict__ hcnt) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-        hcnt[v] = (off[v + 1] - off[v]) - (lo_off[v + 1] - lo_off[v]);
-}
-
+// cn[] in the reference's edge order (GPUSCAN++/Graph.cpp:87-111): edge {u lower, v higher} has
+// id P[u] + (rank of v among the higher neighbours of u), P = prefix of the higher-neighbour
+// counts, which is off[u] - lo_off[u].
 __global__ void k_to_reference_order(uint64_t E, const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
                                      const uint32_t* __restrict__ lo_off, const uint32_t* __restrict__ lo_adj,
-                                     const uint32_t* __restrict__ lo_src, const uint32_t* __restrict__ hpre,
-                                     const uint32_t* __restrict__ cn, uint32_t* __restrict__ out) {
+                                     const uint32_t* __restrict__ lo_src, const uint32_t* __restrict__ cn,
+                                     uint32_t* __restrict__ out) {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t u = lo_adj[e], v = lo_src[e];
         const uint32_t pos = lower_bound_u32(adj, off[u], off[u + 1], v) - off[u];        // v's index in N(u)
         const uint32_t lows = lower_bound_u32(lo_adj, lo_off[u], lo_off[u + 1], v) - lo_off[u];  // lower ones before v
-        out[hpre[u] + (pos - lows)] = cn[e];
+        out[off[u] - lo_off[u] + (pos - lows)] = cn[e];
     }
 }
 
@@ -265,31 +260,66 @@ void device_graph_free(DeviceGraph* d) {
     delete d;
 }
 
+// `bytes` of device memory from the cache or the driver; *got is the block's real size (a
+// cached one may be larger), to be given back with it.
+static scan_status cache_alloc(int device, size_t bytes, void** p, size_t* got) {
+    *got = bytes;
+    *p = cache_take(device, bytes, got);
+    if (*p) return SCAN_OK;
+    cudaError_t err = cudaMalloc(p, bytes);
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        // return cached blocks to the driver and try once more
+        scan_release_cached_memory();
+        err = cudaMalloc(p, bytes);
+    }
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        return fail(SCAN_ERR_OUT_OF_MEMORY, "cudaMalloc of " + std::to_string(bytes) +
+                                                " bytes failed: " + cudaGetErrorString(err));
+    }
+    return SCAN_OK;
+}
+
+static size_t block_bytes(uint64_t count, size_t size) { return (std::max<uint64_t>(count, 1) * size + 255) & ~size_t(255); }
+
 template <typename T>
 static scan_status dalloc(DeviceGraph* d, T** p, uint64_t count) {
-    const size_t want = std::max<uint64_t>(count, 1) * sizeof(T);
-    const size_t bytes = (want + 255) & ~size_t(255);
-    size_t got = bytes;                    // a cached block may be larger: keep its real size
-    void* q = cache_take(d->device, bytes, &got);
-    if (!q) {
-        cudaError_t err = cudaMalloc(&q, bytes);
-        if (err != cudaSuccess) {
-            cudaGetLastError();
-            // return cached blocks to the driver and try once more
-            scan_release_cached_memory();
-            err = cudaMalloc(&q, bytes);
-        }
-        if (err != cudaSuccess) {
-            cudaGetLastError();
-            return fail(SCAN_ERR_OUT_OF_MEMORY, "cudaMalloc of " + std::to_string(bytes) +
-                                                    " bytes failed: " + cudaGetErrorString(err));
-        }
-    }
+    const size_t bytes = block_bytes(count, sizeof(T));
+    size_t got = 0;
+    void* q = nullptr;
+    SCAN_TRY(cache_alloc(d->device, bytes, &q, &got));
     d->allocs.emplace_back(q, got);
     d->device_bytes += bytes;
     *p = static_cast<T*>(q);
     return SCAN_OK;
 }
+
+// Device memory for the length of a call, back to the cache at the end of its scope: no work on
+// it may be in flight then.
+class CallBuffers {
+  public:
+    explicit CallBuffers(int device) : device_(device) {}
+    ~CallBuffers() {
+        for (auto& b : blocks_) cache_give(device_, b.first, b.second);
+    }
+    CallBuffers(const CallBuffers&) = delete;
+    CallBuffers& operator=(const CallBuffers&) = delete;
+    template <typename T>
+    scan_status get(T** p, uint64_t count) {
+        size_t got = 0;
+        void* q = nullptr;
+        SCAN_TRY(cache_alloc(device_, block_bytes(count, sizeof(T)), &q, &got));
+        blocks_.emplace_back(q, got);
+        *p = static_cast<T*>(q);
+        return SCAN_OK;
+    }
+
+  private:
+    int device_;
+    std::vector<std::pair<void*, size_t>> blocks_;
+};
 
 static int grid_for(const DeviceGraph* d, uint64_t items, int threads, int per_sm = 8) {
     uint64_t g = (items + threads - 1) / threads;
@@ -590,8 +620,8 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     const uint64_t fill_tiles = (m + kFillTile - 1) / kFillTile;
     uint32_t* tile_v = nullptr;                                // first vertex of each adjacency tile
     SCAN_TRY(dalloc(d.get(), &tile_v, fill_tiles + 1));
-    uint32_t* lowbits = nullptr;                               // one bit per entry: lower neighbour
-    SCAN_TRY(dalloc(d.get(), &lowbits, m / 32 + 2));
+    SCAN_TRY(dalloc(d.get(), &d->lowbits, m / 32 + 2));
+    uint32_t* lowbits = d->lowbits;
     if (bitmap_path) {
         SCAN_TRY(dalloc(d.get(), &d->hot, n));
         SCAN_TRY(dalloc(d.get(), &d->radj, m + kAdjPad));
@@ -690,8 +720,9 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     SCAN_TRY(dalloc(d.get(), &d->lo_src, d->E));
     if (fill_tiles) {   // word prefix of the lower bits, then the fill
         const uint64_t nwords = (m + 31) / 32;
-        uint32_t *wpre = nullptr, *wsums = nullptr;
-        SCAN_TRY(dalloc(d.get(), &wpre, nwords + 1));
+        uint32_t* wsums = nullptr;
+        SCAN_TRY(dalloc(d.get(), &d->wpre, nwords + 1));
+        uint32_t* wpre = d->wpre;
         SCAN_TRY(dalloc(d.get(), &wsums, (nwords + kScanTile - 1) / kScanTile + 1));
         SCAN_TRY(device_scan(d.get(), lowbits, nwords, wpre, wsums, true));
         k_fill_tiles<<<grid_for(d.get(), fill_tiles * kFillThreads, kFillThreads), kFillThreads, 0, s>>>(
@@ -1112,6 +1143,84 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     return SCAN_OK;
 }
 
+// One write per 4 KB: the pages are mapped before a device-to-host copy lands in them.
+static void touch_pages(void* p, size_t bytes) {
+    if (!p) return;
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+}
+
+// launch_cn's counts in the reference's order (the working memory of the triangles is missing).
+static scan_status full_counts_by_lists(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
+    cudaStream_t s = d->stream;
+    CallBuffers mem(d->device);
+    uint32_t* ref = nullptr;
+    if (out_host) SCAN_TRY(mem.get(&ref, d->E));
+    SCAN_CUDA(cudaEventRecord(d->ev[3], s));
+    const scan_status st = launch_cn(d, launches);
+    cudaEventRecord(d->ev[4], s);
+    if (st == SCAN_OK && out_host && d->E) {
+        k_to_reference_order<<<grid_for(d, d->E, 256), 256, 0, s>>>(d->E, d->off, d->adj, d->lo_off, d->lo_adj, d->lo_src,
+                                                                    d->cn, ref);
+        ++*launches;
+        cudaMemcpyAsync(out_host, ref, d->E * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    }
+    const cudaError_t err = cudaStreamSynchronize(s);      // before the buffers go back
+    if (st != SCAN_OK) return st;
+    SCAN_CUDA(err);
+    SCAN_CUDA(cudaGetLastError());
+    return SCAN_OK;
+}
+
+scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
+    cudaStream_t s = d->stream;
+    const uint64_t E = d->E;
+    CallBuffers mem(d->device);
+    // counters, 256 bytes apart: [0] numbers of small pivots and of slices, then their queues
+    constexpr int kSpan = 64;
+    uint32_t *hi_adj = nullptr, *cnt = nullptr, *small = nullptr, *ctr = nullptr;
+    uint2* big = nullptr;
+    const uint64_t slices = E / kTriSliceEdges + d->m / kSmallDeg + 1;   // at most one short slice per larger pivot
+    scan_status st = mem.get(&hi_adj, E + kAdjPad);
+    if (st == SCAN_OK) st = mem.get(&cnt, E);
+    if (st == SCAN_OK) st = mem.get(&small, std::min<uint64_t>(d->n, E));
+    if (st == SCAN_OK) st = mem.get(&big, slices);
+    if (st == SCAN_OK) st = mem.get(&ctr, 3 * kSpan);
+    if (st == SCAN_ERR_OUT_OF_MEMORY) {
+        clear_error();
+        return full_counts_by_lists(d, launches, out_host);
+    }
+    if (st != SCAN_OK) return st;
+    auto queue = [&]() -> scan_status {
+        SCAN_CUDA(cudaEventRecord(d->ev[3], s));
+        SCAN_CUDA(cudaMemsetAsync(cnt, 0, std::max<uint64_t>(E, 1) * sizeof(uint32_t), s));
+        SCAN_CUDA(cudaMemsetAsync(ctr, 0, 3 * kSpan * sizeof(uint32_t), s));
+        if (E) {
+            k_fill_higher<<<grid_for(d, d->m, 256), 256, 0, s>>>(d->m, d->adj, d->lowbits, d->wpre, hi_adj);
+            k_tri_plan<<<grid_for(d, d->n, 256), 256, 0, s>>>(d->n, d->off, d->lo_off, ctr, small, big);
+            const unsigned gb = (unsigned)std::min<uint64_t>(slices, (uint64_t)d->num_sms * kTriCtas);
+            k_tri_big<<<gb, kTriWarps * 32, 0, s>>>(big, ctr, ctr + kSpan, d->off, d->lo_off, d->lo_adj, hi_adj, cnt);
+            k_tri_small<<<grid_for(d, (uint64_t)d->n * 32, kTriWarps * 32, 6), kTriWarps * 32, 0, s>>>(
+                small, ctr, ctr + 2 * kSpan, d->off, d->lo_off, d->lo_adj, hi_adj, cnt);
+            k_from_reference_order<<<grid_for(d, E, 256), 256, 0, s>>>(E, d->off, d->lo_off, d->lo_adj, d->lo_src, hi_adj,
+                                                                      cnt, d->cn);
+            *launches += 5;
+        }
+        SCAN_CUDA(cudaEventRecord(d->ev[4], s));
+        SCAN_CUDA(cudaGetLastError());
+        if (out_host && E) {
+            touch_pages(out_host, E * sizeof(uint32_t));   // while the kernels run (see run_resident)
+            SCAN_CUDA(cudaMemcpyAsync(out_host, cnt, E * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        }
+        return SCAN_OK;
+    };
+    st = queue();
+    const cudaError_t err = cudaStreamSynchronize(s);      // before the buffers go back
+    if (st != SCAN_OK) return st;
+    SCAN_CUDA(err);
+    return SCAN_OK;
+}
+
 scan_status compute_tau(DeviceGraph* d) {
     if (!d->tau) SCAN_TRY(dalloc(d, &d->tau, 2 * std::max<uint64_t>(d->E, 1)));
     if (d->E) k_tau<<<grid_for(d, d->E, 256), 256, 0, d->stream>>>(d->E, d->lo_adj, d->lo_src, d->off, d->cn, d->tau);
@@ -1148,13 +1257,6 @@ static scan_status ensure_device(scan_graph* g, int device, scan_stats* st) {
 // Full run on a resident graph: cn (unless cached and reuse_cn), then the cluster stages,
 // then D2H of labels/roles.  Counts computed here skip the edges the degree prune rules
 // out at this eps, so they do not fill the cache: cn_valid is left false.
-// One write per 4 KB: the pages are mapped before a device-to-host copy lands in them.
-static void touch_pages(void* p, size_t bytes) {
-    if (!p) return;
-    volatile char* c = static_cast<volatile char*>(p);
-    for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
-}
-
 static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bool reuse_cn, int32_t* out_label,
                                 uint8_t* out_role, scan_stats* st) {
     std::lock_guard<std::mutex> lock(d->mu);
@@ -1339,39 +1441,15 @@ scan_status scan_common_neighbors(scan_graph* g, int device, uint32_t* out_cn, s
     DeviceGraph* d = g->dev;
     std::lock_guard<std::mutex> lock(d->mu);
     SCAN_CUDA(cudaSetDevice(d->device));
-    cudaStream_t s = d->stream;
     uint32_t launches = 0;
-    SCAN_CUDA(cudaEventRecord(d->ev[3], s));
-    SCAN_TRY(launch_cn(d, &launches));
-    SCAN_CUDA(cudaEventRecord(d->ev[4], s));
+    d->cn_valid = false;
+    SCAN_TRY(full_counts(d, &launches, out_cn));
     d->cn_valid = true;
-    // Reorder to the reference's edge ids.
-    uint32_t *hcnt = nullptr, *hpre = nullptr, *sums = nullptr, *ref = nullptr;
-    SCAN_CUDA(cudaMallocAsync(&hcnt, d->n * sizeof(uint32_t), s));
-    SCAN_CUDA(cudaMallocAsync(&hpre, (d->n + 1) * sizeof(uint32_t), s));
-    SCAN_CUDA(cudaMallocAsync(&sums, ((d->n + kScanTile) / kScanTile + 1) * sizeof(uint32_t), s));
-    SCAN_CUDA(cudaMallocAsync(&ref, std::max<uint64_t>(d->E, 1) * sizeof(uint32_t), s));
-    k_higher_count<<<grid_for(d, d->n, 256), 256, 0, s>>>(d->n, d->off, d->lo_off, hcnt);
-    scan_status st = device_scan(d, hcnt, d->n, hpre, sums);
-    if (st == SCAN_OK) {
-        k_to_reference_order<<<grid_for(d, d->E, 256), 256, 0, s>>>(d->E, d->off, d->adj, d->lo_off, d->lo_adj,
-                                                                    d->lo_src, hpre, d->cn, ref);
-        touch_pages(out_cn, d->E * sizeof(uint32_t));   // while the kernels run (see run_resident)
-        cudaMemcpyAsync(out_cn, ref, d->E * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    }
-    cudaFreeAsync(hcnt, s);
-    cudaFreeAsync(hpre, s);
-    cudaFreeAsync(sums, s);
-    cudaFreeAsync(ref, s);
-    SCAN_CUDA(cudaStreamSynchronize(s));
-    SCAN_CUDA(cudaGetLastError());
-    if (st) return st;
     if (stats) {
         stats->n = d->n;
         stats->num_edges = d->E;
         stats->ms_similarity = ev_ms(d->ev[3], d->ev[4]);
-        cn_kernel_times(d, stats);
-        stats->kernel_launches += launches + 5;
+        stats->kernel_launches += launches;
     }
     return SCAN_OK;
 }

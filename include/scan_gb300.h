@@ -81,18 +81,19 @@ typedef struct scan_stats {
     double ms_cluster;          /* core flags, union-find, attach, hub/outlier                */
     double ms_d2h;              /* result copies                                              */
     double ms_total;            /* first event to last event of the run                       */
-    double ms_cn_kernel[5];     /* similarity-stage kernels: small pivots; the three hash-table
-                                   classes (1024 / 4096 / chunk entries); the hubs (mid hubs
-                                   and larger hubs together).  The hubs run on a second stream
-                                   beside the others, so these intervals overlap: each is its
-                                   kernel's span on its own stream                             */
+    double ms_cn_kernel[5];     /* list kernels of the similarity stage (a one-shot run's bitmap
+                                   kernels before them are not among these): small pivots; the
+                                   three hash-table classes (1024 / 4096 / chunk entries); the
+                                   hubs.  The hubs run on a second stream beside the others, so
+                                   these intervals overlap: each is its kernel's span on its own
+                                   stream.  0 for scan_common_neighbors, which counts by
+                                   triangles                                                   */
     uint64_t cn_work_items[5];  /* pivots (small class) or tasks (the others) of each           */
     uint32_t kernel_launches;   /* kernels this library launched for the run                  */
     uint32_t reserved;
-    uint64_t cn_words;          /* 16-byte list words the similarity kernels read (0 when the
-                                   cached counts were used)                                  */
-    uint64_t cn_edges_counted;  /* edges whose lower list was read: all of them for the cached
-                                   counts, those the degree prune leaves in a one-shot run   */
+    uint64_t cn_words;          /* 16-byte words of bitmaps (the lower endpoint's) and lists that
+                                   the similarity kernels read (0 when cached counts were used) */
+    uint64_t cn_edges_counted;  /* edges the degree prune leaves in a one-shot run             */
 } scan_stats;
 
 /* ---- errors ------------------------------------------------------------------------- */
