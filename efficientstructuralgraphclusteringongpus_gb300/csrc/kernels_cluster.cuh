@@ -166,25 +166,66 @@ __device__ __forceinline__ bool uf_union(int32_t* parent, int32_t a, int32_t b, 
     return false;
 }
 
+// Edges of one pivot v are consecutive, so a warp holds runs of them.  Hanging v's root under
+// each lower neighbour's in turn would let one CAS per round succeed; instead the lanes of a
+// run agree on the smallest of their roots and hang their own root under that (all different
+// words), the first lane v's root as well.  Edges whose endpoints already point to one vertex
+// end after two loads.  Communities of 6M edges: 0.29 -> UNIONB ms; 30 served queries 2.24 -> UNIONS.
 __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
                         const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
     if (!*(volatile uint32_t*)&ctr->any_core) return;   // no core: nothing to join
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
-        if (!sim[e]) continue;
-        const int32_t u = (int32_t)lo_adj[e], v = (int32_t)lo_src[e];
-        if (parent[u] < 0 || parent[v] < 0) continue;   // core-core only (cores never change)
-        if (!uf_union(parent, u, v, limit)) atomicOr(&ctr->error_flags, kErrUnionFindLimit);
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t e0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); e0 < E; e0 += stride) {
+        const uint64_t e = e0 + lane;
+        int32_t u = 0, v = 0;
+        bool join = false;
+        if (e < E && sim[e]) {
+            u = (int32_t)lo_adj[e];
+            v = (int32_t)lo_src[e];
+            const int32_t pu = parent[u], pv = parent[v];
+            join = pu >= 0 && pv >= 0 && pu != pv;      // core-core only (cores never change)
+        }
+        if (!__any_sync(kFull, join)) continue;
+        if (join) {
+            u = uf_find(parent, u);
+            const int32_t rv = uf_find(parent, v);
+            join = u != rv;
+        }
+        const uint32_t run = __match_any_sync(kFull, join ? (uint32_t)v : kEmpty);
+        if (join) {
+            const bool first = (__ffs(run) - 1) == (int)lane;
+            const int32_t rv = uf_find(parent, v);
+            const int32_t m = (int32_t)__reduce_min_sync(run, (uint32_t)min(u, rv));
+            bool ok = u == m || uf_union(parent, u, m, limit);
+            if (first && rv != m) ok &= uf_union(parent, rv, m, limit);
+            if (!ok) atomicOr(&ctr->error_flags, kErrUnionFindLimit);
+        }
     }
 }
 
-// Flatten by pointer jumping: round r sets parent[v] = parent[parent[v]] for every core and
-// raises flags[r] if any pointer moved.  The host queues enough rounds for any depth
-// (ceil(log2 n) + 2); a round whose predecessor moved nothing returns at once, so the pass
+// Flatten by pointer jumping: a round moves parent[v] of every core up to kJumpSteps ancestors on
+// and raises flags[r] if any pointer moved, so the distance a pointer spans grows by that
+// factor per round.  The host queues enough rounds for any depth (ceil(log16 n) + 2: eight for
+// 4M vertices, where steps of one took 24 launches); a round whose predecessor moved nothing returns at once, so the pass
 // needs no host synchronisation.  Every value stored is an ancestor of v in the final
 // forest and only v's own thread writes parent[v], so concurrent jumps never undo one
 // another.  (A find with path halving would not be safe here: its halving store can
 // overwrite a vertex whose root another thread has just written with an intermediate
 // ancestor.)
+constexpr int kJumpSteps = 16;
+
+// The ancestor of v up to kJumpSteps beyond p = parent[v], or its root.
+__device__ __forceinline__ int32_t jump_target(const volatile int32_t* parent, int32_t p) {
+    for (int i = 0; i < kJumpSteps; ++i) {
+        const int32_t g = parent[p];
+        if (g == p) break;
+        p = g;
+    }
+    return p;
+}
+
 __global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint32_t round) {
     if (round > 0 && *(volatile uint32_t*)&flags[round - 1] == 0) return;
     volatile int32_t* vp = parent;
@@ -192,7 +233,7 @@ __global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint3
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
         const int32_t p = vp[v];
         if (p < 0) continue;
-        const int32_t g = vp[p];
+        const int32_t g = jump_target(vp, p);
         if (g != p) {
             vp[v] = g;
             ch = 1;
@@ -209,33 +250,27 @@ __global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint3
 constexpr uint32_t kJumpBlockMax = 1u << 16;
 
 __global__ void __launch_bounds__(1024) k_jump_block(uint32_t n, int32_t* parent, uint32_t* flags, uint32_t rounds) {
+    constexpr int kPer = 8;
     volatile int32_t* vp = parent;
     for (uint32_t round = 0; round < rounds; ++round) {
         int ch = 0;
-        for (uint32_t v = threadIdx.x; v < n; v += blockDim.x) {
-            const int32_t p = vp[v];
-            if (p < 0) continue;
-            const int32_t g = vp[p];
-            if (g != p) {
-                vp[v] = g;
-                ch = 1;
-            }
+        for (uint32_t v0 = threadIdx.x; v0 < n; v0 += kPer * blockDim.x) {   // loads of kPer vertices in flight
+            int32_t p[kPer], g[kPer];
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) p[q] = v0 + q * blockDim.x < n ? vp[v0 + q * blockDim.x] : -1;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) g[q] = p[q] < 0 ? p[q] : vp[p[q]];
+#pragma unroll
+            for (int q = 0; q < kPer; ++q)
+                if (g[q] != p[q]) {
+                    vp[v0 + q * blockDim.x] = jump_target(vp, g[q]);
+                    ch = 1;
+                }
         }
         ch = __syncthreads_or(ch);
         if (threadIdx.x == 0) flags[round] = ch ? 1u : 0u;
         if (!ch) break;
     }
-}
-
-// Zeroes a run's similar-degree counts (sd may be null: already done), counters and
-// round flags in one launch.
-__global__ void k_cluster_reset(uint32_t n, int32_t* sd, RunCounters* ctr, uint32_t* flags, uint32_t nflags) {
-    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    if (sd)
-        for (uint64_t v = i0; v < n; v += stride) sd[v] = 0;
-    if (i0 < nflags) flags[i0] = 0;
-    if (ctr && i0 == 0) *ctr = RunCounters{};
 }
 
 // Border attachment: a non-core similar to a core joins that core's cluster.  The

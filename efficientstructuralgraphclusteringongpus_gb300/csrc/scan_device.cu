@@ -341,18 +341,15 @@ size_t run_scratch_bytes(uint32_t n, uint64_t E) {
            align256(4 * kMaxJumpRounds);
 }
 
-// The run counters and, after them, the round flags of a RunScratch.
-static size_t run_counter_bytes() { return align256(sizeof(RunCounters)) + 4 * kMaxJumpRounds; }
-
-// The order is relied on: role follows label, and the round flags follow the counters
-// (each padded to 256 bytes), so the serving loop copies each pair back in one transfer.
+// The order is relied on: role follows label, and the round flags follow the counters (each
+// padded to 256 bytes), so the serving loop copies each pair back in one transfer; sd comes
+// before the counters, so one memset clears what a run starts from.
 void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E) {
     char* p = static_cast<char*>(base);
     auto take = [&](size_t bytes) { char* q = p; p += align256(bytes); return q; };
     r->n = n;
     r->E = E;
     r->sim = reinterpret_cast<uint8_t*>(take(E ? E : 1));
-    r->sd = reinterpret_cast<int32_t*>(take(4ull * n));
     r->parent = reinterpret_cast<int32_t*>(take(4ull * n));
     r->bmin = reinterpret_cast<int32_t*>(take(4ull * n));
     r->bmax = reinterpret_cast<int32_t*>(take(4ull * n));
@@ -361,8 +358,15 @@ void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E) {
     r->lab = reinterpret_cast<int32_t*>(take(4ull * n));
     r->label = reinterpret_cast<int32_t*>(take(4ull * n));
     r->role = reinterpret_cast<uint8_t*>(take(n));
+    r->sd = reinterpret_cast<int32_t*>(take(4ull * n));
     r->ctr = reinterpret_cast<RunCounters*>(take(sizeof(RunCounters)));
     r->jump_flags = reinterpret_cast<uint32_t*>(take(4 * kMaxJumpRounds));
+}
+
+// Zero the similar-degree counts, the run counters and the round flags.
+static cudaError_t run_scratch_clear(const RunScratch& r, cudaStream_t s) {
+    return cudaMemsetAsync(r.sd, 0, reinterpret_cast<char*>(r.jump_flags + kMaxJumpRounds) - reinterpret_cast<char*>(r.sd),
+                           s);
 }
 
 // Limits of the bounded device loops.  Tests shrink them (scan_set_loop_limits) to make
@@ -373,8 +377,9 @@ static std::atomic<uint32_t> g_jump_cap{(uint32_t)kMaxJumpRounds};
 uint32_t union_find_limit() { return g_union_limit.load(); }
 
 uint32_t jump_rounds(uint32_t n) {
+    static_assert(kJumpSteps == 16, "four doublings per round");
     uint32_t r = 2;
-    while ((1ull << (r - 2)) < (uint64_t)n + 1 && r < (uint32_t)kMaxJumpRounds) ++r;
+    while ((1ull << (4 * (r - 2))) < (uint64_t)n + 1 && r < (uint32_t)kMaxJumpRounds) ++r;
     return std::max(1u, std::min(r, g_jump_cap.load()));
 }
 
@@ -999,8 +1004,7 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
     if (!fused || !fp.pend) SCAN_CUDA(cudaMemsetAsync(d->cn, 0, d->E * sizeof(uint32_t), s));
     if (fused || fp.pend) {
         if (!fp.pend) SCAN_CUDA(cudaMemsetAsync(run->sim, 0, d->E, s));
-        SCAN_CUDA(cudaMemsetAsync(run->sd, 0, d->n * sizeof(int32_t), s));
-        SCAN_CUDA(cudaMemsetAsync(run->ctr, 0, run_counter_bytes(), s));   // and the round flags
+        SCAN_CUDA(run_scratch_clear(*run, s));
     }
     SCAN_CUDA(cudaMemsetAsync(d->cn_ctr, 0, kStageCounters * sizeof(uint32_t), s));
     if (prune && d->nmiss) SCAN_CUDA(cudaMemsetAsync(d->miss, 0, (size_t)d->nmiss * sizeof(uint32_t), s));
@@ -1114,8 +1118,7 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     const int ge = grid_for_n(sms, E, T), gn = grid_for_n(sms, n, T);
     const uint32_t* vgid = bp ? bp->vgid : nullptr;
     if (!predicate_done) {   // a one-shot launch_cn has cleared them
-        k_cluster_reset<<<gn, T, 0, s>>>(n, r.sd, r.ctr, r.jump_flags, kMaxJumpRounds);
-        ++*launches;
+        SCAN_CUDA(run_scratch_clear(r, s));
         if (d->tau && !bp && d->cn_valid)
             k_predicate_tau<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, d->off, d->cn, d->tau, pp, r.sim, r.sd, r.ctr);
         else
