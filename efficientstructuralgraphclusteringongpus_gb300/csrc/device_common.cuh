@@ -35,6 +35,7 @@ constexpr uint32_t kErrHashFull = 2u;
 struct RunCounters {
     unsigned long long cores, clusters, hubs, outliers, borders;
     unsigned long long similar_edges, disagreements, multi_borders;
+    unsigned long long list_words, edges_counted;   // the similarity stage's totals (k_finalize)
     uint32_t error_flags;
     uint32_t any_core;      // set by k_core_init: the edge passes after it return at once when 0
     uint32_t any_member;    // set by k_label: the hub test's edge pass returns at once when 0

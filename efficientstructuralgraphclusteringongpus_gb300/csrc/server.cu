@@ -106,12 +106,9 @@ struct Slot {
     cudaEvent_t ev_start = nullptr, ev_end = nullptr;
     Query* q = nullptr;
     uint64_t arena_off = 0, arena_bytes = 0;
-    // Pinned staging.  The run scratch keeps label[n] and role[n] adjacent (label padded
-    // to 256 bytes), and the counters next to the round flags, so each pair comes back in
-    // one copy: h_res holds label then role at res_role_offset(n); h_tail the counters
-    // then the flags at kTailFlags.
-    char* h_res = nullptr;           // capacity for n_cap vertices
-    char* h_tail = nullptr;
+    // Pinned staging for n_cap vertices: a run's results come back in one copy (res_role and
+    // the following give the offsets).
+    char* h_res = nullptr;
     uint32_t n_cap = 0;
     std::atomic<bool> gpu_done{false};
     bool launching = false;          // assigned to q, CUDA work being queued (outside the lock)
@@ -161,12 +158,6 @@ void CUDART_CB on_slot_done(void* arg) {
     delete pair;
 }
 
-size_t pad256(size_t x) { return (x + 255) & ~size_t(255); }
-size_t res_role_offset(uint32_t n) { return pad256(4ull * n); }
-size_t res_bytes(uint32_t n) { return res_role_offset(n) + n; }
-const size_t kTailFlags = pad256(sizeof(RunCounters));
-const size_t kTailBytes = kTailFlags + 4 * kMaxJumpRounds;
-
 uint32_t jump_flag_index(uint32_t n) { return jump_rounds(n) - 1; }
 
 // Queue q's work on slot sl (scheduler thread, lock NOT held: CUDA calls only here).
@@ -179,8 +170,7 @@ uint32_t launch_query(scan_server* s, Slot& sl, Query* q) {
     cudaStream_t st = sl.stream;
     cudaEventRecord(sl.ev_start, st);
     scan_status rc = launch_cluster(g, r, st, q->pp, q->mu, &launches);
-    cudaMemcpyAsync(sl.h_res, r.label, res_bytes(g->n), cudaMemcpyDeviceToHost, st);       // label, role
-    cudaMemcpyAsync(sl.h_tail, r.ctr, kTailBytes, cudaMemcpyDeviceToHost, st);            // counters, flags
+    cudaMemcpyAsync(sl.h_res, r.label, res_bytes(g->n), cudaMemcpyDeviceToHost, st);   // label, role, counters, flags
     cudaEventRecord(sl.ev_end, st);
     cudaError_t err = cudaLaunchHostFunc(st, on_slot_done, new std::pair<scan_server*, Slot*>(s, &sl));
     if (rc != SCAN_OK || err != cudaSuccess) {
@@ -200,16 +190,16 @@ void copy_out(Slot* sl) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, sl->ev_start, sl->ev_end);
     q->device_ms = ms;
-    std::memcpy(&q->counters, sl->h_tail, sizeof(RunCounters));
+    std::memcpy(&q->counters, sl->h_res + res_counters(g->n), sizeof(RunCounters));
     uint32_t last_flag = 0;
-    std::memcpy(&last_flag, sl->h_tail + kTailFlags + 4 * jump_flag_index(g->n), sizeof(uint32_t));
+    std::memcpy(&last_flag, sl->h_res + res_flags(g->n) + 4 * jump_flag_index(g->n), sizeof(uint32_t));
     if (q->status == SCAN_OK && (q->counters.error_flags || last_flag)) {
         q->status = SCAN_ERR_DEVICE;
         q->error = "union-find did not finish within its limits";
     }
     if (q->status == SCAN_OK) {
         std::memcpy(q->out_label, sl->h_res, g->n * sizeof(int32_t));
-        if (q->out_role) std::memcpy(q->out_role, sl->h_res + res_role_offset(g->n), g->n);
+        if (q->out_role) std::memcpy(q->out_role, sl->h_res + res_role(g->n), g->n);
     }
 }
 
@@ -346,8 +336,7 @@ scan_status scan_server_create(int device, uint64_t memory_budget_bytes, uint32_
     s->slots = std::vector<Slot>(max_in_flight);   // Slot holds an atomic: built in place, never moved
     for (Slot& sl : s->slots) {
         if (cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreate(&sl.ev_start) != cudaSuccess || cudaEventCreate(&sl.ev_end) != cudaSuccess ||
-            cudaHostAlloc(&sl.h_tail, kTailBytes, cudaHostAllocDefault) != cudaSuccess) {
+            cudaEventCreate(&sl.ev_start) != cudaSuccess || cudaEventCreate(&sl.ev_end) != cudaSuccess) {
             scan_server_destroy(s.release());
             return fail(SCAN_ERR_CUDA, "cannot create the server's streams");
         }
@@ -586,7 +575,6 @@ void scan_server_destroy(scan_server* s) {
         if (sl.ev_start) cudaEventDestroy(sl.ev_start);
         if (sl.ev_end) cudaEventDestroy(sl.ev_end);
         if (sl.h_res) cudaFreeHost(sl.h_res);
-        if (sl.h_tail) cudaFreeHost(sl.h_tail);
     }
     for (DeviceGraph* d : s->graphs) device_graph_free(d);
     if (s->arena_base) cudaFree(s->arena_base);
