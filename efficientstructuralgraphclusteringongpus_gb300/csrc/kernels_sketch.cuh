@@ -305,11 +305,31 @@ __device__ __forceinline__ uint32_t missing_bits(const uint4 x, const uint4 y) {
     return __popc(x.x & ~y.x) + __popc(x.y & ~y.y) + __popc(x.z & ~y.z) + __popc(x.w & ~y.w);
 }
 
+// Two units (32 bytes, 32-byte aligned) in one load.  What L1 does for a request follows the
+// lines it touches: with 16-byte loads a group's four lanes asked for half a line at a time and
+// L1 was 82% busy (similarity stage, R-MAT s22 at eps
+// 0.2: 19.4 -> 17.9 ms; power law of 57M edges 1.65 -> 1.54).
+struct UnitPair {
+    uint4 lo, hi;
+};
+
+__device__ __forceinline__ UnitPair load_pair(const uint4* p) {
+    UnitPair r;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r.lo.x), "=r"(r.lo.y), "=r"(r.lo.z), "=r"(r.lo.w), "=r"(r.hi.x), "=r"(r.hi.y), "=r"(r.hi.z), "=r"(r.hi.w)
+        : "l"(p));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t missing_bits(const UnitPair& x, const UnitPair& y) {
+    return missing_bits(x.lo, y.lo) + missing_bits(x.hi, y.hi);
+}
+
 // Warps take `chunk` consecutive edges at a time (*queue counts those beyond the first) and work through them in batches
 // of kSketchBatch.  Lane i reads edge i's endpoints and their (base, degree) pairs, prunes it
 // by the degrees and picks a bitmap size for what is left.  By that size:
 //   * up to kSketchLaneLog: one edge per lane, its few units read by that lane;
-//   * up to kSketchGroupLog: groups of G lanes take one edge each, compare G * U units at a
+//   * up to kSketchGroupLog: groups of G lanes take one edge each, compare 2 G U units at a
 //     time until it is decided, and move on to the next;
 //   * larger: the list of k_sketch_long, a warp per edge.  A hub's edges of this kind sit
 //     together in its list (low ids in power-law graphs), and the few warps that drew them
@@ -322,9 +342,9 @@ __device__ __forceinline__ uint32_t missing_bits(const uint4 x, const uint4 y) {
 // all, *total (see pending_work).
 // ctr[0] += units read of the lower endpoints' bitmaps, ctr[1] += edges not pruned.
 constexpr int kSketchBatch = 128;
-// Groups of 4 lanes x 4 units: R-MAT s20 / s22 0.39 / 1.85 ms against 0.41 / 1.95 with 4 x 2,
-// 0.47 / 2.42 against 0.51 / 2.64 (8 x 2) and 0.50 / 2.77 (2 x 4) before edges went to lanes.
-constexpr int kSketchGroup = 4, kSketchUnroll = 4;
+// R-MAT s20 / s22, similarity stage: 4 lanes x 2 loads 0.48 / 1.83 ms, 4 x 1 0.51 / 1.96, 8 x 1
+// 0.52 / 1.99, 2 x 4 0.50 / 1.95.
+constexpr int kSketchGroup = 4, kSketchUnroll = 2;   // lanes; 32-byte loads of each bitmap in flight per lane
 constexpr uint32_t kSketchLaneLog = 10;    // 8 units
 constexpr uint32_t kSketchGroupLog = 15;   // 256 units
 
@@ -352,7 +372,7 @@ __device__ __forceinline__ uint32_t edge_pending(uint8_t* sim, const PendingWork
 }
 
 template <bool kPerGraph>
-__global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint32_t* __restrict__ lo_adj,
+__global__ void __launch_bounds__(256, 4) k_sketch_filter(uint64_t E, const uint32_t* __restrict__ lo_adj,
                                                        const uint32_t* __restrict__ lo_src,
                                                        const uint2* __restrict__ info, const uint4* __restrict__ sk,
                                                        SketchLevels levels, CnPrune pr, uint32_t chunk, uint32_t* queue,
@@ -360,7 +380,7 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                                                        unsigned long long* __restrict__ ctr) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     constexpr int G = kSketchGroup, U = kSketchUnroll;
-    constexpr uint32_t kGroups = 32 / G, kStep = G * U;
+    constexpr uint32_t kGroups = 32 / G, kStep = 2 * G * U;
     static_assert(kStep <= (2u << (kSketchLaneLog - kSketchMinLog)), "a group step must not exceed its smallest bitmap");
     __shared__ SketchSlot slots[8][kSketchBatch];
     __shared__ SketchLevels lv;               // indexed by lane: shared memory, not a parameter
@@ -384,14 +404,29 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
         const uint64_t kend = min((uint64_t)E, (uint64_t)(c + 1ull) * chunk);
         for (uint64_t kb = (uint64_t)c * chunk; kb < kend; kb += kSketchBatch) {
             uint32_t groups = 0, lanes = 0;   // slots for the groups from the front, for the lanes from the back
+            // all loads of the batch first: two round trips for its 128 edges
+            constexpr int kParts = kSketchBatch / 32;
+            uint32_t us[kParts], vs[kParts];
+            uint2 ius[kParts], ivs[kParts];
 #pragma unroll
-            for (int q = 0; q < kSketchBatch / 32; ++q) {
+            for (int q = 0; q < kParts; ++q) {
+                const uint64_t k = min(kb + 32 * q + lane, kend - 1);
+                us[q] = __ldcs(lo_adj + k);
+                vs[q] = __ldcs(lo_src + k);
+            }
+#pragma unroll
+            for (int q = 0; q < kParts; ++q) {
+                ius[q] = __ldg(info + us[q]);
+                ivs[q] = __ldg(info + vs[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < kParts; ++q) {
                 const uint64_t k = kb + 32 * q + lane;
                 uint32_t l = 0;               // bitmap size, 0: none needed
                 SketchSlot s{0, 0, 0, 0};
                 if (k < kend) {
-                    const uint32_t u = __ldcs(lo_adj + k), v = __ldcs(lo_src + k);
-                    const uint2 iu = info[u], iv = info[v];
+                    const uint32_t v = vs[q];
+                    const uint2 iu = ius[q], iv = ivs[q];
                     float floor2 = pr.eps2_floor;
                     double eps = pr.eps;
                     if constexpr (kPerGraph) {
@@ -452,18 +487,13 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                     const uint4* pu = sk + sketch_unit(lv, l, s.ru);
                     const uint4* pv = sk + sketch_unit(lv, l, s.rv);
                     uint32_t miss = 0, pos = 0;
-                    do {
-                        const bool two = units > 1;
-                        const uint4 x0 = __ldg(pu + pos), y0 = __ldg(pv + pos);
-                        uint4 x1 = make_uint4(0, 0, 0, 0), y1 = x1;
-                        if (two) {
-                            x1 = __ldg(pu + pos + 1);
-                            y1 = __ldg(pv + pos + 1);
-                        }
-                        miss += missing_bits(x0, y0) + missing_bits(x1, y1);
-                        pos += 2;
-                    } while (pos < units && miss < s.need);
-                    words += min(pos, units);
+                    if (units == 1) {
+                        miss = missing_bits(__ldg(pu), __ldg(pv));
+                        pos = 1;
+                    }
+                    for (; pos < units && miss < s.need; pos += 2)
+                        miss += missing_bits(load_pair(pu + pos), load_pair(pv + pos));
+                    words += pos;
                     if (miss >= s.need) break;
                     if (l == top) {
                         pending += edge_pending(sim, pw, lo_adj, lo_src, info, kb + (s.code & 0xFFu));
@@ -480,8 +510,8 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                 uint32_t left = 0, miss = 0;               // units left at this size
                 auto open = [&]() {
                     left = 1u << (slot_level(s) - kSketchMinLog);
-                    pu = sk + sketch_unit(lv, slot_level(s), s.ru) + gl;
-                    pv = sk + sketch_unit(lv, slot_level(s), s.rv) + gl;
+                    pu = sk + sketch_unit(lv, slot_level(s), s.ru) + 2 * gl;
+                    pv = sk + sketch_unit(lv, slot_level(s), s.rv) + 2 * gl;
                     miss = 0;
                 };
                 if (on) {
@@ -491,11 +521,11 @@ __global__ void __launch_bounds__(256, 5) k_sketch_filter(uint64_t E, const uint
                 for (;;) {
                     uint32_t m = 0;
                     if (on) {
-                        uint4 x[U], y[U];
+                        UnitPair x[U], y[U];
 #pragma unroll
                         for (int q = 0; q < U; ++q) {
-                            x[q] = __ldg(pu + q * G);
-                            y[q] = __ldg(pv + q * G);
+                            x[q] = load_pair(pu + 2 * q * G);
+                            y[q] = load_pair(pv + 2 * q * G);
                         }
 #pragma unroll
                         for (int q = 0; q < U; ++q) m += missing_bits(x[q], y[q]);
@@ -574,19 +604,17 @@ __global__ void __launch_bounds__(256) k_sketch_long(LongEdges ll, const uint32_
         const SketchSlot s{e.x, e.y, e.z, e.w};
         for (uint32_t level = slot_level(s);; level = min(level + 2, slot_top(s))) {
             const uint32_t units = 1u << (level - kSketchMinLog);
-            const uint4* pu = sk + sketch_unit(lv, level, s.ru) + lane;
-            const uint4* pv = sk + sketch_unit(lv, level, s.rv) + lane;
+            const uint4* pu = sk + sketch_unit(lv, level, s.ru) + 2 * lane;
+            const uint4* pv = sk + sketch_unit(lv, level, s.rv) + 2 * lane;
             uint32_t miss = 0, left = units;
             do {
-                uint4 x[4], y[4];
+                UnitPair x[2], y[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    x[q] = __ldg(pu + 32 * q);
-                    y[q] = __ldg(pv + 32 * q);
+                for (int q = 0; q < 2; ++q) {
+                    x[q] = load_pair(pu + 64 * q);
+                    y[q] = load_pair(pv + 64 * q);
                 }
-                uint32_t m = 0;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) m += missing_bits(x[q], y[q]);
+                const uint32_t m = missing_bits(x[0], y[0]) + missing_bits(x[1], y[1]);
                 miss += __reduce_add_sync(0xFFFFFFFFu, m);
                 pu += 128;
                 pv += 128;
