@@ -76,12 +76,24 @@ __global__ void k_tau(uint64_t E, const uint32_t* __restrict__ lo_adj, const uin
     }
 }
 
+// The threads that share a pass: this one's index among them (a multiple of 32 for lane 0) and
+// their number.  Each pass is a function of these, so that the kernels below run it over a grid
+// and k_cluster_small over one thread-block cluster.  Arrays that another pass writes carry no
+// __restrict__: in the fused kernel a non-coherent load could miss the write.
+struct Team {
+    uint64_t index, size;
+};
+__device__ __forceinline__ Team grid_team() {
+    return Team{blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x};
+}
+
 // k_predicate for a served graph: the cached thresholds decide every edge outside the
 // band; the disagreement counter is not kept (the server does not report it).
-__global__ void k_predicate_tau(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
-                                const uint32_t* __restrict__ off, const uint32_t* __restrict__ cn,
-                                const float* __restrict__ tau, PredParams pp, uint8_t* __restrict__ sim,
-                                int32_t* __restrict__ sd, RunCounters* __restrict__ ctr) {
+__device__ __forceinline__ void predicate_tau_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                                   const uint32_t* __restrict__ lo_src,
+                                                   const uint32_t* __restrict__ off, const uint32_t* __restrict__ cn,
+                                                   const float* __restrict__ tau, const PredParams& pp, uint8_t* sim,
+                                                   int32_t* sd, RunCounters* ctr) {
     const uint32_t lane = threadIdx.x & 31;
     const float* tm = tau + (pp.mode ? E : 0);
     double theta;
@@ -89,9 +101,8 @@ __global__ void k_predicate_tau(uint64_t E, const uint32_t* __restrict__ lo_adj,
     else theta = pp.q == 0 ? 2.0 : ((double)pp.p / (double)pp.q) * ((double)pp.p / (double)pp.q);
     const double hi = theta * (1.0 + kTauBand), lo = theta * (1.0 - kTauBand);
     unsigned long long nsim = 0;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t e0 = (uint64_t)blockIdx.x * blockDim.x; e0 < E; e0 += stride) {
-        const uint64_t e = e0 + threadIdx.x;
+    for (uint64_t e0 = team.index - lane; e0 < E; e0 += team.size) {
+        const uint64_t e = e0 + lane;
         bool s = false;
         uint32_t v = kEmpty;
         if (e < E) {
@@ -118,14 +129,20 @@ __global__ void k_predicate_tau(uint64_t E, const uint32_t* __restrict__ lo_adj,
     if (lane == 0 && nsim) atomicAdd(&ctr->similar_edges, nsim);
 }
 
+__global__ void k_predicate_tau(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
+                                const uint32_t* __restrict__ off, const uint32_t* __restrict__ cn,
+                                const float* __restrict__ tau, PredParams pp, uint8_t* __restrict__ sim,
+                                int32_t* __restrict__ sd, RunCounters* __restrict__ ctr) {
+    predicate_tau_pass(grid_team(), E, lo_adj, lo_src, off, cn, tau, pp, sim, sd, ctr);
+}
+
 // parent[v] = v for cores, -1 otherwise; border/neighbour label ranges reset.  Batched
 // runs pass vgid[] and per-graph gmu[].
-__global__ void k_core_init(uint32_t n, const int32_t* __restrict__ sd, int mu, const uint32_t* __restrict__ vgid,
-                            const int32_t* __restrict__ gmu, int32_t* __restrict__ parent, int32_t* __restrict__ bmin,
-                            int32_t* __restrict__ bmax, int32_t* __restrict__ nmin, int32_t* __restrict__ nmax,
-                            RunCounters* __restrict__ ctr) {
+__device__ __forceinline__ void core_init_pass(Team team, uint32_t n, const int32_t* sd, int mu, const uint32_t* __restrict__ vgid,
+                                               const int32_t* __restrict__ gmu, int32_t* parent, int32_t* bmin,
+                                               int32_t* bmax, int32_t* nmin, int32_t* nmax, RunCounters* ctr) {
     bool core = false;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t v = team.index; v < n; v += team.size) {
         const int m = vgid ? gmu[vgid[v]] : mu;
         const bool c = sd[v] >= m;
         core |= c;
@@ -136,6 +153,12 @@ __global__ void k_core_init(uint32_t n, const int32_t* __restrict__ sd, int mu, 
         nmax[v] = -1;
     }
     if (__any_sync(0xFFFFFFFFu, core) && (threadIdx.x & 31) == 0) atomicOr(&ctr->any_core, 1u);
+}
+__global__ void k_core_init(uint32_t n, const int32_t* __restrict__ sd, int mu, const uint32_t* __restrict__ vgid,
+                            const int32_t* __restrict__ gmu, int32_t* __restrict__ parent, int32_t* __restrict__ bmin,
+                            int32_t* __restrict__ bmax, int32_t* __restrict__ nmin, int32_t* __restrict__ nmax,
+                            RunCounters* __restrict__ ctr) {
+    core_init_pass(grid_team(), n, sd, mu, vgid, gmu, parent, bmin, bmax, nmin, nmax, ctr);
 }
 
 // Root of x with path halving.  parent[y] < y for every non-root y, so every write keeps
@@ -172,13 +195,13 @@ __device__ __forceinline__ bool uf_union(int32_t* parent, int32_t a, int32_t b, 
 // words), the first lane v's root as well.  Edges whose endpoints already point to one vertex
 // end after two loads.  Cluster stage of communities of 6M edges 0.50 -> 0.30 ms; unions of 30
 // served queries 2.24 -> 1.41 ms.
-__global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
-                        const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
+__device__ __forceinline__ void union_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                           const uint32_t* __restrict__ lo_src, const uint8_t* sim, int32_t* parent,
+                                           RunCounters* ctr, uint32_t limit) {
     if (!*(volatile uint32_t*)&ctr->any_core) return;   // no core: nothing to join
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t e0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); e0 < E; e0 += stride) {
+    for (uint64_t e0 = team.index - lane; e0 < E; e0 += team.size) {
         const uint64_t e = e0 + lane;
         int32_t u = 0, v = 0;
         bool join = false;
@@ -205,6 +228,10 @@ __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const u
         }
     }
 }
+__global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
+                        const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
+    union_pass(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit);
+}
 
 // Flatten by pointer jumping: a round moves parent[v] of every core up to kJumpSteps ancestors on
 // and raises flags[r] if any pointer moved, so the distance a pointer spans grows by that
@@ -227,11 +254,11 @@ __device__ __forceinline__ int32_t jump_target(const volatile int32_t* parent, i
     return p;
 }
 
-__global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint32_t round) {
-    if (round > 0 && *(volatile uint32_t*)&flags[round - 1] == 0) return;
+
+__device__ __forceinline__ uint32_t jump_pass(Team team, uint32_t n, int32_t* parent) {
     volatile int32_t* vp = parent;
     uint32_t ch = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t v = team.index; v < n; v += team.size) {
         const int32_t p = vp[v];
         if (p < 0) continue;
         const int32_t g = jump_target(vp, p);
@@ -240,6 +267,12 @@ __global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint3
             ch = 1;
         }
     }
+    return ch;
+}
+
+__global__ void k_jump_round(uint32_t n, int32_t* parent, uint32_t* flags, uint32_t round) {
+    if (round > 0 && *(volatile uint32_t*)&flags[round - 1] == 0) return;
+    const uint32_t ch = jump_pass(grid_team(), n, parent);
     if (__any_sync(0xFFFFFFFFu, ch) && (threadIdx.x & 31) == 0) atomicOr(&flags[round], 1u);
 }
 
@@ -277,11 +310,12 @@ __global__ void __launch_bounds__(1024) k_jump_block(uint32_t n, int32_t* parent
 // Border attachment: a non-core similar to a core joins that core's cluster.  The
 // reference keeps the last write among several clusters (GPUSCAN++/GPUScan.cu:716,722);
 // here the smallest cluster id wins, and bmin != bmax marks a multi-cluster border.
-__global__ void k_attach(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
-                         const uint8_t* __restrict__ sim, const int32_t* __restrict__ parent,
-                         int32_t* __restrict__ bmin, int32_t* __restrict__ bmax, const RunCounters* ctr) {
+__device__ __forceinline__ void attach_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                            const uint32_t* __restrict__ lo_src, const uint8_t* sim,
+                                            const int32_t* parent, int32_t* bmin, int32_t* bmax,
+                                            const RunCounters* ctr) {
     if (!*(const volatile uint32_t*)&ctr->any_core) return;   // no core: no border
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t e = team.index; e < E; e += team.size) {
         if (!sim[e]) continue;
         const uint32_t u = lo_adj[e], v = lo_src[e];
         const int32_t pu = parent[u], pv = parent[v];
@@ -289,12 +323,17 @@ __global__ void k_attach(uint64_t E, const uint32_t* __restrict__ lo_adj, const 
         else if (pv >= 0 && pu < 0) { atomicMin(&bmin[u], pv); atomicMax(&bmax[u], pv); }
     }
 }
+__global__ void k_attach(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
+                         const uint8_t* __restrict__ sim, const int32_t* __restrict__ parent,
+                         int32_t* __restrict__ bmin, int32_t* __restrict__ bmax, const RunCounters* ctr) {
+    attach_pass(grid_team(), E, lo_adj, lo_src, sim, parent, bmin, bmax, ctr);
+}
 
 // Label after attachment: cluster id for cores and borders, -2 for the rest.
-__global__ void k_label(uint32_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ bmin,
-                        int32_t* __restrict__ lab, RunCounters* __restrict__ ctr) {
+__device__ __forceinline__ void label_pass(Team team, uint32_t n, const int32_t* parent, const int32_t* bmin, int32_t* lab,
+                                           RunCounters* ctr) {
     bool member = false;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t v = team.index; v < n; v += team.size) {
         const int32_t p = parent[v];
         const int32_t l = p >= 0 ? p : (bmin[v] != 0x7FFFFFFF ? bmin[v] : -2);
         lab[v] = l;
@@ -302,34 +341,42 @@ __global__ void k_label(uint32_t n, const int32_t* __restrict__ parent, const in
     }
     if (__any_sync(0xFFFFFFFFu, member) && (threadIdx.x & 31) == 0) atomicOr(&ctr->any_member, 1u);
 }
+__global__ void k_label(uint32_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ bmin,
+                        int32_t* __restrict__ lab, RunCounters* __restrict__ ctr) {
+    label_pass(grid_team(), n, parent, bmin, lab, ctr);
+}
 
 // Hub test inputs: for each unlabelled vertex, the smallest and largest label among its
 // neighbours.  Two distinct labels make it a hub (GPUSCAN++/GPUScan.cu:757-780 looks for a
 // second neighbour label different from the first).
-__global__ void k_neighbour_labels(uint64_t E, const uint32_t* __restrict__ lo_adj,
-                                   const uint32_t* __restrict__ lo_src, const int32_t* __restrict__ lab,
-                                   int32_t* __restrict__ nmin, int32_t* __restrict__ nmax, const RunCounters* ctr) {
+__device__ __forceinline__ void neighbour_labels_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                                      const uint32_t* __restrict__ lo_src, const int32_t* lab,
+                                                      int32_t* nmin, int32_t* nmax, const RunCounters* ctr) {
     if (!*(const volatile uint32_t*)&ctr->any_member) return;   // no cluster: every other vertex is an outlier
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t e = team.index; e < E; e += team.size) {
         const uint32_t u = lo_adj[e], v = lo_src[e];
         const int32_t lu = lab[u], lv = lab[v];
         if (lu < 0 && lv >= 0) { atomicMin(&nmin[u], lv); atomicMax(&nmax[u], lv); }
         else if (lv < 0 && lu >= 0) { atomicMin(&nmin[v], lu); atomicMax(&nmax[v], lu); }
     }
 }
+__global__ void k_neighbour_labels(uint64_t E, const uint32_t* __restrict__ lo_adj,
+                                   const uint32_t* __restrict__ lo_src, const int32_t* __restrict__ lab,
+                                   int32_t* __restrict__ nmin, int32_t* __restrict__ nmax, const RunCounters* ctr) {
+    neighbour_labels_pass(grid_team(), E, lo_adj, lo_src, lab, nmin, nmax, ctr);
+}
 
 // Final labels, roles and counters.
-__global__ void k_finalize(uint32_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ bmin,
-                           const int32_t* __restrict__ bmax, const int32_t* __restrict__ nmin,
-                           const int32_t* __restrict__ nmax, int32_t* __restrict__ label,
-                           uint8_t* __restrict__ role, const unsigned long long* __restrict__ stage,
-                           RunCounters* __restrict__ ctr) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {   // so that one copy brings every counter back
+__device__ __forceinline__ void finalize_pass(Team team, uint32_t n, const int32_t* parent, const int32_t* bmin,
+                                              const int32_t* bmax, const int32_t* nmin, const int32_t* nmax,
+                                              int32_t* label, uint8_t* role,
+                                              const unsigned long long* __restrict__ stage, RunCounters* ctr) {
+    if (team.index == 0) {   // so that one copy brings every counter back
         ctr->list_words = stage[0];
         ctr->edges_counted = stage[1];
     }
     unsigned long long c_core = 0, c_clu = 0, c_hub = 0, c_out = 0, c_bor = 0, c_multi = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t v = team.index; v < n; v += team.size) {
         const int32_t p = parent[v];
         int32_t l;
         uint8_t r;
@@ -361,6 +408,76 @@ __global__ void k_finalize(uint32_t n, const int32_t* __restrict__ parent, const
         if (c_bor) atomicAdd(&ctr->borders, c_bor);
         if (c_multi) atomicAdd(&ctr->multi_borders, c_multi);
     }
+}
+__global__ void k_finalize(uint32_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ bmin,
+                           const int32_t* __restrict__ bmax, const int32_t* __restrict__ nmin,
+                           const int32_t* __restrict__ nmax, int32_t* __restrict__ label,
+                           uint8_t* __restrict__ role, const unsigned long long* __restrict__ stage,
+                           RunCounters* __restrict__ ctr) {
+    finalize_pass(grid_team(), n, parent, bmin, bmax, nmin, nmax, label, role, stage, ctr);
+}
+
+// The whole cluster stage of a small graph as one launch over one cluster of eight CTAs: what
+// bounds it there is the chain of eight to sixteen dependent launches, and the hardware's
+// cluster barrier between the passes costs about a microsecond.  A run of 10K edges spends 22 us
+// here instead of 35; from about 80K edges eight SMs take longer over the edges than the launches
+// do (communities: 148 us a run by launches, 171 fused).  Served queries run many at a time and
+// wait for their launches instead: fused up to a million edges, a burst of 30 mixed queries takes
+// 2.0 ms, up to 256K 2.8, by launches alone 3.4-3.8.  predicate: 0 done by the similarity stage,
+// 1 cached thresholds (tau); with 1 it also clears what the passes start from.
+constexpr uint64_t kFusedEdgesRun = 1u << 16, kFusedEdgesServed = 1u << 20;
+constexpr uint32_t kFusedVertices = 1u << 17;
+constexpr int kFusedCtas = 8, kFusedThreads = 1024;
+
+struct FusedCluster {
+    uint64_t E;
+    uint32_t n;
+    const uint32_t *lo_adj, *lo_src, *off, *cn;
+    const float* tau;
+    uint8_t* sim;
+    int32_t *sd, *parent, *bmin, *bmax, *nmin, *nmax, *lab, *label;
+    uint8_t* role;
+    RunCounters* ctr;
+    uint32_t* flags;
+    const unsigned long long* stage;
+    uint32_t rounds, limit;
+    int mu, predicate;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kFusedCtas, 1, 1) __launch_bounds__(kFusedThreads)
+k_cluster_small(FusedCluster f, PredParams pp) {
+    const Team team = grid_team();
+    if (f.predicate == 1) {
+        for (uint64_t i = team.index; i < f.n; i += team.size) f.sd[i] = 0;
+        if (team.index == 0) *f.ctr = RunCounters{};
+        if (team.index < kMaxJumpRounds) f.flags[team.index] = 0;
+        cluster_barrier();
+        predicate_tau_pass(team, f.E, f.lo_adj, f.lo_src, f.off, f.cn, f.tau, pp, f.sim, f.sd, f.ctr);
+        cluster_barrier();
+    }
+    core_init_pass(team, f.n, f.sd, f.mu, nullptr, nullptr, f.parent, f.bmin, f.bmax, f.nmin, f.nmax, f.ctr);
+    cluster_barrier();
+    if (*(volatile uint32_t*)&f.ctr->any_core) {          // the same in every thread, as below
+        union_pass(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.ctr, f.limit);
+        cluster_barrier();
+        for (uint32_t r = 0; r < f.rounds; ++r) {
+            const uint32_t ch = jump_pass(team, f.n, f.parent);
+            if (__any_sync(0xFFFFFFFFu, ch) && (threadIdx.x & 31) == 0) atomicOr(&f.flags[r], 1u);
+            cluster_barrier();
+            if (*(volatile uint32_t*)&f.flags[r] == 0) break;
+        }
+        attach_pass(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.bmin, f.bmax, f.ctr);
+        cluster_barrier();
+        label_pass(team, f.n, f.parent, f.bmin, f.lab, f.ctr);
+        cluster_barrier();
+        neighbour_labels_pass(team, f.E, f.lo_adj, f.lo_src, f.lab, f.nmin, f.nmax, f.ctr);
+        cluster_barrier();
+    }
+    finalize_pass(team, f.n, f.parent, f.bmin, f.bmax, f.nmin, f.nmax, f.label, f.role, f.stage, f.ctr);
 }
 
 // Memberships: every (cluster, border) pair from similar core-border edges.

@@ -1123,9 +1123,19 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     const int sms = d->num_sms, T = 256;
     const int ge = grid_for_n(sms, E, T), gn = grid_for_n(sms, n, T);
     const uint32_t* vgid = bp ? bp->vgid : nullptr;
+    const bool by_tau = !predicate_done && d->tau && !bp && d->cn_valid;
+    if (E <= (by_tau ? kFusedEdgesServed : kFusedEdgesRun) && n <= kFusedVertices && !bp && (predicate_done || by_tau)) {
+        const FusedCluster f{E, n, d->lo_adj, d->lo_src, d->off, d->cn, d->tau, r.sim, r.sd, r.parent, r.bmin, r.bmax,
+                             r.nmin, r.nmax, r.lab, r.label, r.role, r.ctr, r.jump_flags, d->cn_ctr, jump_rounds(n),
+                             union_find_limit(), mu, by_tau ? 1 : 0};
+        k_cluster_small<<<kFusedCtas, kFusedThreads, 0, s>>>(f, pp);
+        ++*launches;
+        SCAN_CUDA(cudaGetLastError());
+        return SCAN_OK;
+    }
     if (!predicate_done) {   // a one-shot launch_cn has cleared them
         SCAN_CUDA(run_scratch_clear(r, s));
-        if (d->tau && !bp && d->cn_valid)
+        if (by_tau)
             k_predicate_tau<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, d->off, d->cn, d->tau, pp, r.sim, r.sd, r.ctr);
         else
             k_predicate<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, d->off, d->cn, pp, vgid, bp ? bp->gpp : nullptr,
