@@ -245,10 +245,10 @@ void device_graph_free(DeviceGraph* d) {
     int prev = -1;
     cudaGetDevice(&prev);
     if (d->device >= 0) cudaSetDevice(d->device);
-    // The side stream's last work is joined into the main stream, and so is the aux stream's
-    // unless an upload gave up in between.
-    bool idle = d->stream && cudaStreamSynchronize(d->stream) == cudaSuccess;
-    idle = idle && d->aux && cudaStreamSynchronize(d->aux) == cudaSuccess;
+    // The other streams' last work is joined into the main one, unless an upload gave up in
+    // between.
+    bool idle = true;
+    for (cudaStream_t st : {d->stream, d->aux, d->side}) idle &= st && cudaStreamSynchronize(st) == cudaSuccess;
     for (auto& a : d->allocs) cache_give(d->device, a.first, a.second);
     if (d->adj_host) cudaFreeHost(d->adj_host);
     const StreamSet x = streams_of(d);
@@ -475,18 +475,19 @@ constexpr int kPendCounts = kPendingLists + 2;
 // queues in one line their atomics waited for one another (k_cn_small 0.105 -> 0.155 ms).
 constexpr int kCounterSpan = 64, kStageCounters = 3 * kCounterSpan;
 
-// The bitmaps of the larger vertices (lists from k_sketch_assign), on stream s.
+// The bitmaps of the larger vertices (lists from k_sketch_assign): the hubs on stream sh, the
+// others on sm.
 static scan_status build_large_sketches(DeviceGraph* d, const SketchPlan& plan, const uint32_t* mid,
-                                        const uint32_t* hub, cudaStream_t s) {
+                                        const uint32_t* hub, cudaStream_t sm, cudaStream_t sh) {
     constexpr int kMidSmem = (1 << kSketchMidLog) / 8, kHubSmem = (1 << kSketchMaxLog) / 8;
     if (plan.list_hub) {
         SCAN_CUDA(cudaFuncSetAttribute(k_sketch_build_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubSmem));
-        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_hub, (uint64_t)d->num_sms), 1024, kHubSmem, s>>>(
+        k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_hub, (uint64_t)d->num_sms), 1024, kHubSmem, sh>>>(
             hub, plan.list_hub, d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
     }
     if (plan.list_mid)
         k_sketch_build_cta<<<(unsigned)std::min<uint64_t>(plan.list_mid, (uint64_t)d->num_sms * 8), 256, kMidSmem,
-                             s>>>(mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
+                             sm>>>(mid, plan.list_mid, d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
     SCAN_CUDA(cudaGetLastError());
     return SCAN_OK;
 }
@@ -640,7 +641,9 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     // hot-id mapping and orientation count (one pass, k_orient_tiles) run on a second stream
     // while the next chunk is copied.  The pass skips ids >= n, so no host check has to come
     // in between; the flags are read once, after the count.
-    cudaStream_t s2 = d->aux;
+    // The bitmaps are built on a third: on the second they made every chunk's work longer than its
+    // copy (R-MAT s22: 1.56 ms left after the last copy, so 1.17).
+    cudaStream_t s2 = d->aux, s3 = d->side;
     constexpr int kMaxChunks = 8;
     static_assert(kMaxChunks + 1 <= sizeof(d->chunk_ev) / sizeof(d->chunk_ev[0]), "one event per chunk and one more");
     cudaEvent_t* ev_chunk = d->chunk_ev;
@@ -650,8 +653,10 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     auto off_at = [&](uint64_t v) -> uint64_t {
         return off64 ? static_cast<const uint64_t*>(off_host)[v] : static_cast<const uint32_t*>(off_host)[v];
     };
-    for (int c = 1; c < chunks; ++c) {            // first vertex whose list starts at or after c*m/chunks
-        uint64_t lo = vcut[c - 1], hi = n, target = m * (uint64_t)c / chunks;
+    // The chunks shrink towards the end: what is left to do after the last copy follows its size.
+    static const uint32_t cut_at[kMaxChunks] = {0, 170, 340, 500, 650, 780, 880, 950};   // thousandths of m
+    for (int c = 1; c < chunks; ++c) {            // first vertex whose list starts at or after the cut
+        uint64_t lo = vcut[c - 1], hi = n, target = m / 1000 * cut_at[c];
         while (lo < hi) {
             const uint64_t mid = (lo + hi) / 2;
             if (off_at(mid) < target) lo = mid + 1; else hi = mid;
@@ -671,7 +676,7 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
             k_hot_assign<<<grid_for(d.get(), n, 256), 256, 0, s2>>>(d->n, d->off, min_bin, kHotBits, d->hot,
                                                                   hist + kDegBins);
         if (d->sk)
-            k_sketch_assign<<<grid_for(d.get(), n, 256), 256, 0, s2>>>(d->n, d->off, sk_plan, sk_cls + kSketchClasses,
+            k_sketch_assign<<<grid_for(d.get(), n, 256), 256, 0, s3>>>(d->n, d->off, sk_plan, sk_cls + kSketchClasses,
                                                                      d->sk_info, sk_mid, sk_hub);
         if (adj_in_host_memory) {
             std::memcpy(d->adj_host, adj_host, m * sizeof(uint32_t));
@@ -693,37 +698,41 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
                     lowbits, flags, kBadId, kBadSelfLoop, kBadOrder);
                 ++orient_launches;
             }
-            if (c == chunks - 1) {
-                if (bitmap_path) SCAN_CUDA(cudaMemsetAsync(d->radj + m, 0, kAdjPad * sizeof(uint32_t), s2));
-                SCAN_CUDA(cudaEventRecord(ev_chunk[kMaxChunks], s2));
-            }
-            if (d->sk && vcut[c + 1] > vcut[c])
+            if (d->sk && vcut[c + 1] > vcut[c]) {
+                SCAN_CUDA(cudaStreamWaitEvent(s3, ev_chunk[c], 0));
                 k_sketch_build_small<<<grid_for(d.get(), vcut[c + 1] - vcut[c], kSketchWarps * 32), kSketchWarps * 32, 0,
-                                       s2>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
+                                       s3>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
+            }
         }
         SCAN_CUDA(cudaEventRecord(d->ev[1], s));   // end of the copies
-        // The orientation continues on s; the larger vertices' bitmaps are built beside it and
-        // joined at the end.
+        if (bitmap_path) SCAN_CUDA(cudaMemsetAsync(d->radj + m, 0, kAdjPad * sizeof(uint32_t), s2));
+        SCAN_CUDA(cudaEventRecord(ev_chunk[kMaxChunks], s2));
         SCAN_CUDA(cudaStreamWaitEvent(s, ev_chunk[kMaxChunks], 0));
-        if (d->sk) SCAN_TRY(build_large_sketches(d.get(), sk_plan, sk_mid, sk_hub, s2));
-        SCAN_CUDA(cudaEventRecord(d->join, s2));
+        // The orientation continues on s; the larger vertices' bitmaps are built beside it and
+        // joined at the end (built per chunk they held the chunks up: drop-in call 6.5 -> 6.8 ms).
+        if (d->sk) {
+            SCAN_CUDA(cudaEventRecord(d->fork, s3));                  // their lists
+            SCAN_CUDA(cudaStreamWaitEvent(s2, d->fork, 0));
+            SCAN_TRY(build_large_sketches(d.get(), sk_plan, sk_mid, sk_hub, s3, s2));
+        }
+        SCAN_CUDA(cudaEventRecord(d->fork, s2));
+        SCAN_CUDA(cudaEventRecord(d->join, s3));
         return SCAN_OK;
     };
     ost = enqueue();
     if (ost != SCAN_OK) {
         cudaStreamSynchronize(s2);
+        cudaStreamSynchronize(s3);
         return ost;
     }
     SCAN_TRY(device_scan(d.get(), cnt, n, d->lo_off, d->scratch));
-    uint32_t E32 = 0;
-    SCAN_CUDA(cudaMemcpyAsync(&E32, d->lo_off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaMemcpyAsync(&bad, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaStreamSynchronize(s));
-    if (bad & kBadId) return fail(SCAN_ERR_FORMAT, "neighbour id >= n");
-    if (bad & kBadSelfLoop) return fail(SCAN_ERR_FORMAT, "self loop");
-    if (bad & kBadOrder) return fail(SCAN_ERR_FORMAT, "neighbour list not sorted strictly ascending");
-    d->E = E32;
-    if (d->E * 2 != m) return fail(SCAN_ERR_FORMAT, "graph is not symmetric (lower entries * 2 != m)");
+    // The lower entries are half of a symmetric graph's, so the fill and the plan need not wait for
+    // their number: it is read, with the entry checks, in the plan's host round trip.  Until then
+    // the kernels may work on a graph that fails them (the fill bounds its writes by E).
+    d->E = m / 2;
+    uint32_t* early = reinterpret_cast<uint32_t*>(d->h_res);   // pinned: these copies do not wait
+    SCAN_CUDA(cudaMemcpyAsync(early, d->lo_off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    SCAN_CUDA(cudaMemcpyAsync(early + 1, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     SCAN_TRY(dalloc(d.get(), &d->lo_adj, d->E));
     SCAN_TRY(dalloc(d.get(), &d->lo_src, d->E));
     if (fill_tiles) {   // word prefix of the lower bits, then the fill
@@ -748,14 +757,23 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     pp.small_strategy = kSmallSerial;
     pp.bitmap_min_deg = kBitmapMinDeg;
     SCAN_TRY(dalloc(d.get(), &d->cn, d->E));
-    SCAN_TRY(plan_tasks(d.get(), pp));
+    const scan_status planned = plan_tasks(d.get(), pp);
+    SCAN_CUDA(cudaStreamSynchronize(s));
+    const uint32_t E32 = early[0];
+    bad = early[1];
+    if (bad & kBadId) return fail(SCAN_ERR_FORMAT, "neighbour id >= n");
+    if (bad & kBadSelfLoop) return fail(SCAN_ERR_FORMAT, "self loop");
+    if (bad & kBadOrder) return fail(SCAN_ERR_FORMAT, "neighbour list not sorted strictly ascending");
+    if ((uint64_t)E32 * 2 != m) return fail(SCAN_ERR_FORMAT, "graph is not symmetric (lower entries * 2 != m)");
+    SCAN_TRY(planned);
 
     // Result and scratch arrays.
     SCAN_TRY(dalloc(d.get(), &d->np_tab, kPruneTable));
     uint8_t* rs_mem = nullptr;
     SCAN_TRY(dalloc(d.get(), &rs_mem, run_scratch_bytes(d->n, d->E)));
     run_scratch_bind(&d->rs, rs_mem, d->n, d->E);
-    SCAN_CUDA(cudaStreamWaitEvent(s, d->join, 0));   // the bitmaps: one stream again
+    SCAN_CUDA(cudaStreamWaitEvent(s, d->fork, 0));   // the bitmaps: one stream again
+    SCAN_CUDA(cudaStreamWaitEvent(s, d->join, 0));
     SCAN_CUDA(cudaEventRecord(d->ev[2], s));
     SCAN_CUDA(cudaEventSynchronize(d->ev[2]));
     if (st) {
@@ -1013,7 +1031,10 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
     }
     SCAN_CUDA(cudaMemsetAsync(d->cn_ctr, 0, kStageCounters * sizeof(uint32_t), s));
     if (prune && d->nmiss) SCAN_CUDA(cudaMemsetAsync(d->miss, 0, (size_t)d->nmiss * sizeof(uint32_t), s));
-    if (prune && !per_graph) {
+    // Prune thresholds by pivot degree.  Behind the sketches a small graph has few pivots left,
+    // which compute theirs and save the launch.
+    if (fp.pend && d->E < (1u << 20)) {
+    } else if (prune && !per_graph) {
         k_prune_table<<<kPruneTable / 256, 256, 0, s>>>(pr, d->np_tab);
         pr.np_tab = d->np_tab;
         ++*launches;
