@@ -498,13 +498,16 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     if (n == 0 || n >= 0xFFFFFFFFull) return fail(SCAN_ERR_INVALID_ARG, "vertex count must be in [1, 2^32-1)");
     if (m >= 0xFFFFFFF0ull) return fail(SCAN_ERR_TOO_LARGE, "m >= 2^32 directed entries");
     SCAN_CUDA(cudaSetDevice(device));
+    CallBuffers tmp(device);   // outlives d, whose deleter waits for the streams
     std::unique_ptr<DeviceGraph, void (*)(DeviceGraph*)> d(new DeviceGraph(), device_graph_free);
     d->device = device;
     d->n = (uint32_t)n;
     d->m = m;
     SCAN_CUDA(cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, device));
     SCAN_TRY(take_streams(d.get()));
-    cudaStream_t s = d->stream;
+    // s: the adjacency copies, then the rest of the orientation; s2: each chunk's orientation
+    // pass; s3: the offsets and what follows from the degrees, then the bitmaps.
+    cudaStream_t s = d->stream, s2 = d->aux, s3 = d->side;
 
     SCAN_TRY(dalloc(d.get(), &d->off, n + 1));
     if (adj_in_host_memory) {
@@ -522,21 +525,48 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     uint32_t* cnt = nullptr;
     SCAN_TRY(dalloc(d.get(), &cnt, n));          // lower-neighbour counts (kept: reused below)
 
-    SCAN_CUDA(cudaEventRecord(d->ev[0], s));
-    SCAN_CUDA(cudaMemsetAsync(flags, 0, 64 * sizeof(uint32_t), s));
+    SCAN_CUDA(cudaEventRecord(d->ev[0], s3));
+    SCAN_CUDA(cudaMemsetAsync(flags, 0, 64 * sizeof(uint32_t), s3));
     if (off64) {
-        uint64_t* tmp = nullptr;
-        SCAN_CUDA(cudaMalloc(&tmp, (n + 1) * sizeof(uint64_t)));
-        cudaError_t e1 = cudaMemcpyAsync(tmp, off_host, (n + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s);
-        if (e1 == cudaSuccess)
-            k_offsets_from_u64<<<grid_for(d.get(), n + 1, 256), 256, 0, s>>>(tmp, n + 1, d->off, flags);
-        cudaError_t e2 = cudaStreamSynchronize(s);
-        cudaFree(tmp);
-        if (e1 != cudaSuccess || e2 != cudaSuccess)
-            return fail(SCAN_ERR_CUDA, std::string("offset upload: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
+        uint64_t* off_in = nullptr;
+        SCAN_TRY(tmp.get(&off_in, n + 1));
+        SCAN_CUDA(cudaMemcpyAsync(off_in, off_host, (n + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s3));
+        k_offsets_from_u64<<<grid_for(d.get(), n + 1, 256), 256, 0, s3>>>(off_in, n + 1, d->off, flags);
     } else {
-        SCAN_CUDA(cudaMemcpyAsync(d->off, off_host, (n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+        SCAN_CUDA(cudaMemcpyAsync(d->off, off_host, (n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s3));
     }
+
+    // The adjacency arrives in chunks of whole vertex ranges.  They shrink towards the end: what
+    // is left to do after the last copy follows its size.  Cut from the offsets as they came;
+    // ones that will fail their check are kept within [0, m].
+    constexpr int kMaxChunks = 8;
+    static_assert(kMaxChunks + 1 <= sizeof(d->chunk_ev) / sizeof(d->chunk_ev[0]), "one event per chunk and one more");
+    cudaEvent_t* ev_chunk = d->chunk_ev;
+    const int chunks = (adj_in_host_memory || m < (16ull << 20)) ? 1 : kMaxChunks;
+    std::vector<uint32_t> vcut(chunks + 1, 0);
+    vcut[chunks] = (uint32_t)n;
+    std::vector<uint64_t> jcut(chunks + 1, 0);
+    jcut[chunks] = m;
+    auto off_at = [&](uint64_t v) -> uint64_t {
+        return off64 ? static_cast<const uint64_t*>(off_host)[v] : static_cast<const uint32_t*>(off_host)[v];
+    };
+    static const uint32_t cut_at[kMaxChunks] = {0, 170, 340, 500, 650, 780, 880, 950};   // thousandths of m
+    for (int c = 1; c < chunks; ++c) {            // first vertex whose list starts at or after the cut
+        uint64_t lo = vcut[c - 1], hi = n, target = m / 1000 * cut_at[c];
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (off_at(mid) < target) lo = mid + 1; else hi = mid;
+        }
+        vcut[c] = (uint32_t)lo;
+        jcut[c] = std::min(std::max(off_at(lo), jcut[c - 1]), m);
+    }
+    auto copy_chunk = [&](int c) -> scan_status {
+        const uint64_t j0 = jcut[c], j1 = jcut[c + 1];
+        if (!adj_in_host_memory && j1 > j0)
+            SCAN_CUDA(cudaMemcpyAsync(d->adj + j0, adj_host + j0, (j1 - j0) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+        SCAN_CUDA(cudaEventRecord(ev_chunk[c], s));
+        return SCAN_OK;
+    };
     // Counters of the similarity stage, cleared together: list words, edges counted and pending
     // work (64 bits each), the kernels' task queues, the pending lists.
     static_assert(2 * kCounterSpan + kPendCounts <= kStageCounters, "similarity-stage counters");
@@ -548,7 +578,9 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     // The offsets are checked first (every later kernel indexes lists by them), with the
     // degree histogram of the hot-id assignment; both need only the offsets, so the host
     // waits for those alone.
-    k_check_offsets32<<<grid_for(d.get(), n, 256), 256, 0, s>>>(d->off, n, m, flags);
+    uint32_t* pinned = reinterpret_cast<uint32_t*>(d->h_res);   // copies to it do not wait
+    static_assert((64 + kDegBins + kSketchClasses) * sizeof(uint32_t) <= kResStage, "staging of the upload's counts");
+    k_check_offsets32<<<grid_for(d.get(), n, 256), 256, 0, s3>>>(d->off, n, m, flags);
 
     // Hot ids for the bitmap path: the kHotBits highest-degree vertices (by degree bin).
     // On by default wherever it applies: its pivots are never split, so the early stop of
@@ -558,26 +590,31 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     const int mode = knob && !std::strcmp(knob, "off") ? 0 : knob && !std::strcmp(knob, "tails-free") ? 2 : 1;
     bool bitmap_path = mode != 0 && n + kHotBits < 0xFFFFFFF0ull && m > 0 && !adj_in_host_memory;
     uint32_t* hist = nullptr;
-    std::vector<uint32_t> h(kDegBins, 0);
+    const uint32_t* h = pinned + 64;
     if (bitmap_path) {
         SCAN_TRY(dalloc(d.get(), &hist, kDegBins + 1));
-        SCAN_CUDA(cudaMemsetAsync(hist, 0, (kDegBins + 1) * sizeof(uint32_t), s));
-        k_deg_hist<<<grid_for(d.get(), n, 256), 256, 0, s>>>(d->n, d->off, hist);
-        SCAN_CUDA(cudaMemcpyAsync(h.data(), hist, kDegBins * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        SCAN_CUDA(cudaMemsetAsync(hist, 0, (kDegBins + 1) * sizeof(uint32_t), s3));
+        k_deg_hist<<<grid_for(d.get(), n, 256), 256, 0, s3>>>(d->n, d->off, hist);
+        SCAN_CUDA(cudaMemcpyAsync(pinned + 64, hist, kDegBins * sizeof(uint32_t), cudaMemcpyDeviceToHost, s3));
     }
     // Sketches for the one-shot runs: their size follows from the degrees.
     uint32_t* sk_cls = nullptr;
-    std::vector<uint32_t> hcls(kSketchClasses, 0);
+    const uint32_t* hcls = pinned + 64 + kDegBins;
     const bool want_sketch = m >= 2 * kSketchMinEdges;
     if (want_sketch) {
         SCAN_TRY(dalloc(d.get(), &sk_cls, 2 * kSketchClasses + 2));   // class sizes; then assignment counters
-        SCAN_CUDA(cudaMemsetAsync(sk_cls, 0, (2 * kSketchClasses + 2) * sizeof(uint32_t), s));
-        k_sketch_classes<<<grid_for(d.get(), n, 256), 256, 0, s>>>(d->n, d->off, sk_cls);
-        SCAN_CUDA(cudaMemcpyAsync(hcls.data(), sk_cls, kSketchClasses * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        SCAN_CUDA(cudaMemsetAsync(sk_cls, 0, (2 * kSketchClasses + 2) * sizeof(uint32_t), s3));
+        k_sketch_classes<<<grid_for(d.get(), n, 256), 256, 0, s3>>>(d->n, d->off, sk_cls);
+        SCAN_CUDA(cudaMemcpyAsync(pinned + 64 + kDegBins, sk_cls, kSketchClasses * sizeof(uint32_t),
+                                  cudaMemcpyDeviceToHost, s3));
     }
-    uint32_t bad = 0;
-    SCAN_CUDA(cudaMemcpyAsync(&bad, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaStreamSynchronize(s));
+    SCAN_CUDA(cudaMemcpyAsync(pinned, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s3));
+    // The first chunk is on its way while the host waits for the checks of the offsets (drop-in
+    // call, R-MAT s22 6.47 -> 6.42 ms, s13 0.51 -> 0.49).  One only: copies from pageable memory block the host.
+    if (!adj_in_host_memory) SCAN_CUDA(cudaMemsetAsync(d->adj + m, 0, kAdjPad * sizeof(uint32_t), s));
+    SCAN_TRY(copy_chunk(0));
+    SCAN_CUDA(cudaStreamSynchronize(s3));
+    uint32_t bad = pinned[0];
     if (bad) return fail(SCAN_ERR_FORMAT, "offsets are not a non-decreasing sequence from 0 to m");
     SketchPlan sk_plan{};
     uint64_t sk_units = 0;
@@ -637,32 +674,10 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         SCAN_TRY(dalloc(d.get(), &d->tailc, n));
     }
 
-    // The adjacency arrives in chunks of whole vertex ranges; each chunk's entry checks,
-    // hot-id mapping and orientation count (one pass, k_orient_tiles) run on a second stream
-    // while the next chunk is copied.  The pass skips ids >= n, so no host check has to come
-    // in between; the flags are read once, after the count.
-    // The bitmaps are built on a third: on the second they made every chunk's work longer than its
-    // copy (R-MAT s22: 1.56 ms left after the last copy, so 1.17).
-    cudaStream_t s2 = d->aux, s3 = d->side;
-    constexpr int kMaxChunks = 8;
-    static_assert(kMaxChunks + 1 <= sizeof(d->chunk_ev) / sizeof(d->chunk_ev[0]), "one event per chunk and one more");
-    cudaEvent_t* ev_chunk = d->chunk_ev;
-    const int chunks = (adj_in_host_memory || m < (16ull << 20)) ? 1 : kMaxChunks;
-    std::vector<uint32_t> vcut(chunks + 1, 0);
-    vcut[chunks] = (uint32_t)n;
-    auto off_at = [&](uint64_t v) -> uint64_t {
-        return off64 ? static_cast<const uint64_t*>(off_host)[v] : static_cast<const uint32_t*>(off_host)[v];
-    };
-    // The chunks shrink towards the end: what is left to do after the last copy follows its size.
-    static const uint32_t cut_at[kMaxChunks] = {0, 170, 340, 500, 650, 780, 880, 950};   // thousandths of m
-    for (int c = 1; c < chunks; ++c) {            // first vertex whose list starts at or after the cut
-        uint64_t lo = vcut[c - 1], hi = n, target = m / 1000 * cut_at[c];
-        while (lo < hi) {
-            const uint64_t mid = (lo + hi) / 2;
-            if (off_at(mid) < target) lo = mid + 1; else hi = mid;
-        }
-        vcut[c] = (uint32_t)lo;
-    }
+    // Each chunk's entry checks, hot-id mapping and orientation count (one pass, k_orient_tiles)
+    // run on s2 while the next chunk is copied.  The pass skips ids >= n, so no host check has to
+    // come in between; the flags are read once, with the plan.  The bitmaps on s2 too made every
+    // chunk's work longer than its copy (R-MAT s22: 1.56 ms left after the last copy, so 1.17).
     scan_status ost = SCAN_OK;
     uint32_t orient_launches = 0;
     auto enqueue = [&]() -> scan_status {
@@ -681,15 +696,10 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         if (adj_in_host_memory) {
             std::memcpy(d->adj_host, adj_host, m * sizeof(uint32_t));
             std::memset(d->adj_host + m, 0, kAdjPad * sizeof(uint32_t));
-        } else {
-            SCAN_CUDA(cudaMemsetAsync(d->adj + m, 0, kAdjPad * sizeof(uint32_t), s));
         }
         for (int c = 0; c < chunks; ++c) {
-            const uint64_t j0 = off_at(vcut[c]), j1 = off_at(vcut[c + 1]);
-            if (!adj_in_host_memory && j1 > j0)
-                SCAN_CUDA(cudaMemcpyAsync(d->adj + j0, adj_host + j0, (j1 - j0) * sizeof(uint32_t),
-                                          cudaMemcpyHostToDevice, s));
-            SCAN_CUDA(cudaEventRecord(ev_chunk[c], s));
+            const uint64_t j0 = jcut[c], j1 = jcut[c + 1];
+            if (c) SCAN_TRY(copy_chunk(c));
             SCAN_CUDA(cudaStreamWaitEvent(s2, ev_chunk[c], 0));
             if (j1 > j0) {
                 const uint64_t tiles = (j1 + kFillTile - 1) / kFillTile - j0 / kFillTile;
@@ -730,9 +740,8 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     // their number: it is read, with the entry checks, in the plan's host round trip.  Until then
     // the kernels may work on a graph that fails them (the fill bounds its writes by E).
     d->E = m / 2;
-    uint32_t* early = reinterpret_cast<uint32_t*>(d->h_res);   // pinned: these copies do not wait
-    SCAN_CUDA(cudaMemcpyAsync(early, d->lo_off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    SCAN_CUDA(cudaMemcpyAsync(early + 1, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    SCAN_CUDA(cudaMemcpyAsync(pinned, d->lo_off + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    SCAN_CUDA(cudaMemcpyAsync(pinned + 1, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     SCAN_TRY(dalloc(d.get(), &d->lo_adj, d->E));
     SCAN_TRY(dalloc(d.get(), &d->lo_src, d->E));
     if (fill_tiles) {   // word prefix of the lower bits, then the fill
@@ -759,8 +768,8 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     SCAN_TRY(dalloc(d.get(), &d->cn, d->E));
     const scan_status planned = plan_tasks(d.get(), pp);
     SCAN_CUDA(cudaStreamSynchronize(s));
-    const uint32_t E32 = early[0];
-    bad = early[1];
+    const uint32_t E32 = pinned[0];
+    bad = pinned[1];
     if (bad & kBadId) return fail(SCAN_ERR_FORMAT, "neighbour id >= n");
     if (bad & kBadSelfLoop) return fail(SCAN_ERR_FORMAT, "self loop");
     if (bad & kBadOrder) return fail(SCAN_ERR_FORMAT, "neighbour list not sorted strictly ascending");
