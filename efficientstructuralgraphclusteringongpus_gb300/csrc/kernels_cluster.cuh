@@ -189,48 +189,66 @@ __device__ __forceinline__ bool uf_union(int32_t* parent, int32_t a, int32_t b, 
     return false;
 }
 
+// The similar ones of the W edges from k on as bits.  W = 4 (k a multiple of 4; the scratch pads
+// sim to 256 bytes): most edges of a sparse result are not similar, four per load and test (R-MAT
+// s22, mu 2: unions 107 -> 38 us, borders 104 -> 38).  W = 1 in the fused kernel, whose threads
+// would work through their four edges one after the other.
+template <int W>
+__device__ __forceinline__ uint32_t similar_bits(const uint8_t* sim, uint64_t k, uint64_t E) {
+    if (k >= E) return 0;
+    if constexpr (W == 1) return sim[k];
+    const uint32_t p = *reinterpret_cast<const uint32_t*>(sim + k) & 0x01010101u;   // 0 or 1 each by now
+    const uint32_t bits = (p | p >> 7 | p >> 14 | p >> 21) & 0xFu;
+    return k + 4 > E ? bits & ((1u << (uint32_t)(E - k)) - 1u) : bits;
+}
+
 // Edges of one pivot v are consecutive, so a warp holds runs of them.  Hanging v's root under
 // each lower neighbour's in turn would let one CAS per round succeed; instead the lanes of a
 // run agree on the smallest of their roots and hang their own root under that (all different
 // words), the first lane v's root as well.  Edges whose endpoints already point to one vertex
 // end after two loads.  Cluster stage of communities of 6M edges 0.50 -> 0.30 ms; unions of 30
 // served queries 2.24 -> 1.41 ms.
+template <int W>
 __device__ __forceinline__ void union_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
                                            const uint32_t* __restrict__ lo_src, const uint8_t* sim, int32_t* parent,
                                            RunCounters* ctr, uint32_t limit) {
     if (!*(volatile uint32_t*)&ctr->any_core) return;   // no core: nothing to join
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31;
-    for (uint64_t e0 = team.index - lane; e0 < E; e0 += team.size) {
-        const uint64_t e = e0 + lane;
-        int32_t u = 0, v = 0;
-        bool join = false;
-        if (e < E && sim[e]) {
-            u = (int32_t)lo_adj[e];
-            v = (int32_t)lo_src[e];
-            const int32_t pu = parent[u], pv = parent[v];
-            join = pu >= 0 && pv >= 0 && pu != pv;      // core-core only (cores never change)
-        }
-        if (!__any_sync(kFull, join)) continue;
-        if (join) {
-            u = uf_find(parent, u);
-            const int32_t rv = uf_find(parent, v);
-            join = u != rv;
-        }
-        const uint32_t run = __match_any_sync(kFull, join ? (uint32_t)v : kEmpty);
-        if (join) {
-            const bool first = (__ffs(run) - 1) == (int)lane;
-            const int32_t rv = uf_find(parent, v);
-            const int32_t m = (int32_t)__reduce_min_sync(run, (uint32_t)min(u, rv));
-            bool ok = u == m || uf_union(parent, u, m, limit);
-            if (first && rv != m) ok &= uf_union(parent, rv, m, limit);
-            if (!ok) atomicOr(&ctr->error_flags, kErrUnionFindLimit);
+    for (uint64_t e0 = W * (team.index - lane); e0 < E; e0 += W * team.size) {
+        uint32_t bits = similar_bits<W>(sim, e0 + W * lane, E);
+        while (__any_sync(kFull, bits)) {
+            int32_t u = 0, v = 0;
+            bool join = false;
+            if (bits) {
+                const uint64_t e = e0 + W * lane + __ffs(bits) - 1;
+                bits &= bits - 1;
+                u = (int32_t)lo_adj[e];
+                v = (int32_t)lo_src[e];
+                const int32_t pu = parent[u], pv = parent[v];
+                join = pu >= 0 && pv >= 0 && pu != pv;      // core-core only (cores never change)
+            }
+            if (!__any_sync(kFull, join)) continue;
+            if (join) {
+                u = uf_find(parent, u);
+                const int32_t rv = uf_find(parent, v);
+                join = u != rv;
+            }
+            const uint32_t run = __match_any_sync(kFull, join ? (uint32_t)v : kEmpty);
+            if (join) {
+                const bool first = (__ffs(run) - 1) == (int)lane;
+                const int32_t rv = uf_find(parent, v);
+                const int32_t m = (int32_t)__reduce_min_sync(run, (uint32_t)min(u, rv));
+                bool ok = u == m || uf_union(parent, u, m, limit);
+                if (first && rv != m) ok &= uf_union(parent, rv, m, limit);
+                if (!ok) atomicOr(&ctr->error_flags, kErrUnionFindLimit);
+            }
         }
     }
 }
 __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
                         const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
-    union_pass(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit);
+    union_pass<4>(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit);
 }
 
 // Flatten by pointer jumping: a round moves parent[v] of every core up to kJumpSteps ancestors on
@@ -310,23 +328,25 @@ __global__ void __launch_bounds__(1024) k_jump_block(uint32_t n, int32_t* parent
 // Border attachment: a non-core similar to a core joins that core's cluster.  The
 // reference keeps the last write among several clusters (GPUSCAN++/GPUScan.cu:716,722);
 // here the smallest cluster id wins, and bmin != bmax marks a multi-cluster border.
+template <int W>
 __device__ __forceinline__ void attach_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
                                             const uint32_t* __restrict__ lo_src, const uint8_t* sim,
                                             const int32_t* parent, int32_t* bmin, int32_t* bmax,
                                             const RunCounters* ctr) {
     if (!*(const volatile uint32_t*)&ctr->any_core) return;   // no core: no border
-    for (uint64_t e = team.index; e < E; e += team.size) {
-        if (!sim[e]) continue;
-        const uint32_t u = lo_adj[e], v = lo_src[e];
-        const int32_t pu = parent[u], pv = parent[v];
-        if (pu >= 0 && pv < 0) { atomicMin(&bmin[v], pu); atomicMax(&bmax[v], pu); }
-        else if (pv >= 0 && pu < 0) { atomicMin(&bmin[u], pv); atomicMax(&bmax[u], pv); }
-    }
+    for (uint64_t e0 = W * team.index; e0 < E; e0 += W * team.size)
+        for (uint32_t bits = similar_bits<W>(sim, e0, E); bits; bits &= bits - 1) {
+            const uint64_t e = e0 + __ffs(bits) - 1;
+            const uint32_t u = lo_adj[e], v = lo_src[e];
+            const int32_t pu = parent[u], pv = parent[v];
+            if (pu >= 0 && pv < 0) { atomicMin(&bmin[v], pu); atomicMax(&bmax[v], pu); }
+            else if (pv >= 0 && pu < 0) { atomicMin(&bmin[u], pv); atomicMax(&bmax[u], pv); }
+        }
 }
 __global__ void k_attach(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
                          const uint8_t* __restrict__ sim, const int32_t* __restrict__ parent,
                          int32_t* __restrict__ bmin, int32_t* __restrict__ bmax, const RunCounters* ctr) {
-    attach_pass(grid_team(), E, lo_adj, lo_src, sim, parent, bmin, bmax, ctr);
+    attach_pass<4>(grid_team(), E, lo_adj, lo_src, sim, parent, bmin, bmax, ctr);
 }
 
 // Label after attachment: cluster id for cores and borders, -2 for the rest.
@@ -462,7 +482,7 @@ k_cluster_small(FusedCluster f, PredParams pp) {
     core_init_pass(team, f.n, f.sd, f.mu, nullptr, nullptr, f.parent, f.bmin, f.bmax, f.nmin, f.nmax, f.ctr);
     cluster_barrier();
     if (*(volatile uint32_t*)&f.ctr->any_core) {          // the same in every thread, as below
-        union_pass(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.ctr, f.limit);
+        union_pass<1>(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.ctr, f.limit);
         cluster_barrier();
         for (uint32_t r = 0; r < f.rounds; ++r) {
             const uint32_t ch = jump_pass(team, f.n, f.parent);
@@ -470,7 +490,7 @@ k_cluster_small(FusedCluster f, PredParams pp) {
             cluster_barrier();
             if (*(volatile uint32_t*)&f.flags[r] == 0) break;
         }
-        attach_pass(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.bmin, f.bmax, f.ctr);
+        attach_pass<1>(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.bmin, f.bmax, f.ctr);
         cluster_barrier();
         label_pass(team, f.n, f.parent, f.bmin, f.lab, f.ctr);
         cluster_barrier();
