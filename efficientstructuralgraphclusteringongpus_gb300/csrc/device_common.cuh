@@ -29,7 +29,6 @@ constexpr int kMaxJumpRounds = 40;          // pointer-jumping rounds of the uni
 
 // Error flags written by bounded device loops.
 constexpr uint32_t kErrUnionFindLimit = 1u;
-constexpr uint32_t kErrHashFull = 2u;
 
 // Device counters gathered by the final per-vertex pass (copied back with the labels).
 struct RunCounters {

@@ -254,8 +254,8 @@ __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const u
 // Flatten by pointer jumping: a round moves parent[v] of every core up to kJumpSteps ancestors on
 // and raises flags[r] if any pointer moved, so the distance a pointer spans grows by that
 // factor per round.  The host queues enough rounds for any depth (ceil(log16 n) + 2: eight for
-// 4M vertices, where steps of one took 24 launches); a round whose predecessor moved nothing returns at once, so the pass
-// needs no host synchronisation.  Every value stored is an ancestor of v in the final
+// 4M vertices, where steps of one took 24 launches); a round whose predecessor moved nothing
+// returns at once, so the pass needs no host synchronisation.  Every value stored is an ancestor of v in the final
 // forest and only v's own thread writes parent[v], so concurrent jumps never undo one
 // another.  (A find with path halving would not be safe here: its halving store can
 // overwrite a vertex whose root another thread has just written with an intermediate

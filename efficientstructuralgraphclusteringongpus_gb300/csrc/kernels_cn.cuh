@@ -5,9 +5,9 @@
 // the link and attach phases (:579-584, :701-706).  Here every edge is counted exactly
 // once, grouped by its higher endpoint v (the pivot):
 //   1. the pivot's list N(v) (or one id-range chunk of it) is staged in shared memory: a
-//      per-warp hash table for small pivots, and per CTA task a hashed bitmap plus a sorted
-//      copy (one-shot runs, k_cn_filter_classes), a bucketed hash table (full counts, k_cn_big) or
-//      a bitmap of hot ids (hubs, k_cn_bitmap);
+//      per-warp hash table for small pivots, and per CTA task a bucketed hash table (k_cn_big), a
+//      bitmap of hot ids (hubs, k_cn_bitmap) or, in one-shot runs without neighbourhood bitmaps
+//      (kernels_sketch.cuh), a hashed bitmap plus a sorted copy (k_cn_filter_classes);
 //   2. warps stream the lower endpoints' lists N(u) with 16-byte loads and probe each
 //      element against it; ballots and warp reductions give the counts;
 //   3. in one-shot runs the degree prune, the early stop and the predicate skip use integer

@@ -22,6 +22,7 @@
 #include "device_common.cuh"
 #include "device_graph.h"
 #include "kernels_cn.cuh"
+#include "pending_slices.cuh"
 
 namespace scan {
 
@@ -325,8 +326,8 @@ __device__ __forceinline__ uint32_t missing_bits(const UnitPair& x, const UnitPa
     return missing_bits(x.lo, y.lo) + missing_bits(x.hi, y.hi);
 }
 
-// Warps take `chunk` consecutive edges at a time (*queue counts those beyond the first) and work through them in batches
-// of kSketchBatch.  Lane i reads edge i's endpoints and their (base, degree) pairs, prunes it
+// Warps take `chunk` consecutive edges at a time (*queue counts those beyond the first) and
+// work through them in batches of kSketchBatch.  Lane i reads edge i's endpoints and their (base, degree) pairs, prunes it
 // by the degrees and picks a bitmap size for what is left.  By that size:
 //   * up to kSketchLaneLog: one edge per lane, its few units read by that lane;
 //   * up to kSketchGroupLog: groups of G lanes take one edge each, compare 2 G U units at a
@@ -579,11 +580,13 @@ __global__ void __launch_bounds__(256, 4) k_sketch_filter(uint64_t E, const uint
     }
     words = __reduce_add_sync(kFull, words);
     counted = __reduce_add_sync(kFull, counted);
-    pending = __reduce_add_sync(kFull, pending);
+    // 64 bits: a total short of the pivots' sums would be cut into more slices than fit
+    const uint32_t pend_lo = __reduce_add_sync(kFull, pending & 0xFFFFu);
+    const uint32_t pend_hi = __reduce_add_sync(kFull, pending >> 16);
     if (lane == 0 && (words | counted)) {
         atomicAdd(&ctr[0], (unsigned long long)words);
         atomicAdd(&ctr[1], (unsigned long long)counted);
-        if (pending) atomicAdd(pw.total, (unsigned long long)pending);
+        if (pend_lo | pend_hi) atomicAdd(pw.total, pend_lo + ((unsigned long long)pend_hi << 16));
     }
 }
 
@@ -854,8 +857,6 @@ __global__ void __launch_bounds__(256) k_predicate_pending(uint64_t E, const uin
 // its edges and keep one CTA busy after the others are done.  Per task list, entries of
 // TaskPick::order; counts[c] hash class c, counts[kNumBigClasses] the hubs.
 constexpr int kPendingLists = kNumBigClasses + 1;
-constexpr uint32_t kPendingSlices = 8;        // slices aimed at per SM, over all lists
-constexpr uint32_t kPendingMinWork = 512;     // 32K list entries: a slice stages its pivot again
 struct PendingLists {
     const CnTask* tasks[kPendingLists];
     uint32_t count[kPendingLists];
@@ -925,13 +926,10 @@ __global__ void __launch_bounds__(256) k_pending_tasks(PendingLists pl, PendingW
                                                        uint32_t* __restrict__ counts) {
     __shared__ uint32_t warp_sums[8], place;
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t even = (uint32_t)min(*pw.total / slices + 1, 0x7FFFFFFFull);
-    // slices for `found` pending edges of task t
+    const uint64_t even = pending_even(*pw.total, slices);
     auto cut = [&](const CnTask& t, uint32_t work, uint32_t found) {
         const uint32_t dv = off[t.v + 1] - off[t.v], all = lo_off[t.v + 1] - lo_off[t.v];
-        const uint64_t mine = (uint64_t)work * (t.e1 - t.e0) / all;          // the task's share of its pivot's
-        const uint32_t aim = max(even, max(kPendingMinWork, dv / 16));       // 4 d_v entries at least
-        return (uint32_t)min(mine / aim + 1, (uint64_t)((found + 7) / 8));
+        return pending_slices(even, work, t.e1 - t.e0, all, t.chunked ? t.ce - t.cb : dv, dv, found);
     };
     for (int a = 2; a < kPendingLists; ++a)
         for (uint32_t i = blockIdx.x; i < pl.count[a]; i += gridDim.x) {

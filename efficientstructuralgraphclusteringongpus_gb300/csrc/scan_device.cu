@@ -71,10 +71,6 @@ __global__ void k_check_offsets32(const uint32_t* __restrict__ off, uint64_t n, 
     if (blockIdx.x == 0 && threadIdx.x == 0 && (off[0] != 0 || off[n] != m)) atomicOr(bad, kBadOffsets);
 }
 
-__global__ void k_fill_u32(uint32_t* p, uint64_t n, uint32_t x) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) p[i] = x;
-}
-
 // cn[] in the reference's edge order (GPUSCAN++/Graph.cpp:87-111): edge {u lower, v higher} has
 // id P[u] + (rank of v among the higher neighbours of u), P = prefix of the higher-neighbour
 // counts, which is off[u] - lo_off[u].
@@ -859,8 +855,8 @@ static scan_status launch_sketch_filter(DeviceGraph* d, uint32_t* launches, cons
                                      d->pend_counts + kPendCounts - 2, sim, pw, d->long_edges, d->cn_ctr);
     ++*launches;
     if (d->long_edges.cap) {
-        k_sketch_long<<<d->num_sms * 6, kThreads, 0, s>>>(d->long_edges, d->lo_adj, d->lo_src, d->sk_info, d->sk, d->sk_levels, sim,
-                                                          pw, d->cn_ctr);
+        k_sketch_long<<<d->num_sms * 6, kThreads, 0, s>>>(d->long_edges, d->lo_adj, d->lo_src, d->sk_info, d->sk,
+                                                          d->sk_levels, sim, pw, d->cn_ctr);
         ++*launches;
     }
     return SCAN_OK;
@@ -1131,8 +1127,8 @@ scan_status autotune_similarity(DeviceGraph* d, float* best_ms, const std::funct
     return SCAN_OK;
 }
 
-// Main stream: ev[7] (the list kernels' start, after the sketches of a one-shot run), class 2 -> ev[11], class 1 -> ev[10], class 0 -> ev[9],
-// small pivots -> ev[8]; side stream: the hubs from ev[7] to ev[15], then, after the sketches, the
+// Main stream: ev[7] (the list kernels' start, after the sketches of a one-shot run), class 2 ->
+// ev[11], class 1 -> ev[10], class 0 -> ev[9], small pivots -> ev[8]; side stream: the hubs from ev[7] to ev[15], then, after the sketches, the
 // small pivots -> ev[8].
 static void cn_kernel_times(DeviceGraph* d, scan_stats* st) {
     st->ms_cn_kernel[0] = ev_ms(d->sk && d->nhub ? d->ev[15] : d->ev[9], d->ev[8]);

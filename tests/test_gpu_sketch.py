@@ -127,3 +127,16 @@ def test_streamed_without_room_for_sketches():
     used = g.upload_streamed(0, 31 << 20)
     assert used < with_sketches - 2 * g.m
     check(g, [("0.3", 2), ("0.5", 5)], modes=(REF,))
+
+
+def test_hubs_of_many_chunks_with_their_edges_pending(monkeypatch):
+    """96 joined hubs over 120,000 shared leaves, each hub's list in 20 chunks: nearly every edge
+    between hubs is left open, so each chunk task of a hub has edges to be cut into slices, and
+    charged with their whole lists the tasks would ask for about twice the slices there is room
+    for."""
+    monkeypatch.setenv("SCAN_GB300_BITMAP", "off")
+    hubs, leaves = 96, 120_000
+    i, j = np.triu_indices(hubs, 1)
+    h, x = np.divmod(np.arange(hubs * leaves), leaves)
+    pairs = np.concatenate([np.stack([i, j], 1), np.stack([h, hubs + x], 1)])
+    check(sg.Graph.from_edges(hubs + leaves, pairs), [("0.5", 2)])
