@@ -176,8 +176,9 @@ def byte_models(off: np.ndarray, adj: np.ndarray, eps: str) -> dict:
     this eps (du + 1 >= eps^2 (dv + 1), u the lower endpoint); each such list once (4 du),
     every pivot list staged once (4 d_v), and every edge costs its endpoint, two offsets
     and its count (16 B) plus the zeroing of cn (4 B):  B = 4 sum_counted du + 4 sum_v d_v + 20 E.
-    (The roofline's own figure replaces 4 sum_counted du by the list words the kernels
-    report reading, which also reflects the early stop.)
+    (The roofline's own figure replaces 4 sum_counted du by the words of bitmaps and lists that
+    the kernels report reading.  Most of them come from L1 and L2, so it can pass the HBM rate;
+    `traffic` is what DRAM supplies.)
     full model: the same with every edge counted (the cached counts of the serving path).
     merge model (what a merge intersection of every edge reads): each edge streams both lists,
       B = sum_e [4 (du + dv) + 16] + 4 E = 4 sum_v d_v^2 + 20 E.
@@ -608,7 +609,8 @@ def main():
             "frac": run_bytes / sim_s / 1e9 / peak, "traffic": traffic, "traffic_source": traffic_src,
             "peak_source": peak_src,
             "bytes": run_bytes, "list_words_read": words, "counted_edges": int(last["cn_edges_counted"]),
-            "bytes_model": "16*(list words read, reported by the kernels) + 4*sum_v d_v + 20E",
+            "bytes_model": "16*(bitmap and list words read, reported by the kernels; from L1, L2 and HBM) "
+                           "+ 4*sum_v d_v + 20E",
             "prune_model": dict(gbs(bm["prune"]), counted_edges=bm["counted_edges"],
                                 definition="4*sum over edges left by the degree prune of min(du,dv) + 4*sum_v d_v + 20E"),
             "full_model": dict(gbs(bm["full"]), definition="every edge counted (serving cache)"),

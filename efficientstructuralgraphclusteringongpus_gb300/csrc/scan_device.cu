@@ -162,7 +162,7 @@ static void cache_give(int dev, void* p, size_t bytes) {
 
 // Streams, events and the pinned result staging of a resident graph come from a per-device pool
 // and go back to it when the graph is freed, so that a GPUScan() call (upload, run, free)
-// creates and destroys none of its 3 streams and 29 events.
+// creates and destroys none of its 3 streams and 27 events.
 struct StreamSet {
     cudaStream_t stream, side, aux;
     cudaEvent_t fork, join, ev[16], chunk_ev[9];
