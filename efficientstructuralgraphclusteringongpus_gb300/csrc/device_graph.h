@@ -153,15 +153,15 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
 // cn for every edge on d->stream.
 // With `prune` (a one-shot run; the result is not a reusable cache, and run is the run's
 // scratch): edges that the degree prune rules out at that eps are skipped and keep cn = 0,
-// and where the graph has sketches they decide most of the others (run->sim holds the edge
-// states meanwhile).  When one_shot_predicate(d), the predicate is run too, into run's sim,
+// and where the graph has sketches (and they pay at that eps) they decide most of the others
+// (run->sim holds the edge states meanwhile).  When one_shot_predicate(d, *prune), the predicate is run too, into run's sim,
 // sd and counters, and launch_cluster is then told so (predicate_done).
 struct BatchParams;
 // bp (batched runs, with prune, no split pivot): each pivot takes eps and the predicate from
 // its graph's entry of bp->gpp (prune then only supplies "on").
 scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune = nullptr,
                       const RunScratch* run = nullptr, const BatchParams* bp = nullptr);
-bool one_shot_predicate(const DeviceGraph* d);
+bool one_shot_predicate(const DeviceGraph* d, const PredParams& p);
 // Counts of every edge into d->cn by triangles (kernels_tri.cuh), on d->stream, waiting for it.
 // The counts in the reference's order are copied to out_host unless it is null.  Working
 // memory comes from the device-buffer cache; where there is none left, by launch_cn.

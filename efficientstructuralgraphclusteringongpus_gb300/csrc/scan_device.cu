@@ -1011,6 +1011,18 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     return SCAN_OK;
 }
 
+// Below this eps the sketches of a graph of kSketchLowEdges edges leave most of its edges open,
+// and the list kernels that bound a count first (k_cn_filter_classes) are the faster ones for so
+// many.  Whole runs in ms, by sketches / by lists alone: power law of 57M edges, eps 0.1 49 / 37,
+// 0.12 45 / 36, 0.15 31 / 34; R-MAT s22 (64M) 0.1 92 / 51, 0.15 47 / 45, 0.2 16 / 39; s23 0.1
+// 248 / 174, 0.2 47 / 132.  On smaller graphs the sketches win at most eps (R-MAT s18 0.05 4.4 /
+// 9.9, 0.1 4.4 / 9.0; s20 18 / 28, 19 / 19; s21 24 / 37, 25 / 17).
+constexpr double kSketchLowEps = 0.15;
+constexpr uint64_t kSketchLowEdges = 1u << 25;
+static bool with_sketches(const DeviceGraph* d, const PredParams& p) {
+    return d->sk && (p.eps >= kSketchLowEps || d->E < kSketchLowEdges);
+}
+
 // cn for every edge (the similarity stage); events 7..12 bracket its kernels.
 scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune, const RunScratch* run,
                       const BatchParams* bp) {
@@ -1026,7 +1038,7 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
     FusedPred fp{nullptr, nullptr, nullptr, nullptr};
     const bool fused = run && prune && !d->has_split;
     if (fused) fp = FusedPred{run->sim, run->sd, run->ctr, nullptr};
-    if (run && prune && d->sk) fp.pend = run->sim;
+    if (run && prune && (per_graph ? d->sk != nullptr : with_sketches(d, *prune))) fp.pend = run->sim;
     if (per_graph && !fp.sim) return fail(SCAN_ERR_INVALID_ARG, "per-graph parameters need the fused one-shot path");
     cudaStream_t s = d->stream;
     if (!fused || !fp.pend) SCAN_CUDA(cudaMemsetAsync(d->cn, 0, d->E * sizeof(uint32_t), s));
@@ -1059,7 +1071,7 @@ scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prun
 // A one-shot launch_cn also runs the predicate: with no split pivot the counting kernels do
 // (each count is final in the lane that computes it), and after the sketches the few edges of
 // split pivots take a pass of their own.
-bool one_shot_predicate(const DeviceGraph* d) { return !d->has_split || d->sk; }
+bool one_shot_predicate(const DeviceGraph* d, const PredParams& p) { return !d->has_split || with_sketches(d, p); }
 
 // Autotuner: a coordinate search over the plan, each setting timed on this graph with
 // `stage` (the similarity stage as the caller runs it; null: full counts).  In order:
@@ -1128,10 +1140,10 @@ scan_status autotune_similarity(DeviceGraph* d, float* best_ms, const std::funct
 }
 
 // Main stream: ev[7] (the list kernels' start, after the sketches of a one-shot run), class 2 ->
-// ev[11], class 1 -> ev[10], class 0 -> ev[9], small pivots -> ev[8]; side stream: the hubs from ev[7] to ev[15], then, after the sketches, the
-// small pivots -> ev[8].
-static void cn_kernel_times(DeviceGraph* d, scan_stats* st) {
-    st->ms_cn_kernel[0] = ev_ms(d->sk && d->nhub ? d->ev[15] : d->ev[9], d->ev[8]);
+// ev[11], class 1 -> ev[10], class 0 -> ev[9], small pivots -> ev[8]; side stream: the hubs from
+// ev[7] to ev[15], then, after the sketches, the small pivots -> ev[8].
+static void cn_kernel_times(DeviceGraph* d, bool sketches, scan_stats* st) {
+    st->ms_cn_kernel[0] = ev_ms(sketches && d->nhub ? d->ev[15] : d->ev[9], d->ev[8]);
     for (int c = 0; c < kNumBigClasses; ++c)
         st->ms_cn_kernel[1 + c] = ev_ms(c == kNumBigClasses - 1 ? d->ev[7] : d->ev[10 + c], d->ev[9 + c]);
     st->ms_cn_kernel[4] = d->nhub ? ev_ms(d->ev[7], d->ev[15]) : 0.0;
@@ -1311,7 +1323,7 @@ static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bo
     SCAN_CUDA(cudaEventRecord(d->ev[3], s));
     d->cn_valid_before = d->cn_valid;
     const bool count = !(reuse_cn && d->cn_valid);
-    const bool fused = count && one_shot_predicate(d);
+    const bool fused = count && one_shot_predicate(d, pp);
     if (count) {
         d->cn_valid = false;
         SCAN_TRY(launch_cn(d, &launches, &pp, &d->rs));
@@ -1367,7 +1379,7 @@ static scan_status run_resident(DeviceGraph* d, const PredParams& pp, int mu, bo
         st->ms_d2h = ev_ms(d->ev[5], d->ev[6]);
         st->ms_total = ev_ms(d->ev[3], d->ev[6]);
         if (count) {
-            cn_kernel_times(d, st);
+            cn_kernel_times(d, with_sketches(d, pp), st);
             st->cn_words = hc.list_words;
             st->cn_edges_counted = hc.edges_counted;
         }
