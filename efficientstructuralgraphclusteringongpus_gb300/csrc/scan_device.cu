@@ -152,7 +152,17 @@ extern "C" uint64_t scan_cached_memory_bytes(int device) {
     return g_cache_bytes[device];
 }
 
+// Device memory this host thread may still take (scan_set_device_memory_left).
+static thread_local uint64_t t_memory_left = UINT64_MAX;
+
+extern "C" void scan_set_device_memory_left(uint64_t bytes) { t_memory_left = bytes; }
+
+static void memory_left_take(size_t bytes) {
+    if (t_memory_left != UINT64_MAX) t_memory_left -= std::min<uint64_t>(bytes, t_memory_left);
+}
+
 static void cache_give(int dev, void* p, size_t bytes) {
+    if (t_memory_left != UINT64_MAX) t_memory_left += bytes;
     if (dev < 0 || dev >= 64) { cudaFree(p); return; }
     std::lock_guard<std::mutex> lock(g_cache_mu);
     if (g_cache_bytes[dev] + bytes > g_cache_cap) { cudaFree(p); return; }
@@ -265,8 +275,14 @@ void device_graph_free(DeviceGraph* d) {
 // cached one may be larger), to be given back with it.
 static scan_status cache_alloc(int device, size_t bytes, void** p, size_t* got) {
     *got = bytes;
+    *p = nullptr;
+    if (bytes > t_memory_left)
+        return fail(SCAN_ERR_OUT_OF_MEMORY, std::to_string(bytes) + " bytes of device memory, above the limit of this thread");
     *p = cache_take(device, bytes, got);
-    if (*p) return SCAN_OK;
+    if (*p) {
+        memory_left_take(*got);
+        return SCAN_OK;
+    }
     cudaError_t err = cudaMalloc(p, bytes);
     if (err != cudaSuccess) {
         cudaGetLastError();
@@ -280,6 +296,7 @@ static scan_status cache_alloc(int device, size_t bytes, void** p, size_t* got) 
         return fail(SCAN_ERR_OUT_OF_MEMORY, "cudaMalloc of " + std::to_string(bytes) +
                                                 " bytes failed: " + cudaGetErrorString(err));
     }
+    memory_left_take(bytes);
     return SCAN_OK;
 }
 
@@ -1229,7 +1246,8 @@ static scan_status full_counts_by_lists(DeviceGraph* d, uint32_t* launches, uint
     return SCAN_OK;
 }
 
-scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
+// SCAN_ERR_OUT_OF_MEMORY: nothing was queued and no memory is held.
+static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
     cudaStream_t s = d->stream;
     const uint64_t E = d->E;
     CallBuffers mem(d->device);
@@ -1243,10 +1261,6 @@ scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) 
     if (st == SCAN_OK) st = mem.get(&small, std::min<uint64_t>(d->n, E));
     if (st == SCAN_OK) st = mem.get(&big, slices);
     if (st == SCAN_OK) st = mem.get(&ctr, 3 * kSpan);
-    if (st == SCAN_ERR_OUT_OF_MEMORY) {
-        clear_error();
-        return full_counts_by_lists(d, launches, out_host);
-    }
     if (st != SCAN_OK) return st;
     auto queue = [&]() -> scan_status {
         SCAN_CUDA(cudaEventRecord(d->ev[3], s));
@@ -1276,6 +1290,13 @@ scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) 
     if (st != SCAN_OK) return st;
     SCAN_CUDA(err);
     return SCAN_OK;
+}
+
+scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
+    const scan_status st = full_counts_by_triangles(d, launches, out_host);
+    if (st != SCAN_ERR_OUT_OF_MEMORY) return st;
+    clear_error();
+    return full_counts_by_lists(d, launches, out_host);   // half the memory: what the triangles had got is back
 }
 
 scan_status compute_tau(DeviceGraph* d) {

@@ -363,6 +363,10 @@ scan_status scan_eps_to_decimal(double eps, char* buf, size_t buflen);
  * completes with that status); the device stays usable.  Applies to work queued after the
  * call, process-wide; a batch keeps the rounds it was captured with. */
 void scan_set_loop_limits(int64_t union_find_iterations, int32_t jump_rounds_cap);
+/* The engine's device allocations from this host thread behave as on a device with `bytes` left:
+ * one above what is left fails like a cudaMalloc without memory, and what the engine gives back
+ * on this thread (into its cache too) is left again.  UINT64_MAX, the default: no limit. */
+void scan_set_device_memory_left(uint64_t bytes);
 
 #ifdef __cplusplus
 }
