@@ -206,27 +206,46 @@ __device__ __forceinline__ uint32_t similar_bits(const uint8_t* sim, uint64_t k,
 // each lower neighbour's in turn would let one CAS per round succeed; instead the lanes of a
 // run agree on the smallest of their roots and hang their own root under that (all different
 // words), the first lane v's root as well.  Edges whose endpoints already point to one vertex
-// end after two loads.  Cluster stage of communities of 6M edges 0.50 -> 0.30 ms; unions of 30
-// served queries 2.24 -> 1.41 ms.
+// end after two loads, and since L1 may keep a pointer from before the unions, after two from
+// L2.  Cluster stage of communities of 6M edges 0.50 -> 0.30 ms.
+//
+// A warp takes 32 W edges: where many of them are similar in turns of 32 consecutive ones, else
+// in turns of each lane's next.  (Each lane's next throughout: grid of 2000 x 2000 at eps 0.2
+// 1.4-1.7 ms, now 0.8.)
+//
+// Of the tiles of 32 W edges, every `every`-th is visited.
 template <int W>
 __device__ __forceinline__ void union_pass(Team team, uint64_t E, const uint32_t* __restrict__ lo_adj,
                                            const uint32_t* __restrict__ lo_src, const uint8_t* sim, int32_t* parent,
-                                           RunCounters* ctr, uint32_t limit) {
+                                           RunCounters* ctr, uint32_t limit, uint32_t every) {
     if (!*(volatile uint32_t*)&ctr->any_core) return;   // no core: nothing to join
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31;
-    for (uint64_t e0 = W * (team.index - lane); e0 < E; e0 += W * team.size) {
+    for (uint64_t e0 = W * (team.index - lane) * every; e0 < E; e0 += W * team.size * every) {
         uint32_t bits = similar_bits<W>(sim, e0 + W * lane, E);
-        while (__any_sync(kFull, bits)) {
+        const uint32_t most = __reduce_max_sync(kFull, (uint32_t)__popc(bits));
+        const bool dense = most > 2;
+        for (uint32_t q = 0; q < (dense ? (uint32_t)W : most); ++q) {
+            uint32_t i = W * lane + __ffs(bits) - 1;     // this lane's edge of the turn
+            bool mine = bits != 0;
+            if (dense) {
+                i = 32 * q + lane;
+                mine = __shfl_sync(kFull, bits, i / W) >> (i % W) & 1u;
+            } else {
+                bits &= bits - 1;
+            }
             int32_t u = 0, v = 0;
             bool join = false;
-            if (bits) {
-                const uint64_t e = e0 + W * lane + __ffs(bits) - 1;
-                bits &= bits - 1;
+            if (mine) {
+                const uint64_t e = e0 + i;
                 u = (int32_t)lo_adj[e];
                 v = (int32_t)lo_src[e];
                 const int32_t pu = parent[u], pv = parent[v];
                 join = pu >= 0 && pv >= 0 && pu != pv;      // core-core only (cores never change)
+                if (join) {
+                    const volatile int32_t* vp = parent;
+                    join = vp[u] != vp[v];
+                }
             }
             if (!__any_sync(kFull, join)) continue;
             if (join) {
@@ -248,7 +267,23 @@ __device__ __forceinline__ void union_pass(Team team, uint64_t E, const uint32_t
 }
 __global__ void k_union(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
                         const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit) {
-    union_pass<4>(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit);
+    union_pass<4>(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit, 1);
+}
+
+// A sample of the edges, before the others.  When a run starts every core is its own root, and
+// where most cores belong to one cluster all resident warps then swing the same few pointers:
+// the fewer the edges, the more of them do so at once (served query at eps 0.2 on R-MAT of 213K
+// edges 70-330 us of unions, of 15.7M 40-180; complete graph of 1,500 vertices 140-370).  A
+// sample of few warps joins most of such a cluster, and the others find it joined (31, 41-60
+// and 50-75 us, both launches).  Where there is no such cluster it costs its launch, about 3 us,
+// and where the cores form small clusters up to 10 (run on communities of 6M edges 843 -> 858
+// us): served queries, whose unions are most of their time, take it, runs do not.
+constexpr uint64_t kUnionSample = 1u << 15;      // edges; 2^17 is no faster and costs up to 25 us where nothing contends
+constexpr uint32_t kUnionSampleLeast = 16;       // at most every 16th tile
+__global__ void k_union_sample(uint64_t E, const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
+                               const uint8_t* __restrict__ sim, int32_t* parent, RunCounters* ctr, uint32_t limit,
+                               uint32_t every) {
+    union_pass<1>(grid_team(), E, lo_adj, lo_src, sim, parent, ctr, limit, every);
 }
 
 // Flatten by pointer jumping: a round moves parent[v] of every core up to kJumpSteps ancestors on
@@ -482,7 +517,7 @@ k_cluster_small(FusedCluster f, PredParams pp) {
     core_init_pass(team, f.n, f.sd, f.mu, nullptr, nullptr, f.parent, f.bmin, f.bmax, f.nmin, f.nmax, f.ctr);
     cluster_barrier();
     if (*(volatile uint32_t*)&f.ctr->any_core) {          // the same in every thread, as below
-        union_pass<1>(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.ctr, f.limit);
+        union_pass<1>(team, f.E, f.lo_adj, f.lo_src, f.sim, f.parent, f.ctr, f.limit, 1);
         cluster_barrier();
         for (uint32_t r = 0; r < f.rounds; ++r) {
             const uint32_t ch = jump_pass(team, f.n, f.parent);

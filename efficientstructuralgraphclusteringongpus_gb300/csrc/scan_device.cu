@@ -1199,6 +1199,12 @@ scan_status launch_cluster(const DeviceGraph* d, const RunScratch& r, cudaStream
     }
     k_core_init<<<gn, T, 0, s>>>(n, r.sd, mu, vgid, bp ? bp->gmu : nullptr, r.parent, r.bmin, r.bmax, r.nmin, r.nmax,
                                  r.ctr);
+    if (by_tau) {
+        const uint32_t every = (uint32_t)std::max<uint64_t>(kUnionSampleLeast, E / kUnionSample);
+        k_union_sample<<<grid_for_n(sms, E / every, T), T, 0, s>>>(E, d->lo_adj, d->lo_src, r.sim, r.parent, r.ctr,
+                                                                   union_find_limit(), every);
+        ++*launches;
+    }
     k_union<<<ge, T, 0, s>>>(E, d->lo_adj, d->lo_src, r.sim, r.parent, r.ctr, union_find_limit());
     const uint32_t rounds = jump_rounds(n);
     if (n <= kJumpBlockMax) {

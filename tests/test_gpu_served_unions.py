@@ -1,0 +1,76 @@
+"""Served queries join their cores rightly.
+
+A sample of the edges is joined before the others (every tile of 32 edges of 16 or more), then a
+warp takes 128 edges, in turns of 32 consecutive ones where more than two of four are similar and
+of each lane's next otherwise; queries on up to 2^14 edges take one launch instead.  The graphs sit
+at those sizes, with one cluster of everything, many small ones, long thin ones, and few similar
+edges.  All results are whole numbers: they equal the oracle's.
+"""
+import numpy as np
+import pytest
+
+import efficientstructuralgraphclusteringongpus_gb300 as sg
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def complete(n):
+    i, j = np.triu_indices(n, 1)
+    return sg.Graph.from_edges(n, np.stack([i, j], 1))
+
+
+def cliques(count, size, extra, seed):
+    i, j = np.triu_indices(size, 1)
+    base = np.arange(count)[:, None] * size
+    r = np.random.RandomState(seed)
+    n = count * size
+    return sg.Graph.from_edges(n, np.concatenate([np.stack([(base + i).ravel(), (base + j).ravel()], 1),
+                                                  r.randint(0, n, (extra, 2))]))
+
+
+def ring(n, k):
+    i = np.arange(n)
+    return sg.Graph.from_edges(n, np.concatenate([np.stack([i, (i + s) % n], 1) for s in range(1, k + 1)]))
+
+
+def grid(w):
+    i = np.arange(w * w)
+    right, down = i[i % w != w - 1], i[:-w]
+    return sg.Graph.from_edges(w * w, np.concatenate([np.stack([right, right + 1], 1), np.stack([down, down + w], 1)]))
+
+
+def random_edges(n, edges, seed):
+    r = np.random.RandomState(seed)
+    e = np.unique(np.sort(r.randint(0, n, (3 * edges, 2)), axis=1), axis=0)
+    e = e[e[:, 0] != e[:, 1]]
+    return sg.Graph.from_edges(n, e[r.permutation(len(e))[:edges]])
+
+
+GRAPHS = {
+    "around_2^14": lambda: [random_edges(3000, e, e) for e in (16383, 16384, 16385, 16512, 16513)],
+    "around_2^19": lambda: [random_edges(20000, e, e) for e in ((1 << 19) - 1, (1 << 19) + 1, (1 << 19) + 33)],
+    "complete": lambda: [complete(n) for n in (182, 183, 400, 1201)],
+    "cliques": lambda: [cliques(700, 9, 5000, 1), cliques(60, 41, 20000, 2), cliques(9000, 3, 3000, 3)],
+    "rings": lambda: [ring(20000, 3), ring(70001, 1), ring(4001, 40)],
+    "grids": lambda: [grid(150), grid(401)],
+    "rmat": lambda: [sg.Graph.rmat(11, 9, seed=3), sg.Graph.rmat(14, 16, seed=4), sg.Graph.rmat(16, 13, seed=5)],
+}
+
+
+@pytest.mark.parametrize("name", GRAPHS)
+def test_served_equal_the_oracle(name):
+    graphs = GRAPHS[name]()
+    counts = [oracle.common_neighbors(g.offsets(), g.adjacency()) for g in graphs]
+    points = [("0.05", 2), ("0.2", 2), ("0.5", 3), ("0.9", 2)]
+    with sg.Server(0, 256 << 20, 4) as srv:
+        ids = [srv.add_graph(g) for g in graphs]
+        queries = [(k, eps, mu, mode) for k in range(len(graphs)) for eps, mu in points
+                   for mode in (sg.PRED_EXACT, sg.PRED_REF_F64)]
+        tickets = [srv.submit(ids[k], eps, mu, mode) for k, eps, mu, mode in queries]
+        for (k, eps, mu, mode), t in zip(queries, tickets):
+            label, role, st = srv.wait(t)
+            want = oracle.scan_ex(graphs[k].offsets(), graphs[k].adjacency(), eps, mu, mode, cn=counts[k])
+            assert np.array_equal(label, want[0]) and np.array_equal(role, want[1]), (name, k, eps, mu, mode)
+            assert st["num_cores"] == want[2]["cores"] and st["num_clusters"] == want[2]["clusters"]
+            assert st["num_similar_edges"] == want[2]["similar_edges"]
