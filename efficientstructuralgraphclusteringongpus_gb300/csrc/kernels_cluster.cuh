@@ -476,11 +476,13 @@ __global__ void k_finalize(uint32_t n, const int32_t* __restrict__ parent, const
 // bounds it there is the chain of eight to sixteen dependent launches, and the hardware's
 // cluster barrier between the passes costs about a microsecond.  A run of 10K edges spends 22 us
 // here instead of 35; from about 80K edges eight SMs take longer over the edges than the launches
-// do (communities: 148 us a run by launches, 171 fused).  Served queries run many at a time and
-// wait for their launches instead: fused up to a million edges, a burst of 30 mixed queries takes
-// 2.0 ms, up to 256K 2.8, by launches alone 3.4-3.8.  predicate: 0 done by the similarity stage,
-// 1 cached thresholds (tau); with 1 it also clears what the passes start from.
-constexpr uint64_t kFusedEdgesRun = 1u << 16, kFusedEdgesServed = 1u << 20;
+// do (communities: 148 us a run by launches, 171 fused).  A served query also has the predicate
+// over every edge in it, so its line lies lower (a query alone / sixteen at once, us, fused and by
+// launches: R-MAT of 10K edges 155 / 550 and 170 / 540, complete graph of 20K 160 / 800 and 165 /
+// 530, R-MAT of 213K at eps 0.5 195 / 580 and 169 / 550, communities of 750K 860 / 3150 and 235 /
+// 810).  predicate: 0 done by the similarity stage, 1 cached thresholds (tau); with 1 it also
+// clears what the passes start from.
+constexpr uint64_t kFusedEdgesRun = 1u << 16, kFusedEdgesServed = 1u << 14;
 constexpr uint32_t kFusedVertices = 1u << 17;
 constexpr int kFusedCtas = 8, kFusedThreads = 1024;
 

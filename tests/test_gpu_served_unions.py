@@ -1,4 +1,4 @@
-"""Served queries join their cores rightly.
+"""Served queries join their cores in the time the same launches take a run, and rightly.
 
 A sample of the edges is joined before the others (every tile of 32 edges of 16 or more), then a
 warp takes 128 edges, in turns of 32 consecutive ones where more than two of four are similar and
@@ -74,3 +74,14 @@ def test_served_equal_the_oracle(name):
             assert np.array_equal(label, want[0]) and np.array_equal(role, want[1]), (name, k, eps, mu, mode)
             assert st["num_cores"] == want[2]["cores"] and st["num_clusters"] == want[2]["clusters"]
             assert st["num_similar_edges"] == want[2]["similar_edges"]
+
+
+def test_served_query_takes_no_longer_than_a_runs_cluster_stage():
+    """The stage is the same but for the predicate (one compare per edge), so three times a run's and
+    a tenth of a millisecond is ample; in one launch over eight SMs it took ten times a run's."""
+    g = cliques(1100, 37, 50_000, 7)           # 780,000 edges in small clusters
+    run_ms = min(g.run("0.4", 3).stats["ms_cluster"] for _ in range(5))
+    with sg.Server(0, 64 << 20, 1) as srv:
+        gid = srv.add_graph(g)
+        served_ms = min(srv.wait(srv.submit(gid, "0.4", 3))[2]["device_ms"] for _ in range(5))
+    assert served_ms < 3 * run_ms + 0.1, (served_ms, run_ms)
