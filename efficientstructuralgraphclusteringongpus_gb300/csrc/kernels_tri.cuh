@@ -296,4 +296,49 @@ __global__ void k_from_reference_order(uint64_t E, const uint32_t* __restrict__ 
     }
 }
 
+// Whether the list kernels count faster: graphs of nearly complete neighbourhoods.  A streamed
+// entry that is in the table costs two to three times one that is not (the queue, the lookup, three
+// atomics), and where degrees are alike the lists are only 1.5 to 2 times the entries the triangles
+// stream.  Full counts, ms, by lists / by triangles: complete graphs of 1,500 and 4,000 vertices
+// 2.5 / 3.8 and 39 / 72, disjoint ones of 120, 300 and 800 1.70 / 1.98, 3.37 / 3.76 and 7.2 / 9.2,
+// ring lattices of degree 200 and 600 1.33 / 1.52 and 2.32 / 2.55; half of the entries of each are
+// hits.  With a quarter hits (communities of degree 170) 1.75 / 1.61, a sixth 5.0 / 4.0; and at
+// lower degrees launches and latency decide (disjoint ones of 48 0.97 / 0.85, a ring lattice of
+// degree 32 1.43 / 0.85).  So graphs of at least kTriDenseDegree neighbours on average are looked
+// at: random entries of the lists of random edges (the first few thousand multiples of a prime),
+// about 20 us.  sums[0] entries of the lists, [1] of those the triangles stream, [2] samples found.
+constexpr uint64_t kTriDenseEdges = 1u << 19;
+constexpr uint32_t kTriDenseDegree = 96, kTriSamples = 8192;
+__host__ __device__ constexpr bool tri_dense(uint64_t lists, uint64_t streamed, uint64_t hits) {
+    return 4 * lists <= 9 * streamed && 5 * hits >= 2 * streamed;
+}
+
+__global__ void k_tri_sample(uint64_t E, const uint32_t* __restrict__ off, const uint32_t* __restrict__ lo_off,
+                             const uint32_t* __restrict__ lo_adj, const uint32_t* __restrict__ lo_src,
+                             const uint32_t* __restrict__ hi_adj, unsigned long long* __restrict__ sums) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t lists = 0, streamed = 0, hits = 0;
+    if (i < kTriSamples) {
+        const uint64_t e = (i * 2654435761ull) % E;
+        const uint32_t a = lo_adj[e], b = lo_src[e];
+        const uint32_t ab = hi_begin(off, lo_off, a), ae = hi_begin(off, lo_off, a + 1);
+        lists = off[a + 1] - off[a];
+        streamed = ae - ab;
+        if (streamed) {
+            const uint32_t c = hi_adj[ab + __umulhi(i * 0x9E3779B1u, streamed)];
+            const uint32_t be = hi_begin(off, lo_off, b + 1);
+            const uint32_t at = lower_bound_u32(hi_adj, hi_begin(off, lo_off, b), be, c);
+            if (at < be && hi_adj[at] == c) hits = streamed;      // an entry stands for its list
+        }
+    }
+    lists = __reduce_add_sync(0xFFFFFFFFu, lists);
+    streamed = __reduce_add_sync(0xFFFFFFFFu, streamed);
+    hits = __reduce_add_sync(0xFFFFFFFFu, hits);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sums[0], (unsigned long long)lists);
+        atomicAdd(&sums[1], (unsigned long long)streamed);
+        atomicAdd(&sums[2], (unsigned long long)hits);
+    }
+}
+
 }  // namespace scan

@@ -1252,12 +1252,12 @@ static scan_status full_counts_by_lists(DeviceGraph* d, uint32_t* launches, uint
     return SCAN_OK;
 }
 
-// SCAN_ERR_OUT_OF_MEMORY: nothing was queued and no memory is held.
-static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
+// SCAN_ERR_OUT_OF_MEMORY, or *dense set: nothing was counted and no memory is held.
+static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, uint32_t* out_host, bool* dense) {
     cudaStream_t s = d->stream;
     const uint64_t E = d->E;
     CallBuffers mem(d->device);
-    // counters, 256 bytes apart: [0] numbers of small pivots and of slices, then their queues
+    // counters, 256 bytes apart: [0] numbers of small pivots and of slices, then their queues, the sample
     constexpr int kSpan = 64;
     uint32_t *hi_adj = nullptr, *cnt = nullptr, *small = nullptr, *ctr = nullptr;
     uint2* big = nullptr;
@@ -1266,14 +1266,25 @@ static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, 
     if (st == SCAN_OK) st = mem.get(&cnt, E);
     if (st == SCAN_OK) st = mem.get(&small, std::min<uint64_t>(d->n, E));
     if (st == SCAN_OK) st = mem.get(&big, slices);
-    if (st == SCAN_OK) st = mem.get(&ctr, 3 * kSpan);
+    if (st == SCAN_OK) st = mem.get(&ctr, 4 * kSpan);
     if (st != SCAN_OK) return st;
     auto queue = [&]() -> scan_status {
         SCAN_CUDA(cudaEventRecord(d->ev[3], s));
         SCAN_CUDA(cudaMemsetAsync(cnt, 0, std::max<uint64_t>(E, 1) * sizeof(uint32_t), s));
-        SCAN_CUDA(cudaMemsetAsync(ctr, 0, 3 * kSpan * sizeof(uint32_t), s));
+        SCAN_CUDA(cudaMemsetAsync(ctr, 0, 4 * kSpan * sizeof(uint32_t), s));
         if (E) {
             k_fill_higher<<<grid_for(d, d->m, 256), 256, 0, s>>>(d->m, d->adj, d->lowbits, d->wpre, hi_adj);
+            // (a streamed graph's lists are read over the host link: triangles, however dense)
+            if (!d->adj_host && E >= kTriDenseEdges && d->m >= (uint64_t)kTriDenseDegree * d->n) {
+                auto* sums = reinterpret_cast<unsigned long long*>(ctr + 3 * kSpan);
+                k_tri_sample<<<kTriSamples / 256, 256, 0, s>>>(E, d->off, d->lo_off, d->lo_adj, d->lo_src, hi_adj, sums);
+                ++*launches;
+                const auto* h = reinterpret_cast<const unsigned long long*>(d->h_res);
+                SCAN_CUDA(cudaMemcpyAsync(d->h_res, sums, 3 * sizeof(*sums), cudaMemcpyDeviceToHost, s));
+                SCAN_CUDA(cudaStreamSynchronize(s));
+                *dense = tri_dense(h[0], h[1], h[2]);
+                if (*dense) return SCAN_OK;
+            }
             k_tri_plan<<<grid_for(d, d->n, 256), 256, 0, s>>>(d->n, d->off, d->lo_off, ctr, small, big);
             const unsigned gb = (unsigned)std::min<uint64_t>(slices, (uint64_t)d->num_sms * kTriCtas);
             k_tri_big<<<gb, kTriWarps * 32, 0, s>>>(big, ctr, ctr + kSpan, d->off, d->lo_off, d->lo_adj, hi_adj, cnt);
@@ -1299,8 +1310,9 @@ static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, 
 }
 
 scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host) {
-    const scan_status st = full_counts_by_triangles(d, launches, out_host);
-    if (st != SCAN_ERR_OUT_OF_MEMORY) return st;
+    bool dense = false;
+    const scan_status st = full_counts_by_triangles(d, launches, out_host, &dense);
+    if (st != SCAN_ERR_OUT_OF_MEMORY && !dense) return st;
     clear_error();
     return full_counts_by_lists(d, launches, out_host);   // half the memory: what the triangles had got is back
 }
