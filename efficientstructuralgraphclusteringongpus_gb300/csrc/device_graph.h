@@ -98,6 +98,7 @@ struct DeviceGraph {
     uint32_t* hot = nullptr;       // n: hot id or kHotBits + v
     uint32_t* radj = nullptr;      // m + pad: adjacency mapped through hot[]
     uint32_t* tailc = nullptr;     // n: non-hot neighbours per vertex
+    bool tails = false;            // some vertex with an edge is not hot
     scan::CnTask* hubs = nullptr;  // hub tasks (pivots above plan.bitmap_min_deg)
     uint32_t nhub = 0;
     uint32_t cap_small = 0, cap_big[scan::kNumBigClasses] = {}, cap_hubs = 0;   // task array capacities

@@ -37,10 +37,16 @@ constexpr uint32_t kChunkMax = 6144;       // default max pivot entries staged b
 constexpr uint32_t kChunkMaxCap = 12288;   // largest allowed (load 1/2 in the same table)
 // Bitmap path: the kHotBits highest-degree vertices get ids in [0, kHotBits) ("hot");
 // every other vertex x is kHotBits + x.  A pivot's hot neighbours go into a shared-memory
-// bitmap (one bit per hot id, 128 KB), the rest (its "tail") into a bucketed table.
+// bitmap (one bit per hot id, 128 KB), the rest (its "tail") into a bucketed table with a hashed
+// bitmap in front.  In graphs with no more than kHotBits vertices of a neighbour there are no tails.
 constexpr uint32_t kHotBits = 1u << 20;
-constexpr uint32_t kTailSlots = 24576;     // 96 KB; tails up to kTailMax entries (load <= 1/2)
-constexpr uint32_t kTailMax = kTailSlots / 2;
+constexpr uint32_t kTailMax = 12288;       // longest tail
+constexpr uint32_t kTailSlots = 20480;     // 80 KB (load <= 0.6)
+constexpr uint32_t kTailBitsLog = 17;      // a hashed bitmap of the tail, 16 KB behind the hot one
+constexpr uint32_t kBitmapBits = kHotBits + (1u << kTailBitsLog);
+__host__ __device__ constexpr size_t bitmap_smem(bool tails) {
+    return tails ? (kBitmapBits / 32 + kTailSlots) * sizeof(uint32_t) : kHotBits / 8;
+}
 // Pivots above kBitmapMinDeg (the default of the plan's bitmap_min_deg) use the bitmap path
 // (when it is on): those the largest hash table would split.  Smaller pivots stay on the hash classes, which run several CTAs per
 // SM: a bitmap task of a mid-size pivot leaves most of its 32 warps waiting at the task
@@ -880,8 +886,18 @@ k_cn_filter_classes(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t 
 }
 
 // Bitmap path: one CTA of kBitmapThreads per task (pivot, edge slice), one CTA per SM.
-// Shared memory: the hot bitmap (zeroed once; each task sets its pivot's bits and clears
-// them again) and the tail table.  Probing an entry is one 4-byte shared load for hot ids.
+// Shared memory: the hot bitmap, behind it the tails' (zeroed once; each task sets its pivot's bits
+// and clears them again), and the tail table.  Probing an entry is one 4-byte shared load, and for the
+// few non-hot ids whose bit is set a lookup: looking up every non-hot entry, a warp did so in nearly
+// every round (R-MAT s22 at eps 0.15: this kernel 28 -> 22 ms; by lists alone at eps 0.1 the whole run
+// 52.7 -> 44.9).  Without tails (kTails false) the kernel knows none of it and leaves their shared
+// memory to L1 (R-MAT of 2^20 vertices and 51M edges at eps 0.2: 31.5 -> 24 ms).
+template <bool kTails>
+__device__ __forceinline__ uint32_t bitmap_bit(uint32_t w) {
+    return !kTails || w < kHotBits ? w : kHotBits + filter_bit(w, kTailBitsLog);
+}
+
+template <bool kTails>
 __device__ __forceinline__ uint32_t bitmap_probe_word(const uint4 x, uint32_t p, uint32_t lb, uint32_t le,
                                                       const uint32_t* bits, const uint32_t* tail, uint32_t ntb) {
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
@@ -890,11 +906,12 @@ __device__ __forceinline__ uint32_t bitmap_probe_word(const uint4 x, uint32_t p,
     for (int i = 0; i < 4; ++i) {
         const uint32_t pos = p + i;
         if (pos >= lb && pos < le) {
-            if (w[i] < kHotBits) c += (bits[w[i] >> 5] >> (w[i] & 31u)) & 1u;
-            else tails |= 1u << i;
+            const uint32_t b = bitmap_bit<kTails>(w[i]), hit = (bits[b >> 5] >> (b & 31u)) & 1u;
+            if (!kTails || w[i] < kHotBits) c += hit;
+            else tails |= hit << i;
         }
     }
-    while (tails) {
+    while (kTails && tails) {
         const int i = __ffs(tails) - 1;
         tails &= tails - 1;
         c += bucket_has(tail, ntb, w[i]);
@@ -904,7 +921,7 @@ __device__ __forceinline__ uint32_t bitmap_probe_word(const uint4 x, uint32_t p,
 
 // task.cb carries the pivot's tail size.
 // kPick: as in k_cn_big.
-template <bool kPerGraph, bool kPick>
+template <bool kPerGraph, bool kPick, bool kTails>
 __global__ void __launch_bounds__(kBitmapThreads, 1)
 k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, const uint32_t* __restrict__ off,
             const uint32_t* __restrict__ radj, const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn,
@@ -915,14 +932,15 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
         if (ntasks == 0) return;
     }
     extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* bits = smem;                              // kHotBits / 32 words
-    uint32_t* tail = smem + kHotBits / 32;              // kTailSlots words
+    uint32_t* bits = smem;                              // kBitmapBits / 32 words
+    uint32_t* tail = smem + kBitmapBits / 32;           // kTailSlots words
+    constexpr uint32_t kBits = kTails ? kBitmapBits : kHotBits;
     __shared__ uint32_t next_batch, task_slot;
     __shared__ CtaTotals totals;
     totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long nsim = 0, ndis = 0;
-    for (uint32_t i = threadIdx.x; i < kHotBits / 128; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < kBits / 128; i += blockDim.x)
         reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
     for (uint32_t t = next_task(queue, 0, true, &task_slot); t < ntasks;
          t = next_task(queue, t, false, &task_slot)) {
@@ -936,17 +954,20 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
         const uint32_t vb = off[tk.v], ve = off[tk.v + 1];
         const PivotTests pt = pivot_tests(ve - vb, P);
         uint32_t ntb = 8;                                // tail buckets: >= tail size (load <= 1/4),
-        while (ntb < tk.cb) ntb <<= 1;                   // capped at the table (load <= 1/2 there)
-        ntb = min(ntb, kTailSlots / 4);
-        for (uint32_t i = threadIdx.x; i < ntb; i += blockDim.x)
-            reinterpret_cast<uint4*>(tail)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+        if constexpr (kTails) {
+            while (ntb < tk.cb) ntb <<= 1;               // capped at the table (load <= 0.6 there)
+            ntb = min(ntb, kTailSlots / 4);
+            for (uint32_t i = threadIdx.x; i < ntb; i += blockDim.x)
+                reinterpret_cast<uint4*>(tail)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
+        }
         if (threadIdx.x == 0) next_batch = 0;
         __syncthreads();
 #pragma unroll 4
         for (uint32_t j = vb + threadIdx.x; j < ve; j += blockDim.x) {
             const uint32_t w = radj[j];
-            if (w < kHotBits) atomicOr(&bits[w >> 5], 1u << (w & 31u));
-            else bucket_insert(tail, ntb, w);
+            const uint32_t b = bitmap_bit<kTails>(w);
+            atomicOr(&bits[b >> 5], 1u << (b & 31u));
+            if (kTails && w >= kHotBits) bucket_insert(tail, ntb, w);
         }
         __syncthreads();
         for (;;) {
@@ -982,8 +1003,8 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
             uint32_t words = 0;
             const uint32_t cnt = count_batch<kWordsInFlightBitmap>(radj, lane, ub, ue, tlo, long_words, words,
                                                                    [&](uint4 x, uint32_t p, uint32_t lb, uint32_t le) {
-                                                                       return bitmap_probe_word(x, p, lb, le, bits,
-                                                                                                tail, ntb);
+                                                                       return bitmap_probe_word<kTails>(x, p, lb, le, bits,
+                                                                                                        tail, ntb);
                                                                    });
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, ue > ub));
             if (lane == 0) totals_add(&totals, words, kPick ? 0u : nc);
@@ -994,7 +1015,7 @@ k_cn_bitmap(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t* queue, 
 #pragma unroll 4
         for (uint32_t j = vb + threadIdx.x; j < ve; j += blockDim.x) {   // clear this pivot's bits
             const uint32_t w = radj[j];
-            if (w < kHotBits) bits[w >> 5] = 0u;
+            bits[bitmap_bit<kTails>(w) >> 5] = 0u;
         }
         __syncthreads();
     }

@@ -674,7 +674,8 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
             if (acc + h[b] > kHotBits) { min_bin = b + 1; break; }
             acc += h[b];
         }
-        if (mode == 2 && min_bin > 1) bitmap_path = false;   // some vertex would have a tail
+        d->tails = min_bin > 1;                              // some vertex is not hot
+        if (mode == 2 && d->tails) bitmap_path = false;
     }
     const uint64_t fill_tiles = (m + kFillTile - 1) / kFillTile;
     uint32_t* tile_v = nullptr;                                // first vertex of each adjacency tile
@@ -826,7 +827,7 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
 // Kernel attributes and occupancies, found once per device (so capturing launch_cn into a
 // CUDA graph queries nothing).  [g] is 1 for the instantiations with per-graph parameters.
 static bool g_attr_set[64][2][2] = {};      // k_cn_big, [g][after the sketches]
-static bool g_attr_bitmap[64][2][2] = {};   // [g][after the sketches]
+static bool g_attr_bitmap[64][2][2][2] = {};   // [g][after the sketches][with tails]
 static bool g_attr_filter[64][2] = {};      // k_cn_filter_classes, [g]
 static int g_per_sm[64][2][2][kNumBigClasses] = {};         // k_cn_big, [g][after the sketches][hash class]
 static int g_per_sm_sketch[64][2] = {};                      // k_sketch_filter
@@ -943,16 +944,21 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     // search (hubs of 6,145-12,288 entries, R-MAT s20 at eps 0.2: 3.66 ms, on the bitmap kernel
     // 0.9).
     if (d->nhub) {
-        const size_t smem = (kHotBits / 32 + kTailSlots) * sizeof(uint32_t);
-        if (!g_attr_bitmap[d->device][g][kPick]) {
-            SCAN_CUDA(cudaFuncSetAttribute(k_cn_bitmap<kPerGraph, kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-            g_attr_bitmap[d->device][g][kPick] = true;
-        }
         const uint64_t grid = std::min<uint64_t>(items(d->nhub), (uint64_t)d->num_sms);
-        k_cn_bitmap<kPerGraph, kPick><<<(unsigned)grid, kBitmapThreads, smem, sh>>>(
-            d->hubs, d->nhub, d->task_queue + 3, d->off, d->radj, d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp,
-            pr.on, pick_hub);
+        auto launch_hubs = [&](auto tails) -> scan_status {
+            constexpr bool kTails = decltype(tails)::value;
+            const size_t smem = bitmap_smem(kTails);
+            bool& set = g_attr_bitmap[d->device][g][kPick][kTails];
+            if (!set)
+                SCAN_CUDA(cudaFuncSetAttribute(k_cn_bitmap<kPerGraph, kPick, kTails>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            set = true;
+            k_cn_bitmap<kPerGraph, kPick, kTails><<<(unsigned)grid, kBitmapThreads, smem, sh>>>(
+                d->hubs, d->nhub, d->task_queue + 3, d->off, d->radj, d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp,
+                pr.on, pick_hub);
+            return SCAN_OK;
+        };
+        SCAN_TRY(d->tails ? launch_hubs(std::true_type()) : launch_hubs(std::false_type()));
         ++*launches;
     }
     for (int c = kNumBigClasses - 1; c >= 0; --c) {   // longest tasks first
