@@ -112,6 +112,7 @@ struct DeviceGraph {
     uint32_t* pend_edges = nullptr;    // E: those edges, gathered per task (cn's memory unless pivots are split)
     scan::TaskSlice* pend_lists = nullptr;   // slices of those tasks (one array, the task lists' order), ...
     uint32_t* pend_counts = nullptr;   // ... their number per list, and the filter's queue counter
+    unsigned long long* pend_votes = nullptr;   // k_cn_big: words read per class, and of lists that reached their threshold
     uint32_t cap_pend = 0;
     scan::LongEdges long_edges{};
     uint32_t* cn = nullptr;        // E: common-neighbour counts (the serving cache)

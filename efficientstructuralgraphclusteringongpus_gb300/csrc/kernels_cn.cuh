@@ -54,8 +54,15 @@ __host__ __device__ constexpr size_t bitmap_smem(bool tails) {
 constexpr uint32_t kBitmapMinDeg = kChunkMax;
 constexpr int kBitmapThreads = 1024;
 __host__ __device__ constexpr uint32_t big_class_entries(int c) { return c == 0 ? 1024u : c == 1 ? 4096u : kChunkMax; }
-__host__ __device__ constexpr uint32_t big_class_slots(int c) { return 4u * big_class_entries(c); }   // load <= 1/4
-                                                                                                   // (class 2: <= 1/2)
+// Table slots of a class: load at most 1/4, 1/2 for chunks of kChunkMaxCap; with a bitmap behind it
+// (k_cn_big, kBoundOpen) 3/8 and 3/4 in the largest class, so that two CTAs fit on an SM.
+__host__ __device__ constexpr uint32_t big_class_slots(int c, bool bound) {
+    return bound && c == 2 ? 16384u : 4u * big_class_entries(c);
+}
+__host__ __device__ constexpr uint32_t big_class_bits(int c) { return c == 0 ? 15u : c == 1 ? 17u : 18u; }   // log2
+__host__ __device__ constexpr size_t big_class_smem(int c, bool bound) {
+    return big_class_slots(c, bound) * sizeof(uint32_t) + (bound ? (size_t(1) << big_class_bits(c)) / 8 : 0);
+}
 
 struct CnTask {
     uint32_t v;      // pivot
@@ -213,6 +220,7 @@ struct TaskPick {
     const TaskSlice* order;
     const uint32_t* count;
     const uint32_t* edges;
+    unsigned long long* votes;   // k_cn_big, zeroed: words read, and those of lists that reached their threshold
 };
 
 // How a slice's edges are dealt to warps: batches small enough that every warp of the CTA has
@@ -339,6 +347,35 @@ __device__ __forceinline__ uint32_t probe_word(const uint4 x, uint32_t p, uint32
     if (p + 1 >= lb && p + 1 < le) c += bucket_has(tab, nb, x.y);
     if (p + 2 >= lb && p + 2 < le) c += bucket_has(tab, nb, x.z);
     if (p + 3 >= lb && p + 3 < le) c += bucket_has(tab, nb, x.w);
+    return c;
+}
+
+// Bit of entry w in a hashed bitmap of 2^log2bits bits.
+__device__ __forceinline__ uint32_t filter_bit(uint32_t w, uint32_t log2bits) {
+    return (w * 0x9E3779B1u) >> (32u - log2bits);
+}
+
+__device__ __forceinline__ uint32_t filter_probe_word(const uint4 x, uint32_t p, uint32_t lb, uint32_t le,
+                                                      const uint32_t* bits, uint32_t log2bits) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    uint32_t c = 0;
+#pragma unroll
+    if (p >= lb && p + 4u <= le) {            // the whole word lies in the list
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t x32 = w[i] * 0x9E3779B1u;
+            const uint32_t word = bits[x32 >> (37u - log2bits)];
+            c += __funnelshift_r(word, word, x32 >> (32u - log2bits)) & 1u;
+        }
+        return c;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t x32 = w[i] * 0x9E3779B1u;
+        const uint32_t word = bits[x32 >> (37u - log2bits)];
+        const uint32_t b = __funnelshift_r(word, word, x32 >> (32u - log2bits)) & 1u;
+        c += (p + i >= lb && p + i < le) ? b : 0u;
+    }
     return c;
 }
 
@@ -615,20 +652,40 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* queue, uint32_t prev, bo
     return *slot;
 }
 
-// kPick: a one-shot run after the sketches (pick given); full counts keep the plain form.  The
-// edges the sketches leave open are similar or close to it, so they are counted exactly at
-// once; k_cn_filter_classes' bound and then its recount by binary search took longer (whole
-// runs at eps 0.3: R-MAT of 16,384 vertices 553 -> 369 us, of 65,536 536 -> 405).  fp.sim null:
-// plans with split pivots, counts only.
-template <bool kPerGraph, bool kPick>
-__global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32_t* queue,
-                         const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                         const uint32_t* __restrict__ lo_adj, uint32_t* __restrict__ cn, uint32_t long_words,
-                         CnPrune pr, unsigned long long* __restrict__ ctr, uint32_t* __restrict__ miss,
-                         uint32_t nmiss, uint32_t stride, FusedPred fp, TaskPick pick) {
+// What k_cn_big counts: every edge of its tasks, or in a one-shot run after the sketches (pick given)
+// the edges they leave open, each exactly at once or by a bound first.  fp.sim null: plans with split
+// pivots, counts only.
+//
+// Exactly at once where open edges are mostly similar or close to it, as they are unless eps is low:
+// a bound decides few and comes on top (whole runs at eps 0.3 with k_cn_filter_classes here, whose
+// recounts are binary searches: R-MAT of 16,384 vertices 553 us, by this kernel 369; of 65,536 536 and
+// 405).  By a bound first, a hashed bitmap of the table's entries as in k_cn_filter_classes, where most
+// are rejected: its probe is a 4-byte shared load where the table's is one of 16 (R-MAT s21 at eps 0.15
+// 20.4 -> 16.4 ms, random graph of 50K vertices and 5M edges at eps 0.05 2.24 -> 1.86).  Only counting
+// tells them apart, so the second form is launched behind the first with the same queue, and the CTAs
+// of the first leave it the rest once less than 1 / kBoundShare of the words they read were of lists
+// that reached their threshold (of kBoundLeast words at least).  As two forms of one loop the exact one
+// took 20% longer (cliques of 800 vertices 7.4 -> 8.8 ms).
+enum CountForm { kCountAll, kCountOpen, kBoundOpen };
+constexpr uint64_t kBoundShare = 2, kBoundLeast = 1u << 18;
+// Fewer edges do without the second launch (2-3 us per class).
+constexpr uint64_t kBoundEdges = 1u << 22;
+
+// Two CTAs of 512 threads per SM: unbounded, the open forms took 66 registers, and one fitted (R-MAT
+// s21 at eps 0.1, whole run: 43.7 -> 31.9 ms, s18 at 0.15 3.4 -> 2.7).
+template <bool kPerGraph, CountForm kForm>
+__global__ void __launch_bounds__(512, 2)
+k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32_t* queue,
+         const uint32_t* __restrict__ off, const uint32_t* __restrict__ adj, const uint32_t* __restrict__ lo_adj,
+         uint32_t* __restrict__ cn, uint32_t long_words, CnPrune pr, unsigned long long* __restrict__ ctr,
+         uint32_t* __restrict__ miss, uint32_t nmiss, uint32_t stride, FusedPred fp, TaskPick pick, uint32_t log2bits) {
+    constexpr bool kPick = kForm != kCountAll, kBound = kForm == kBoundOpen;
     if constexpr (kPick) ntasks = *pick.count;
     extern __shared__ __align__(16) uint32_t tab[];
+    uint32_t* bits = tab + cap;                          // kBound: the bitmap
     __shared__ uint32_t next_batch, task_slot;
+    __shared__ uint32_t seen, passed, leave;             // of a task: words read, of lists that reached their threshold
+    uint32_t w_seen = 0, w_passed = 0;
     __shared__ CtaTotals totals;
     totals_clear(&totals);
     const uint32_t lane = threadIdx.x & 31;
@@ -646,9 +703,22 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
         const CnTask tk = tasks[slice.task];
         for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x)
             reinterpret_cast<uint4*>(tab)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
-        if (threadIdx.x == 0) next_batch = 0;
+        if constexpr (kBound)
+            for (uint32_t i = threadIdx.x; i < (1u << log2bits) / 128; i += blockDim.x)
+                reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
+        if (threadIdx.x == 0) {
+            next_batch = 0;
+            if (kForm == kCountOpen) seen = passed = 0;
+        }
         __syncthreads();
-        for (uint32_t j = tk.cb + threadIdx.x; j < tk.ce; j += blockDim.x) bucket_insert(tab, nb, adj[j]);
+        for (uint32_t j = tk.cb + threadIdx.x; j < tk.ce; j += blockDim.x) {
+            const uint32_t w = adj[j];
+            bucket_insert(tab, nb, w);
+            if constexpr (kBound) {
+                const uint32_t bit = filter_bit(w, log2bits);
+                atomicOr(&bits[bit >> 5], 1u << (bit & 31u));
+            }
+        }
         __syncthreads();
         const uint32_t vb = off[tk.v], ve = off[tk.v + 1];
         CnPrune Pg;
@@ -701,11 +771,27 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                     }
                 }
             }
-            uint32_t words = 0;
-            const uint32_t cnt = count_batch<kWordsInFlight>(adj, lane, ub, ue, tlo, long_words, words,
-                                                             [&](uint4 x, uint32_t p, uint32_t lb, uint32_t le) {
-                                                                 return probe_word(x, p, lb, le, tab, nb);
-                                                             });
+            uint32_t words = 0, cnt = 0;
+            bool exact = true;                                  // false: decided by the bound, cnt is that
+            auto look_up = [&](uint4 x, uint32_t p, uint32_t lb, uint32_t le) { return probe_word(x, p, lb, le, tab, nb); };
+            if constexpr (kBound) {
+                cnt = count_batch<kWordsInFlight>(adj, lane, ub, tlo ? ue : ub, tlo, long_words, words,
+                                                  [&](uint4 x, uint32_t p, uint32_t lb, uint32_t le) {
+                                                      return filter_probe_word(x, p, lb, le, bits, log2bits);
+                                                  });
+                exact = cnt >= tlo;
+                if (__any_sync(0xFFFFFFFFu, exact && ue > ub)) {
+                    const uint32_t c = count_batch<kWordsInFlight>(adj, lane, ub, exact ? ue : ub, exact ? tlo : 0u,
+                                                                   long_words, words, look_up);
+                    if (exact) cnt = c;
+                }
+            } else {
+                cnt = count_batch<kWordsInFlight>(adj, lane, ub, ue, tlo, long_words, words, look_up);
+            }
+            if constexpr (kForm == kCountOpen) {
+                w_seen += words;
+                if (cnt >= tlo) w_passed += (ue - ub + 3u) >> 2;
+            }
             const uint32_t nc = __popc(__ballot_sync(0xFFFFFFFFu, counted));
             if (lane == 0) totals_add(&totals, words, kPick ? 0u : nc);   // else k_sketch_filter counted them
             if (kPick && fp.sim) {                              // no split pivot
@@ -715,7 +801,7 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                 if (!tk.chunked) {
                     cn[k] = cnt;
                 } else {
-                    if (cnt) atomicAdd(&cn[k], cnt);            // cn was zeroed before the launch
+                    if (exact && cnt) atomicAdd(&cn[k], cnt);   // cn was zeroed before the launch
                     if (mi != 0xFFFFFFFFu && ue > ub) {
                         // below its threshold the chunk decided the edge (stopped early, or read
                         // in full with too few hits); otherwise it read all ue - ub entries
@@ -725,7 +811,25 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
                 }
             }
         }
+        if constexpr (kForm == kCountOpen) {
+            w_passed = __reduce_add_sync(0xFFFFFFFFu, w_passed);
+            if (lane == 0) {
+                atomicAdd(&seen, w_seen);
+                atomicAdd(&passed, w_passed);
+            }
+            w_seen = w_passed = 0;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                leave = 0;
+                if (pick.votes) {
+                    const unsigned long long all = atomicAdd(pick.votes, (unsigned long long)seen) + seen;
+                    const unsigned long long those = atomicAdd(pick.votes + 1, (unsigned long long)passed) + passed;
+                    leave = all >= kBoundLeast && kBoundShare * those < all;
+                }
+            }
+        }
         __syncthreads();
+        if (kForm == kCountOpen && leave) break;
     }
     if constexpr (kPick) fused_totals(fp, lane, nsim, ndis);
     totals_flush(&totals, ctr);
@@ -745,34 +849,6 @@ __global__ void k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint
 // the bucketed table of k_cn_big.  The bit is taken with a wrapping funnel shift (its shift
 // count uses the low five bits), and a word wholly inside the list skips the bound tests
 // (R-MAT s22: both together 17.5 -> 16.6 ms over the stage).
-__device__ __forceinline__ uint32_t filter_bit(uint32_t w, uint32_t log2bits) {
-    return (w * 0x9E3779B1u) >> (32u - log2bits);
-}
-
-__device__ __forceinline__ uint32_t filter_probe_word(const uint4 x, uint32_t p, uint32_t lb, uint32_t le,
-                                                      const uint32_t* bits, uint32_t log2bits) {
-    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-    uint32_t c = 0;
-#pragma unroll
-    if (p >= lb && p + 4u <= le) {            // the whole word lies in the list
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t x32 = w[i] * 0x9E3779B1u;
-            const uint32_t word = bits[x32 >> (37u - log2bits)];
-            c += __funnelshift_r(word, word, x32 >> (32u - log2bits)) & 1u;
-        }
-        return c;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t x32 = w[i] * 0x9E3779B1u;
-        const uint32_t word = bits[x32 >> (37u - log2bits)];
-        const uint32_t b = __funnelshift_r(word, word, x32 >> (32u - log2bits)) & 1u;
-        c += (p + i >= lb && p + i < le) ? b : 0u;
-    }
-    return c;
-}
-
 // |adj[b, e) ∩ list[0, dv)|, list sorted ascending: warp-wide, the result in every lane.
 __device__ __forceinline__ uint32_t sorted_count(const uint32_t* list, uint32_t dv, const uint32_t* __restrict__ adj,
                                                  uint32_t b, uint32_t e, uint32_t lane) {

@@ -486,7 +486,7 @@ constexpr uint64_t kSketchSmallEdges = 1u << 19;
 constexpr int kPendCounts = kPendingLists + 2;
 // Counters of one kind share 256 bytes, different kinds do not: with the totals and the task
 // queues in one line their atomics waited for one another (k_cn_small 0.105 -> 0.155 ms).
-constexpr int kCounterSpan = 64, kStageCounters = 3 * kCounterSpan;
+constexpr int kCounterSpan = 64, kStageCounters = 4 * kCounterSpan;
 
 // The bitmaps of the larger vertices (lists from k_sketch_assign): the hubs on stream sh, the
 // others on sm.
@@ -582,12 +582,13 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     };
     // Counters of the similarity stage, cleared together: list words, edges counted and pending
     // work (64 bits each), the kernels' task queues, the pending lists.
-    static_assert(2 * kCounterSpan + kPendCounts <= kStageCounters, "similarity-stage counters");
+    static_assert(kPendCounts <= kCounterSpan && 4 * kPendingLists <= kCounterSpan, "similarity-stage counters");
     uint32_t* stage = nullptr;
     SCAN_TRY(dalloc(d.get(), &stage, kStageCounters));
     d->cn_ctr = reinterpret_cast<unsigned long long*>(stage);
     d->task_queue = stage + kCounterSpan;
     d->pend_counts = stage + 2 * kCounterSpan;
+    d->pend_votes = reinterpret_cast<unsigned long long*>(stage + 3 * kCounterSpan);
     // The offsets are checked first (every later kernel indexes lists by them), with the
     // degree histogram of the hot-id assignment; both need only the offsets, so the host
     // waits for those alone.
@@ -826,10 +827,9 @@ scan_status device_upload(int device, uint64_t n, uint64_t m, const void* off_ho
 
 // Kernel attributes and occupancies, found once per device (so capturing launch_cn into a
 // CUDA graph queries nothing).  [g] is 1 for the instantiations with per-graph parameters.
-static bool g_attr_set[64][2][2] = {};      // k_cn_big, [g][after the sketches]
 static bool g_attr_bitmap[64][2][2][2] = {};   // [g][after the sketches][with tails]
 static bool g_attr_filter[64][2] = {};      // k_cn_filter_classes, [g]
-static int g_per_sm[64][2][2][kNumBigClasses] = {};         // k_cn_big, [g][after the sketches][hash class]
+static int g_per_sm[64][2][3][kNumBigClasses] = {};         // k_cn_big, [g][CountForm][hash class]
 static int g_per_sm_sketch[64][2] = {};                      // k_sketch_filter
 static int g_per_sm_filter[64][2][kNumBigClasses][2] = {};  // k_cn_filter_classes, [g][class][largest class at
                                                             // the default chunk, or at the cap]
@@ -898,7 +898,8 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
             pl.tasks[a] = tasks;
             pl.count[a] = count;
             pl.out[a] = out;
-            const TaskPick pick{out, d->pend_counts + a, d->pend_edges};
+            const TaskPick pick{out, d->pend_counts + a, d->pend_edges,
+                                d->E >= kBoundEdges ? d->pend_votes + 2 * a : nullptr};
             if (count) out += count + kPendingSlices * d->num_sms;
             longest = std::max(longest, count);
             return pick;
@@ -913,11 +914,6 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
         }
     }
     SCAN_CUDA(cudaEventRecord(d->ev[7], s));
-    if (!g_attr_set[d->device][g][kPick]) {
-        SCAN_CUDA(cudaFuncSetAttribute(k_cn_big<kPerGraph, kPick>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(big_class_slots(kNumBigClasses - 1) * sizeof(uint32_t))));
-        g_attr_set[d->device][g][kPick] = true;
-    }
     // One-shot fused runs without sketches (every pivot unsplit) decide most edges from an upper
     // bound on their count (k_cn_filter_classes); the others use the bucketed table.
     const bool filter = fp.sim != nullptr && !kPick;
@@ -979,20 +975,36 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
                     d->big[c], d->nbig[c], entries, d->task_queue + c, d->off, d->adj,
                     d->lo_adj, d->cn, d->long_words, pr, d->cn_ctr, fp);
             } else {
-                const size_t smem = big_class_slots(c) * sizeof(uint32_t);
-                int& per_sm = g_per_sm[d->device][g][kPick][c];
-                if (per_sm == 0) {
-                    SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_big<kPerGraph, kPick>, threads, smem));
-                    per_sm = std::max(per_sm, 1);
+                auto launch_big = [&](auto form) -> scan_status {
+                    constexpr CountForm kForm = decltype(form)::value;
+                    constexpr bool kBound = kForm == kBoundOpen;
+                    auto* kernel = k_cn_big<kPerGraph, kForm>;
+                    const size_t smem = big_class_smem(c, kBound);
+                    int& per_sm = g_per_sm[d->device][g][kForm][c];
+                    if (per_sm == 0) {
+                        SCAN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)big_class_smem(kNumBigClasses - 1, kBound)));
+                        int fit = 0;
+                        SCAN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem));
+                        per_sm = std::max(fit, 1);
+                    }
+                    const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
+                    kernel<<<(unsigned)grid, threads, smem, s>>>(
+                        d->big[c], d->nbig[c], big_class_slots(c, kBound), d->task_queue + c, d->off, d->adj, d->lo_adj,
+                        d->cn, d->long_words, pr, d->cn_ctr, pr.on ? d->miss : nullptr, d->nmiss,
+                        !pr.on || !d->nmiss ? 0u : fp.pend ? kSpreadPrime : spread_stride(d->nbig[c]), fp, pick_class[c],
+                        big_class_bits(c));
+                    return SCAN_OK;
+                };
+                if constexpr (kPick) {
+                    SCAN_TRY(launch_big(std::integral_constant<CountForm, kCountOpen>()));
+                    if (d->E >= kBoundEdges) {
+                        SCAN_TRY(launch_big(std::integral_constant<CountForm, kBoundOpen>()));
+                        ++*launches;
+                    }
+                } else {
+                    SCAN_TRY(launch_big(std::integral_constant<CountForm, kCountAll>()));
                 }
-                const uint64_t grid = std::min<uint64_t>(items(d->nbig[c]), (uint64_t)d->num_sms * per_sm);
-                k_cn_big<kPerGraph, kPick><<<(unsigned)grid, threads, smem, s>>>(d->big[c], d->nbig[c], big_class_slots(c),
-                                                                d->task_queue + c, d->off,
-                                                                d->adj, d->lo_adj, d->cn, d->long_words, pr,
-                                                                d->cn_ctr, pr.on ? d->miss : nullptr, d->nmiss,
-                                                                !pr.on || !d->nmiss ? 0u
-                                                                : fp.pend ? kSpreadPrime : spread_stride(d->nbig[c]),
-                                                                fp, pick_class[c]);
             }
             ++*launches;
         }
