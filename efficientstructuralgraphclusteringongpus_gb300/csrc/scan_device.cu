@@ -1046,16 +1046,18 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     return SCAN_OK;
 }
 
-// Below this eps the sketches of a graph of kSketchLowEdges edges leave most of its edges open,
-// and the list kernels that bound a count first (k_cn_filter_classes) are the faster ones for so
-// many.  Whole runs in ms, by sketches / by lists alone: power law of 57M edges, eps 0.1 49 / 37,
-// 0.12 45 / 36, 0.15 31 / 34; R-MAT s22 (64M) 0.1 92 / 51, 0.15 47 / 45, 0.2 16 / 39; s23 0.1
-// 248 / 174, 0.2 47 / 132.  On smaller graphs the sketches win at most eps (R-MAT s18 0.05 4.4 /
-// 9.9, 0.1 4.4 / 9.0; s20 18 / 28, 19 / 19; s21 24 / 37, 25 / 17).
+// Below this eps the sketches leave most edges of a large graph open, and where hubs have tails the
+// list kernels that bound a count first (k_cn_filter_classes) are the faster ones for so many.  Whole
+// runs in ms, by sketches / by lists alone: R-MAT s22 (64M edges) eps 0.1 63 / 45, 0.12 54 / 42, 0.15
+// 39 / 40; power law of 57M 0.1 40 / 35, 0.12 38 / 34, 0.15 27 / 32.  Without tails the sketches win
+// at any eps (R-MAT of 2^20 vertices and 51M edges 0.05 100 / 208, 0.1 106 / 166; s20 of 16M 0.1 14 /
+// 18), and on smaller graphs what the lists win is less (s21 of 32M 0.1 32 / 37, 0.15 16.2 / 15.2).
+// Streamed graphs, whose pivots are split, count as with tails.  Batches always take the sketches.
 constexpr double kSketchLowEps = 0.15;
 constexpr uint64_t kSketchLowEdges = 1u << 25;
 static bool with_sketches(const DeviceGraph* d, const PredParams& p) {
-    return d->sk && (p.eps >= kSketchLowEps || d->E < kSketchLowEdges);
+    const bool tails = !d->radj || d->tails;
+    return d->sk && (p.eps >= kSketchLowEps || d->E < kSketchLowEdges || !tails);
 }
 
 // cn for every edge (the similarity stage); events 7..12 bracket its kernels.
