@@ -111,6 +111,8 @@ _SIGS = {
     "scan_graph_release_device": (C.c_int, [_vp]),
     "scan_graph_upload_streamed": (C.c_int, [_vp, C.c_int, C.c_uint64, _u64p]),
     "scan_graph_device_bytes": (C.c_uint64, [_vp]),
+    "scan_graph_bitmap_bytes": (C.c_uint64, [_vp]),
+    "scan_graph_release_bitmaps": (C.c_int, [_vp]),
     "scan_release_cached_memory": (None, []),
     "scan_set_cached_memory_limit": (None, [C.c_uint64]),
     "scan_cached_memory_bytes": (C.c_uint64, [C.c_int]),
@@ -346,6 +348,15 @@ class Graph:
     @property
     def device_bytes(self) -> int:
         return load_library().scan_graph_device_bytes(self._h)
+
+    @property
+    def bitmap_bytes(self) -> int:
+        """Device bytes of the neighbourhood bitmaps of one-shot runs (0: none)."""
+        return load_library().scan_graph_bitmap_bytes(self._h)
+
+    def release_bitmaps(self) -> None:
+        """Give the bitmaps' device memory back; runs go by lists alone, with the same results."""
+        _check(load_library().scan_graph_release_bitmaps(self._h))
 
     def release_device(self) -> None:
         _check(load_library().scan_graph_release_device(self._h))

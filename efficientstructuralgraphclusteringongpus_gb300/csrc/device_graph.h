@@ -107,6 +107,7 @@ struct DeviceGraph {
     // neighbourhood sketches (kernels_sketch.cuh; null when off)
     uint2* sk_info = nullptr;          // n: rank, degree
     uint4* sk = nullptr;               // the bitmaps
+    uint64_t sk_units = 0;             // their 16-byte units
     scan::SketchLevels sk_levels{};
     uint32_t* pend_pivot = nullptr;    // n: one-shot runs, list work of the edges the sketches leave open
     uint32_t* pend_edges = nullptr;    // E: those edges, gathered per task (cn's memory unless pivots are split)

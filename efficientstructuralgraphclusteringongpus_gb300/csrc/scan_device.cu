@@ -314,6 +314,44 @@ static scan_status dalloc(DeviceGraph* d, T** p, uint64_t count) {
     return SCAN_OK;
 }
 
+// Give an array of `count` back to the cache before the graph is freed: no work on it may be in flight.
+template <typename T>
+static void dfree(DeviceGraph* d, T** p, uint64_t count) {
+    auto it = std::find_if(d->allocs.begin(), d->allocs.end(), [&](const auto& a) { return a.first == *p; });
+    if (it != d->allocs.end()) {
+        cache_give(d->device, it->first, it->second);
+        d->allocs.erase(it);
+        d->device_bytes -= block_bytes(count, sizeof(T));
+    }
+    *p = nullptr;
+}
+
+// The bitmaps and what the runs that use them need; runs then go by lists alone.
+static void release_sketches(DeviceGraph* d) {
+    for (cudaStream_t st : {d->stream, d->aux, d->side}) cudaStreamSynchronize(st);
+    dfree(d, &d->sk, d->sk_units);
+    dfree(d, &d->sk_info, d->n);
+    dfree(d, &d->pend_pivot, d->n);
+    dfree(d, &d->long_edges.slot, d->long_edges.cap);
+    dfree(d, &d->long_edges.edge, d->long_edges.cap);
+    d->long_edges = LongEdges{};
+    if (d->pend_edges != d->cn) dfree(d, &d->pend_edges, d->E);
+    d->pend_edges = nullptr;
+    dfree(d, &d->pend_lists, d->cap_pend);
+    d->cap_pend = 0;
+    d->sk_units = 0;
+}
+
+// f(), and once more without the bitmaps where it finds no memory with them.
+template <typename F>
+static scan_status with_room(DeviceGraph* d, F f) {
+    const scan_status st = f();
+    if (st != SCAN_ERR_OUT_OF_MEMORY || !d->sk) return st;
+    release_sketches(d);
+    clear_error();
+    return f();
+}
+
 // Device memory for the length of a call, back to the cache at the end of its scope: no work on
 // it may be in flight then.
 class CallBuffers {
@@ -664,8 +702,9 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
                 SCAN_TRY(dalloc(d.get(), &ll.slot, ll.cap));
                 SCAN_TRY(dalloc(d.get(), &ll.edge, ll.cap));
             }
-            SCAN_TRY(dalloc(d.get(), &sk_mid, sk_plan.list_mid));
-            SCAN_TRY(dalloc(d.get(), &sk_hub, sk_plan.list_hub));
+            SCAN_TRY(tmp.get(&sk_mid, sk_plan.list_mid));
+            SCAN_TRY(tmp.get(&sk_hub, sk_plan.list_hub));
+            d->sk_units = sk_units;
         }
     }
     uint32_t min_bin = 1;                            // isolated vertices are never hot
@@ -1494,6 +1533,26 @@ scan_status scan_graph_upload_streamed(scan_graph* g, int device, uint64_t devic
 
 uint64_t scan_graph_device_bytes(const scan_graph* g) { return g && g->dev ? g->dev->device_bytes : 0; }
 
+uint64_t scan_graph_bitmap_bytes(const scan_graph* g) {
+    const DeviceGraph* d = g ? g->dev : nullptr;
+    if (!d || !d->sk) return 0;
+    return block_bytes(d->sk_units, sizeof(uint4)) + block_bytes(d->n, sizeof(uint2)) + block_bytes(d->n, sizeof(uint32_t)) +
+           (d->long_edges.cap ? block_bytes(d->long_edges.cap, sizeof(uint4)) + block_bytes(d->long_edges.cap, sizeof(uint32_t)) : 0) +
+           (d->cap_pend ? block_bytes(d->cap_pend, sizeof(TaskSlice)) : 0) +
+           (d->pend_edges != d->cn ? block_bytes(d->E, sizeof(uint32_t)) : 0);
+}
+
+scan_status scan_graph_release_bitmaps(scan_graph* g) {
+    clear_error();
+    if (!g) return fail(SCAN_ERR_INVALID_ARG, "graph is null");
+    if (!g->dev) return SCAN_OK;
+    DeviceGraph* d = g->dev;
+    std::lock_guard<std::mutex> lock(d->mu);
+    SCAN_CUDA(cudaSetDevice(d->device));
+    if (d->sk) release_sketches(d);
+    return SCAN_OK;
+}
+
 scan_status scan_graph_release_device(scan_graph* g) {
     clear_error();
     if (!g) return fail(SCAN_ERR_INVALID_ARG, "graph is null");
@@ -1558,7 +1617,7 @@ scan_status scan_graph_set_plan(scan_graph* g, int device, uint32_t small_deg, u
     pp.small_strategy = small_strategy;
     pp.bitmap_min_deg = hub_min_deg;
     pp.chunk_max = chunk_max;
-    SCAN_TRY(plan_tasks(d, pp));
+    SCAN_TRY(with_room(d, [&] { return plan_tasks(d, pp); }));
     d->cn_valid = false;
     return SCAN_OK;
 }
@@ -1573,7 +1632,7 @@ scan_status scan_common_neighbors(scan_graph* g, int device, uint32_t* out_cn, s
     SCAN_CUDA(cudaSetDevice(d->device));
     uint32_t launches = 0;
     d->cn_valid = false;
-    SCAN_TRY(full_counts(d, &launches, out_cn));
+    SCAN_TRY(with_room(d, [&] { return full_counts(d, &launches, out_cn); }));
     d->cn_valid = true;
     if (stats) {
         stats->n = d->n;
@@ -1599,8 +1658,9 @@ scan_status scan_memberships(scan_graph* g, int device, const char* eps_decimal,
     std::lock_guard<std::mutex> lock(d->mu);
     cudaStream_t s = d->stream;
     // Border pairs: count, then collect.
-    unsigned long long* cnt = nullptr;
-    SCAN_CUDA(cudaMallocAsync(&cnt, sizeof(unsigned long long), s));
+    CallBuffers mem(d->device);
+    unsigned long long *cnt = nullptr, *buf = nullptr;
+    SCAN_TRY(with_room(d, [&] { return mem.get(&cnt, 1); }));
     SCAN_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s));
     k_border_pairs<<<grid_for(d, d->E, 256), 256, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->rs.sim, d->rs.parent, cnt,
                                                           nullptr, 0);
@@ -1609,16 +1669,14 @@ scan_status scan_memberships(scan_graph* g, int device, const char* eps_decimal,
     SCAN_CUDA(cudaStreamSynchronize(s));
     std::vector<unsigned long long> keys(nb);
     if (nb) {
-        unsigned long long* buf = nullptr;
-        SCAN_CUDA(cudaMallocAsync(&buf, nb * sizeof(unsigned long long), s));
+        SCAN_TRY(with_room(d, [&] { return mem.get(&buf, nb); }));
         SCAN_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s));
         k_border_pairs<<<grid_for(d, d->E, 256), 256, 0, s>>>(d->E, d->lo_adj, d->lo_src, d->rs.sim, d->rs.parent, cnt,
                                                               buf, nb);
-        SCAN_CUDA(cudaMemcpyAsync(keys.data(), buf, nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-        SCAN_CUDA(cudaFreeAsync(buf, s));
+        cudaMemcpyAsync(keys.data(), buf, nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+        SCAN_CUDA(cudaStreamSynchronize(s));                  // before the buffers go back
+        SCAN_CUDA(cudaGetLastError());
     }
-    SCAN_CUDA(cudaFreeAsync(cnt, s));
-    SCAN_CUDA(cudaStreamSynchronize(s));
     // Output formatting: add the cores, order by (cluster, vertex), drop repeats.
     for (uint32_t v = 0; v < d->n; ++v)
         if (role[v] == SCAN_ROLE_CORE) keys.push_back(((unsigned long long)(uint32_t)label[v] << 32) | v);

@@ -140,6 +140,12 @@ scan_status scan_graph_upload_streamed(scan_graph* g, int device, uint64_t devic
                                        uint64_t* device_bytes_used);
 /* Device memory held by the graph's resident copy (0 if none). */
 uint64_t scan_graph_device_bytes(const scan_graph* g);
+/* Of that, what the neighbourhood bitmaps of one-shot runs take (0 if the graph has none); they add a
+ * third to a half to a resident graph.  scan_graph_release_bitmaps gives it back: runs then go by
+ * neighbour lists alone, with the same results.  A call that finds no memory does so by itself before
+ * it fails. */
+uint64_t scan_graph_bitmap_bytes(const scan_graph* g);
+scan_status scan_graph_release_bitmaps(scan_graph* g);
 /* Drop the device copy (the host copy stays). */
 scan_status scan_graph_release_device(scan_graph* g);
 /* Device buffers of freed graphs (and of each drop-in GPUScan() call) are kept per device,
