@@ -103,6 +103,7 @@ struct DeviceGraph {
     uint32_t nhub = 0;
     uint32_t cap_small = 0, cap_big[scan::kNumBigClasses] = {}, cap_hubs = 0;   // task array capacities
     scan::PlanParams plan{};
+    bool planned = false;          // the task arrays are those of plan
     uint32_t long_words = 32;      // lists of >= long_words 16-byte words get a whole warp
     // neighbourhood sketches (kernels_sketch.cuh; null when off)
     uint2* sk_info = nullptr;          // n: rank, degree

@@ -468,6 +468,7 @@ static scan_status device_scan(DeviceGraph* d, const uint32_t* cnt, uint64_t n, 
 // re-plans with other task sizes).  Needs the orientation (lo_off, work, tailc).
 scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
     cudaStream_t s = d->stream;
+    d->planned = false;   // a plan that fails halfway fits neither these parameters nor the ones before
     uint32_t* counts = d->dflags + 1;
     const unsigned pg = (unsigned)((d->n + 255) / 256);
     SCAN_CUDA(cudaMemsetAsync(counts, 0, (4 + kNumBigClasses) * sizeof(uint32_t), s));
@@ -510,6 +511,7 @@ scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp) {
                               d->big[1], d->big[2], d->hubs);
     SCAN_CUDA(cudaGetLastError());
     d->plan = pp;
+    d->planned = true;
     return SCAN_OK;
 }
 
@@ -1103,6 +1105,7 @@ static bool with_sketches(const DeviceGraph* d, const PredParams& p) {
 scan_status launch_cn(DeviceGraph* d, uint32_t* launches, const PredParams* prune, const RunScratch* run,
                       const BatchParams* bp) {
     if (d->device < 0 || d->device >= 64) return fail(SCAN_ERR_INVALID_ARG, "device index must be < 64");
+    if (!d->planned) SCAN_TRY(with_room(d, [&] { return plan_tasks(d, d->plan); }));
     CnPrune pr{0.0, 0, 1, 0u, 0, nullptr, nullptr, 0.0, 0.f, nullptr};
     if (prune) pr = CnPrune{prune->eps, prune->p, prune->q, 1u, prune->mode, nullptr, nullptr, prune->pq2,
                             prune->eps2_floor, nullptr};

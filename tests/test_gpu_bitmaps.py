@@ -64,6 +64,22 @@ def test_a_new_plan_takes_the_room_of_the_bitmaps(rmat):
     g.release_device()
 
 
+def test_a_plan_that_finds_no_room_leaves_the_graph_usable(rmat):
+    g, cn = rmat
+    g.upload()
+    g.release_bitmaps()
+    sg.release_cached_memory()
+    before = g.plan()
+    sg.set_device_memory_left(0)
+    with pytest.raises(sg.ScanError) as e:
+        g.set_plan(1, sg.SMALL_SERIAL, 1 << 30, 6144)
+    assert e.value.status == 5
+    sg.set_device_memory_left(None)
+    check(g, cn)
+    assert g.plan() == before
+    g.release_device()
+
+
 def test_memberships_take_the_room_of_the_bitmaps(rmat):
     g, cn = rmat
     want = g.memberships("0.2", 2)
