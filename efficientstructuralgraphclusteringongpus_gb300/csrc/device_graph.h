@@ -125,6 +125,7 @@ struct DeviceGraph {
     uint32_t* dflags = nullptr;    // [0] input checks, [1..8] planner counters, [16] long lists
     std::vector<std::pair<void*, size_t>> allocs;   // (pointer, bytes), returned to the cache on free
     uint64_t device_bytes = 0;     // device memory held by this graph
+    uint64_t budget = 0;           // streamed mode: device memory the caller allows (0: no limit)
     char* h_res = nullptr;         // pinned, kResStage bytes: results of small graphs, else counters and flags
     uint32_t* adj_host = nullptr;  // streamed mode: pinned, GPU-mapped adjacency (adj points into it)
     cudaEvent_t ev[16] = {};       // 0-2 upload, 3-6 run stages, 7-12 and 15 similarity kernels

@@ -692,14 +692,22 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
             d->sk_levels.base[c] = (uint32_t)sk_units;
             sk_units += (((uint64_t)holders[c] << c) + 7) & ~7ull;
         }
-        if (sk_units && sk_units < 0xFFFFFFF0ull && (!sketch_budget || sk_units * 16 + 13 * n <= sketch_budget)) {
+        uint32_t long_cap = 0;
+        for (int c = kSketchGroupLog + 1 - kSketchMinLog; c < kSketchClasses; ++c)
+            if (hcls[c]) long_cap = (uint32_t)std::max<uint64_t>(m / 32, 4096);
+        // What goes with the bitmaps: ranks and pending work by vertex, the long edges, and with
+        // split pivots (no hub tasks; some degree above the chunk, by its size class) the pending
+        // edges; their slices are few.
+        bool split = !bitmap_path;
+        split &= holders[sketch_log(kChunkMax + 1) - kSketchMinLog] > 0;
+        const uint64_t need = sk_units * 16 + 12 * n + 20ull * long_cap + (split ? 2 * m : 0) + m / 8 + (1u << 20);
+        if (sk_units && sk_units < 0xFFFFFFF0ull && (!sketch_budget || need <= sketch_budget)) {
             SCAN_TRY(dalloc(d.get(), &d->sk, sk_units));
             SCAN_TRY(dalloc(d.get(), &d->sk_info, n));
             SCAN_TRY(dalloc(d.get(), &d->pend_pivot, n));   // 4 bytes a vertex
             LongEdges& ll = d->long_edges;
             ll.count = d->pend_counts + kPendCounts - 1;
-            for (int c = kSketchGroupLog + 1 - kSketchMinLog; c < kSketchClasses; ++c)
-                if (hcls[c]) ll.cap = (uint32_t)std::max<uint64_t>(m / 32, 4096);
+            ll.cap = long_cap;
             if (ll.cap) {   // a sixteenth of the edges; what finds no room has a slower path
                 SCAN_TRY(dalloc(d.get(), &ll.slot, ll.cap));
                 SCAN_TRY(dalloc(d.get(), &ll.edge, ll.cap));
@@ -1324,6 +1332,10 @@ static scan_status full_counts_by_triangles(DeviceGraph* d, uint32_t* launches, 
     uint32_t *hi_adj = nullptr, *cnt = nullptr, *small = nullptr, *ctr = nullptr;
     uint2* big = nullptr;
     const uint64_t slices = E / kTriSliceEdges + d->m / kSmallDeg + 1;   // at most one short slice per larger pivot
+    const uint64_t need = block_bytes(E + kAdjPad, 4) + block_bytes(E, 4) + block_bytes(std::min<uint64_t>(d->n, E), 4) +
+                          block_bytes(slices, sizeof(uint2));
+    if (d->budget && d->device_bytes + need > d->budget)
+        return fail(SCAN_ERR_OUT_OF_MEMORY, "full counts by triangles: above the graph's device budget");
     scan_status st = mem.get(&hi_adj, E + kAdjPad);
     if (st == SCAN_OK) st = mem.get(&cnt, E);
     if (st == SCAN_OK) st = mem.get(&small, std::min<uint64_t>(d->n, E));
@@ -1517,12 +1529,8 @@ scan_status scan_graph_upload_streamed(scan_graph* g, int device, uint64_t devic
     const uint64_t spare = device_budget_bytes > est + g->m / 4 ? device_budget_bytes - est - g->m / 4 : kNoSketches;
     SCAN_TRY(device_upload(device, g->n, g->m, g->off.data(), true, g->adj.data(), &g->dev, nullptr, true,
                            device_budget_bytes ? spare : 0));
-    if (device_budget_bytes && g->dev->device_bytes > device_budget_bytes && g->dev->sk) {
-        device_graph_free(g->dev);
-        g->dev = nullptr;
-        SCAN_TRY(device_upload(device, g->n, g->m, g->off.data(), true, g->adj.data(), &g->dev, nullptr, true,
-                               kNoSketches));
-    }
+    g->dev->budget = device_budget_bytes;
+    if (device_budget_bytes && g->dev->device_bytes > device_budget_bytes && g->dev->sk) release_sketches(g->dev);
     if (device_bytes_used) *device_bytes_used = g->dev->device_bytes;
     if (device_budget_bytes && g->dev->device_bytes > device_budget_bytes) {
         const uint64_t used = g->dev->device_bytes;
