@@ -175,8 +175,7 @@ scan_status full_counts(DeviceGraph* d, uint32_t* launches, uint32_t* out_host);
 scan_status plan_tasks(DeviceGraph* d, const PlanParams& pp);
 // Time the similarity stage under plan settings (small-pivot strategy and degree cut, task
 // size, chunk, long-list threshold, hub threshold; a coordinate search) and keep the
-// fastest; returns its time in *best_ms.  stage (may be empty) queues the stage as the caller
-// runs it (launch_cn with full counts when empty).
+// fastest; returns its time in *best_ms.  stage queues the stage as the caller runs it.
 scan_status autotune_similarity(DeviceGraph* d, float* best_ms, const std::function<scan_status(uint32_t*)>& stage);
 // Per-graph parameters of a batched run (many graphs as one disjoint union): the graph of
 // each vertex and each graph's predicate parameters and mu (all device pointers).

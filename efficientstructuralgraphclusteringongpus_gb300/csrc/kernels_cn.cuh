@@ -359,7 +359,6 @@ __device__ __forceinline__ uint32_t filter_probe_word(const uint4 x, uint32_t p,
                                                       const uint32_t* bits, uint32_t log2bits) {
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
     uint32_t c = 0;
-#pragma unroll
     if (p >= lb && p + 4u <= le) {            // the whole word lies in the list
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

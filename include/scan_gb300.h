@@ -191,12 +191,13 @@ scan_status scan_run(scan_graph* g, int device, const char* eps_decimal, int mu,
                      scan_predicate predicate, int32_t* out_label, uint8_t* out_role,
                      scan_stats* stats);
 
-/* Autotune the similarity stage of the resident graph (uploading it first), timing full
- * counts: a coordinate search over the small-pivot intersection strategy (lists counted one
- * at a time through a hash table, a batch's lists streamed through it, or streamed with
- * binary search in the sorted list) and degree cut, the task size
- * and largest table chunk, the long-list threshold, and the degree above which pivots take
- * the hub path.  The fastest plan is kept for later runs.  Outputs may be NULL. */
+/* Autotune the similarity stage of the resident graph (uploading it first), timing that of
+ * scan_run at eps 0.5: a coordinate search over the small-pivot intersection strategy (lists
+ * counted one at a time through a hash table, a batch's lists streamed through it, or streamed
+ * with binary search in the sorted list; graphs with neighbourhood bitmaps have one form only)
+ * and degree cut, the task size and largest table chunk, the long-list threshold, and the degree
+ * above which pivots take the hub path.  The fastest plan is kept for later runs.  Outputs may be
+ * NULL. */
 scan_status scan_graph_autotune(scan_graph* g, int device, double* best_similarity_ms,
                                 uint32_t* long_words, uint64_t* target_probes);
 
