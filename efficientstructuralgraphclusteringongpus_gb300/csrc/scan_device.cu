@@ -625,6 +625,8 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     static_assert(kPendCounts <= kCounterSpan && 4 * kPendingLists <= kCounterSpan, "similarity-stage counters");
     uint32_t* stage = nullptr;
     SCAN_TRY(dalloc(d.get(), &stage, kStageCounters));
+    // (a served graph runs no similarity stage, but its queries' last pass reads the totals)
+    SCAN_CUDA(cudaMemsetAsync(stage, 0, kStageCounters * sizeof(uint32_t), s3));
     d->cn_ctr = reinterpret_cast<unsigned long long*>(stage);
     d->task_queue = stage + kCounterSpan;
     d->pend_counts = stage + 2 * kCounterSpan;
@@ -743,7 +745,7 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
     // come in between; the flags are read once, with the plan.  The bitmaps on s2 too made every
     // chunk's work longer than its copy (R-MAT s22: 1.56 ms left after the last copy, so 1.17).
     scan_status ost = SCAN_OK;
-    uint32_t orient_launches = 0;
+    uint32_t orient_launches = 0, sketch_launches = 0;
     auto enqueue = [&]() -> scan_status {
         // on s2, needing only the offsets (already on the device)
         SCAN_CUDA(cudaMemsetAsync(lowbits, 0, (m / 32 + 2) * sizeof(uint32_t), s2));
@@ -754,9 +756,11 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         if (bitmap_path)
             k_hot_assign<<<grid_for(d.get(), n, 256), 256, 0, s2>>>(d->n, d->off, min_bin, kHotBits, d->hot,
                                                                   hist + kDegBins);
-        if (d->sk)
+        if (d->sk) {
             k_sketch_assign<<<grid_for(d.get(), n, 256), 256, 0, s3>>>(d->n, d->off, sk_plan, sk_cls + kSketchClasses,
                                                                      d->sk_info, sk_mid, sk_hub);
+            sketch_launches = 1 + (sk_plan.list_mid > 0) + (sk_plan.list_hub > 0);
+        }
         if (adj_in_host_memory) {
             std::memcpy(d->adj_host, adj_host, m * sizeof(uint32_t));
             std::memset(d->adj_host + m, 0, kAdjPad * sizeof(uint32_t));
@@ -776,6 +780,7 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
                 SCAN_CUDA(cudaStreamWaitEvent(s3, ev_chunk[c], 0));
                 k_sketch_build_small<<<grid_for(d.get(), vcut[c + 1] - vcut[c], kSketchWarps * 32), kSketchWarps * 32, 0,
                                        s3>>>(vcut[c], vcut[c + 1], d->off, d->adj, d->sk_info, d->sk, d->sk_levels);
+                ++sketch_launches;
             }
         }
         SCAN_CUDA(cudaEventRecord(d->ev[1], s));   // end of the copies
@@ -853,9 +858,10 @@ static scan_status upload_once(int device, uint64_t n, uint64_t m, const void* o
         st->ms_h2d = ev_ms(d->ev[0], d->ev[1]);
         st->ms_orient = ev_ms(d->ev[1], d->ev[2]);
         // offsets check (+ conversion), tile map, orientation passes, count scan, word scan +
-        // fill, two planner passes; the bitmap path adds the degree histogram and hot ids
+        // fill, two planner passes; the bitmap path adds the degree histogram and hot ids, the
+        // sketches their size classes, ranks and bitmaps
         st->kernel_launches += 2 + (off64 ? 1 : 0) + (bitmap_path ? 2 : 0) + orient_launches + (n ? 3 : 0) +
-                               (fill_tiles ? 4 : 0) + 2;
+                               (fill_tiles ? 4 : 0) + 2 + (want_sketch ? 1 : 0) + sketch_launches;
     }
     *out = d.release();
     return SCAN_OK;
