@@ -667,8 +667,10 @@ __device__ __forceinline__ uint32_t next_task(uint32_t* queue, uint32_t prev, bo
 // took 20% longer (cliques of 800 vertices 7.4 -> 8.8 ms).
 enum CountForm { kCountAll, kCountOpen, kBoundOpen };
 constexpr uint64_t kBoundShare = 2, kBoundLeast = 1u << 18;
-// Fewer edges do without the second launch (2-3 us per class).
+// Fewer edges, and eps from which on the first form is left to finish nearly always, do without the
+// second launch (4 us per class: R-MAT of 400K vertices at eps 0.5 404 -> 416 us).
 constexpr uint64_t kBoundEdges = 1u << 22;
+constexpr double kBoundEps = 0.25;
 
 // Two CTAs of 512 threads per SM: unbounded, the open forms took 66 registers, and one fitted (R-MAT
 // s21 at eps 0.1, whole run: 43.7 -> 31.9 ms, s18 at 0.15 3.4 -> 2.7).

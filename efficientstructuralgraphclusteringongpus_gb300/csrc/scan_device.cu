@@ -943,6 +943,7 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
     // The sketches first: they settle most edges, and the list kernels below then work on the
     // tasks with a pending edge only (pick; the counts stay on the device).
     TaskPick pick_class[kNumBigClasses] = {}, pick_hub{};
+    const bool bound = d->E >= kBoundEdges && pr.eps < kBoundEps;   // (batches: the graphs' eps differ, pr.eps is 0)
     if constexpr (kPick) {
         const PendingWork pw{d->pend_pivot, d->cn_ctr + 2, d->plan.small_deg};
         SCAN_TRY(launch_sketch_filter<kPerGraph>(d, launches, pr, const_cast<uint8_t*>(fp.pend), pw));
@@ -954,7 +955,7 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
             pl.count[a] = count;
             pl.out[a] = out;
             const TaskPick pick{out, d->pend_counts + a, d->pend_edges,
-                                d->E >= kBoundEdges ? d->pend_votes + 2 * a : nullptr};
+                                bound ? d->pend_votes + 2 * a : nullptr};
             if (count) out += count + kPendingSlices * d->num_sms;
             longest = std::max(longest, count);
             return pick;
@@ -1053,7 +1054,7 @@ static scan_status launch_cn_impl(DeviceGraph* d, uint32_t* launches, const CnPr
                 };
                 if constexpr (kPick) {
                     SCAN_TRY(launch_big(std::integral_constant<CountForm, kCountOpen>()));
-                    if (d->E >= kBoundEdges) {
+                    if (bound) {
                         SCAN_TRY(launch_big(std::integral_constant<CountForm, kBoundOpen>()));
                         ++*launches;
                     }
@@ -1180,14 +1181,11 @@ scan_status autotune_similarity(DeviceGraph* d, float* best_ms, const std::funct
         d->long_words = lw;
         uint32_t launches = 0;
         SCAN_TRY(stage(&launches));   // warm
-        *ms = 3.4e38f;
-        for (int i = 0; i < 3; ++i) {   // the least of three: settings lie closer than single runs do
-            SCAN_CUDA(cudaEventRecord(d->ev[13], d->stream));
-            SCAN_TRY(stage(&launches));
-            SCAN_CUDA(cudaEventRecord(d->ev[14], d->stream));
-            SCAN_CUDA(cudaEventSynchronize(d->ev[14]));
-            *ms = std::min(*ms, ev_ms(d->ev[13], d->ev[14]));
-        }
+        SCAN_CUDA(cudaEventRecord(d->ev[13], d->stream));
+        SCAN_TRY(stage(&launches));
+        SCAN_CUDA(cudaEventRecord(d->ev[14], d->stream));
+        SCAN_CUDA(cudaEventSynchronize(d->ev[14]));
+        *ms = ev_ms(d->ev[13], d->ev[14]);
         return SCAN_OK;
     };
     PlanParams best_pp = d->plan;

@@ -91,7 +91,7 @@ def build_reference() -> bool:
               "cstring", "-include", "string", f"-I{REFERENCE}", str(REFERENCE / "Graph.cpp"),
               str(HERE / "ref_graph_shim.cpp"), "-o", str(REF_GRAPH_LIB)])
     # The reference's GPUScan program (GPUSCAN++/main.cpp + Graph.cpp, unmodified) with the
-    # engine in place of GPUScan.cu: the link-level drop-in of the makefile in INTEGRATION.md.
+    # engine in place of GPUScan.cu: the link-level drop-in.
     lib = PKG_BUILD / "libscan_gb300.so"
     if platform.machine() == "x86_64" and lib.exists() and _stale(
             REF_DROPIN, REFERENCE / "main.cpp", REFERENCE / "Graph.cpp", lib, Path(__file__)):
