@@ -8,7 +8,8 @@ cores, union-find, attach, hub/outlier) over the graph.
   value     device time, graph resident in HBM (CUDA events on the library's stream)
   e2e       the reference-facing drop-in GPUScan() (scan_gpuscan_compat) from pinned host
             CSR buffers to host labels: H2D, orientation, SCAN, D2H and device allocation
-  roofline  the common-neighbour stage, HBM bound
+  roofline  the similarity stage's DRAM traffic against the HBM rate, and the words of bitmaps and
+            lists that its kernels read (bound by L1 and L2, which supply most of them)
   cpu_baseline  the oracle (a plain OpenMP SCAN: the reference's degree prune, merge or
             binary-search intersection, predicate, union-find, attach, hub/outlier) over the
             whole graph, one pass on every host core
@@ -133,7 +134,10 @@ class Dist:
 
 
 class ClockSampler:
-    """nvidia-smi clocks and throttle reasons sampled every 200 ms during the timed region."""
+    """nvidia-smi clocks and throttle reasons, sampled every 50 ms under the timed steps' load.
+
+    The timed steps may be over before the first sample: start() returns once nvidia-smi prints,
+    and hold() repeats the step, untimed, until some samples have come in under load."""
 
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -143,23 +147,36 @@ class ClockSampler:
         self.index = index
         self.proc = None
         self.file = None
+        self.idle = 0          # samples before the load
 
     def start(self):
         try:
             self.file = tempfile.NamedTemporaryFile("w+", suffix=".csv", delete=False)
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.index}", f"--query-gpu={self.FIELDS}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"], stdout=self.file,
+                                          "--format=csv,noheader,nounits", "-lms", "50"], stdout=self.file,
                                          stderr=subprocess.DEVNULL)
         except Exception:
             self.proc = None
+            return
+        limit = time.perf_counter() + 5.0
+        while not self.rows() and self.proc.poll() is None and time.perf_counter() < limit:
+            time.sleep(0.01)
+        self.idle = len(self.rows())
+
+    def rows(self) -> list:
+        return [r.split(",") for r in Path(self.file.name).read_text().splitlines() if r.count(",") >= 8]
+
+    def hold(self, step, samples: int = 4, seconds: float = 2.0):
+        limit = time.perf_counter() + seconds
+        while self.proc and len(self.rows()) < self.idle + samples and time.perf_counter() < limit:
+            step()
 
     def stop(self) -> dict:
         if not self.proc:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
         self.proc.terminate()
         self.proc.wait()
-        self.file.flush()
-        rows = [r.split(",") for r in Path(self.file.name).read_text().strip().splitlines() if r.count(",") >= 8]
+        rows = self.rows()[self.idle:]
         os.unlink(self.file.name)
         sm = [float(r[1]) for r in rows if r[1].strip().replace(".", "").isdigit()]
         mx = [float(r[2]) for r in rows if r[2].strip().replace(".", "").isdigit()]
@@ -170,15 +187,14 @@ class ClockSampler:
 
 
 def byte_models(off: np.ndarray, adj: np.ndarray, eps: str) -> dict:
-    """Algorithmic bytes of one launch of the common-neighbour stage, from the graph alone.
+    """Algorithmic bytes of one launch of the similarity stage, from the graph alone.
 
+    compulsory: what a run with bitmaps cannot do without but for the bitmaps themselves: each
+    edge's endpoints (8 B) and state (1 B), each vertex's rank and degree (8 B).
     prune model: a one-shot run reads only the lists of edges the degree prune leaves at
     this eps (du + 1 >= eps^2 (dv + 1), u the lower endpoint); each such list once (4 du),
     every pivot list staged once (4 d_v), and every edge costs its endpoint, two offsets
     and its count (16 B) plus the zeroing of cn (4 B):  B = 4 sum_counted du + 4 sum_v d_v + 20 E.
-    (The roofline's own figure replaces 4 sum_counted du by the words of bitmaps and lists that
-    the kernels report reading.  Most of them come from L1 and L2, so it can pass the HBM rate;
-    `traffic` is what DRAM supplies.)
     full model: the same with every edge counted (the cached counts of the serving path).
     merge model (what a merge intersection of every edge reads): each edge streams both lists,
       B = sum_e [4 (du + dv) + 16] + 4 E = 4 sum_v d_v^2 + 20 E.
@@ -196,7 +212,7 @@ def byte_models(off: np.ndarray, adj: np.ndarray, eps: str) -> dict:
     counted = ~((du + 1.0) < (dv + 1.0) * e * e)
     staged = 4.0 * float(deg.sum())
     d = deg.astype(np.float64)
-    return {"prune": 4.0 * float(du[counted].sum()) + staged + 20.0 * E, "fixed": staged + 20.0 * E,
+    return {"prune": 4.0 * float(du[counted].sum()) + staged + 20.0 * E, "compulsory": 9.0 * E + 8.0 * n,
             "full": 4.0 * float(du.sum()) + staged + 20.0 * E,
             "merge": 4.0 * float((d * d).sum()) + 20.0 * E,
             "counted_edges": int(counted.sum())}
@@ -548,6 +564,7 @@ def main():
     torch.cuda.synchronize()
     dist.barrier()
     wall = time.perf_counter() - t0
+    clocks.hold(lambda: g.run(args.eps, args.mu, mode, device=local))
     clk = clocks.stop() if rank == 0 else None
     dev_ms = sum(s["ms_similarity"] + s["ms_cluster"] for s in stats)
     dev_ms = dist.max(dev_ms)
@@ -602,15 +619,19 @@ def main():
         return {"achieved": b / sim_s / 1e9, "frac": b / sim_s / 1e9 / peak, "bytes": b}
 
     words = float(np.mean([s["cn_words"] for s in stats]))
-    run_bytes = 16.0 * words + bm["fixed"]
     traffic, traffic_src = stage_traffic() if (args.scale, args.edge_factor, args.seed, args.eps) == (22, 16, 1, "0.5") \
         else (None, "no ncu summary for this configuration")
-    roof = {"bound": "hbm", "achieved": run_bytes / sim_s / 1e9, "peak": peak, "unit": "GB/s",
-            "frac": run_bytes / sim_s / 1e9 / peak, "traffic": traffic, "traffic_source": traffic_src,
-            "peak_source": peak_src,
-            "bytes": run_bytes, "list_words_read": words, "counted_edges": int(last["cn_edges_counted"]),
-            "bytes_model": "16*(bitmap and list words read, reported by the kernels; from L1, L2 and HBM) "
-                           "+ 4*sum_v d_v + 20E",
+    compulsory = bm["compulsory"] + g.bitmap_bytes
+    hbm_bytes = traffic if traffic else compulsory
+    roof = {"bound": "l1/l2", "achieved": hbm_bytes / sim_s / 1e9, "peak": peak, "unit": "GB/s",
+            "frac": hbm_bytes / sim_s / 1e9 / peak, "traffic": traffic, "traffic_source": traffic_src,
+            "peak_source": peak_src, "bytes": hbm_bytes,
+            "bytes_model": "DRAM traffic of the stage (ncu)" if traffic else
+                           "9E + 8n + every bitmap once (what DRAM must supply at least)",
+            "compulsory_bytes": compulsory, "counted_edges": int(last["cn_edges_counted"]),
+            "cache_words": {"words": words, "bytes": 16.0 * words, "gbs": 16.0 * words / sim_s / 1e9,
+                            "definition": "16-byte words of bitmaps (the lower endpoints') and lists the kernels report "
+                                          "reading; L1 and L2 supply most, so there is no fraction of the HBM rate"},
             "prune_model": dict(gbs(bm["prune"]), counted_edges=bm["counted_edges"],
                                 definition="4*sum over edges left by the degree prune of min(du,dv) + 4*sum_v d_v + 20E"),
             "full_model": dict(gbs(bm["full"]), definition="every edge counted (serving cache)"),

@@ -15,8 +15,9 @@
 // order of the vertices' ranks; ranks descend by L, so the vertices that have a size are the
 // first ones.  Every bitmap is aligned to its own size (up to 128 bytes), and what a run reads
 // (mostly one or two sizes per vertex) lies together: with each vertex's sizes side by side
-// instead, the similarity stage of R-MAT s22 at eps 0.5 took 2.06 ms, so 1.87.  All arrays
-// together are about as large as the adjacency.
+// instead, the similarity stage of R-MAT s22 at eps 0.5 took 2.06 ms, so 1.87.  All arrays and
+// what goes with them take 0.9 times the adjacency (random graphs, rings) to 1.5 times (R-MAT s22),
+// plans with split pivots half the adjacency more.
 #pragma once
 
 #include "device_common.cuh"
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(256, 4) k_sketch_filter(uint64_t E, const uint
                 uint32_t mine = gi, next = kGroups;        // slot of this group, first slot not taken
                 bool on = mine < groups;
                 SketchSlot s{0, 0, 0, 0};
-                const uint4 *pu = sk, *pv = sk;            // a group without an edge reads unit 0 on
+                const uint4 *pu = sk, *pv = sk;
                 uint32_t left = 0, miss = 0;               // units left at this size
                 auto open = [&]() {
                     left = 1u << (slot_level(s) - kSketchMinLog);
@@ -867,9 +868,7 @@ struct PendingLists {
     TaskSlice* out[kPendingLists];            // count + kPendingSlices per SM entries
 };
 
-// The pending edges of [e0, e1) in order to edges[e0...]; returns their number.  In order: the
-// chunk tasks of a split pivot gather the same edges at the same place, perhaps at the same
-// time.
+// Sum of the lanes before this one, and of all.
 __device__ __forceinline__ uint32_t warp_exclusive(uint32_t n, uint32_t lane, uint32_t* total) {
     uint32_t incl = n;
 #pragma unroll
@@ -881,6 +880,9 @@ __device__ __forceinline__ uint32_t warp_exclusive(uint32_t n, uint32_t lane, ui
     return incl - n;
 }
 
+// The pending edges of [e0, e1) in order to edges[e0...]; returns their number.  In order: the
+// chunk tasks of a split pivot gather the same edges at the same place, perhaps at the same
+// time.
 __device__ __forceinline__ uint32_t gather_pending_warp(const uint8_t* sim, uint32_t e0, uint32_t e1,
                                                         uint32_t* __restrict__ edges, uint32_t lane) {
     uint32_t found = 0;
