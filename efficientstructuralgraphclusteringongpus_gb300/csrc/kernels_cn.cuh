@@ -812,7 +812,7 @@ k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32
                 }
             }
         }
-        if constexpr (kForm == kCountOpen) {
+        if (kForm == kCountOpen && pick.votes) {
             w_passed = __reduce_add_sync(0xFFFFFFFFu, w_passed);
             if (lane == 0) {
                 atomicAdd(&seen, w_seen);
@@ -821,16 +821,13 @@ k_cn_big(const CnTask* __restrict__ tasks, uint32_t ntasks, uint32_t cap, uint32
             w_seen = w_passed = 0;
             __syncthreads();
             if (threadIdx.x == 0) {
-                leave = 0;
-                if (pick.votes) {
-                    const unsigned long long all = atomicAdd(pick.votes, (unsigned long long)seen) + seen;
-                    const unsigned long long those = atomicAdd(pick.votes + 1, (unsigned long long)passed) + passed;
-                    leave = all >= kBoundLeast && kBoundShare * those < all;
-                }
+                const unsigned long long all = atomicAdd(pick.votes, (unsigned long long)seen) + seen;
+                const unsigned long long those = atomicAdd(pick.votes + 1, (unsigned long long)passed) + passed;
+                leave = all >= kBoundLeast && kBoundShare * those < all;
             }
         }
         __syncthreads();
-        if (kForm == kCountOpen && leave) break;
+        if (kForm == kCountOpen && pick.votes && leave) break;
     }
     if constexpr (kPick) fused_totals(fp, lane, nsim, ndis);
     totals_flush(&totals, ctr);
