@@ -117,14 +117,15 @@ scan_status scan_batch_create(const scan_graph* const* graphs, uint32_t count, i
     }
     off[N] = M;
     B_CUDA(cudaSetDevice(device));
-    scan_status st = device_upload(device, N, M, off.data(), true, adj.data(), &b->d, nullptr);
-    if (st != SCAN_OK) return st;
     B_CUDA(cudaMalloc(&b->vgid, N * sizeof(uint32_t)));
     B_CUDA(cudaMalloc(&b->gpp, count * sizeof(PredParams)));
     B_CUDA(cudaMalloc(&b->gmu, count * sizeof(int32_t)));
     B_CUDA(cudaMalloc(&b->sets, kPruneSets * sizeof(PredParams)));
     B_CUDA(cudaMalloc(&b->nsets, sizeof(uint32_t)));
     B_CUDA(cudaMalloc(&b->np_tabs, (size_t)kPruneSets * kPruneTable * sizeof(uint32_t)));
+    // after the batch's own arrays: an upload that finds no room for its bitmaps goes without them
+    scan_status st = device_upload(device, N, M, off.data(), true, adj.data(), &b->d, nullptr);
+    if (st != SCAN_OK) return st;
     B_CUDA(cudaHostAlloc(&b->h_sets, (kPruneSets + 1) * sizeof(PredParams), cudaHostAllocDefault));
     B_CUDA(cudaMemcpy(b->vgid, vgid.data(), N * sizeof(uint32_t), cudaMemcpyHostToDevice));
     B_CUDA(cudaHostAlloc(&b->h_gpp, count * sizeof(PredParams), cudaHostAllocDefault));
